@@ -153,16 +153,32 @@ int Handle::ensure_levels() {
     if ((rc = reset_ctl())) return rc;
     const int sgrid = sm_count * 4;
     CUDA_TRY(cudaMemsetAsync(levels.p, 0, sizeof(int) * (size_t)n, st));
-    if (levels_kernel() == 0) {
+    int found = 0;  // the largest level, once the chunked walk has settled
+    if (levels_kernel() == 0 && level_chunks_apply(n, nnz)) {
+        if ((rc = scratch.ensure(level_chunks_scratch(n, nnz, sm_count)))) return rc;
+        if ((rc = launch_level_chunks(n, nnz, rp, col, levels.as<int>(), scratch.p, ctl, kDefaultBudgetNs, sm_count, st,
+                                      &launches, &found)))
+            return rc;
+        if (!found) {
+            if ((rc = reset_ctl())) return rc;
+            CUDA_TRY(cudaMemsetAsync(levels.p, 0, sizeof(int) * (size_t)n, st));
+        }
+    }
+    if (found) {
+        // settled: exact whatever the chunks' walks reported
+    } else if (levels_kernel() == 0) {
         if ((rc = launch_window_levels(n, nnz, rp, col, levels.as<int>(), ctl, kDefaultBudgetNs, st, &launches))) return rc;
     } else {
         k_levels<<<sm_count * 2, 256, 0, st>>>(n, rp, col, levels.as<int>(), ctl, kDefaultBudgetNs);
         ++launches;
         CUDA_TRY(cudaGetLastError());
     }
-    if ((rc = read_ctl(&c))) return rc;
-    if (c.status) return c.status;
-    max_level = c.max_level;
+    if (!found) {
+        if ((rc = read_ctl(&c))) return rc;
+        if (c.status) return c.status;
+        found = c.max_level;
+    }
+    max_level = found;
     // level buckets: counts -> level_ptr; stable radix sort of level keys -> level_rows
     if ((rc = level_ptr.ensure(sizeof(int) * (size_t)(max_level + 2)))) return rc;
     if ((rc = level_rows.ensure(sizeof(int) * (size_t)n))) return rc;

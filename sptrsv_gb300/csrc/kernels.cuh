@@ -78,6 +78,11 @@ int launch_window_levels(int n, long long nnz, const int* rp, const int* col, in
                          cudaStream_t st,
                          int64_t* launches);
 int window_warps();
+// levels by chunks of rows walked at once (window.cu)
+bool level_chunks_apply(int n, long long nnz);
+size_t level_chunks_scratch(int n, long long nnz, int sm_count);
+int launch_level_chunks(int n, long long nnz, const int* rp, const int* col, int* level, void* mem, Ctl* ctl,
+                        int64_t budget, int sm_count, cudaStream_t st, int64_t* launches, int* max_level);
 int launch_transpose(bool to_row_major, const double* src, double* dst, int n, int rhs, cudaStream_t st,
                      int64_t* launches);
 

@@ -40,19 +40,20 @@
 // as p = fma(-U_ij / U_ii, x_j, p), so a dependency hop costs one FP64 FMA.  The levels
 // (core.cpp:244-270) take the maximum over the row's columns: level_i = 1 + max_j level_j
 // (1 for a diagonal-only row), with 0 as the pending value, bit-exact.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
 #include "common.cuh"
 #include "kernels.cuh"
-namespace sptrsv { int window_backoff_ns(); int window_warps(); }
-namespace sptrsv { int window_backoff_ns(); int window_warps(); }
+namespace sptrsv { int window_warps(); }
 
 namespace sptrsv {
 
 constexpr int kWinRing = 4096;   // rows of x held in shared memory (power of two)
 constexpr int kWinFlags = 64;    // done-flag slots (power of two, multiple of W, >= 2W)
 constexpr int kWinSmemBudget = 200 * 1024;
+constexpr int kWinChunkBudget = 56 * 1024;  // chunked level walk: four CTAs per SM
 
 template <typename T> struct WinVal;
 template <> struct WinVal<double> {
@@ -70,14 +71,14 @@ template <> struct WinVal<int> {
 
 // Shared-memory layout: the ring and the done flags, then per warp three row-pointer slots,
 // two reciprocal-diagonal / right-hand-side slots and two entry buffers of kCap entries.
-template <typename T, int W> struct WinLayout {
+template <typename T, int W, int B = kWinSmemBudget> struct WinLayout {
     static constexpr bool kLevels = std::is_same<T, int>::value;
     static constexpr int kRpSlot = 36;  // 33 row pointers, padded to 16 bytes
     static constexpr size_t kFixed = (size_t)kWinRing * sizeof(T) + kWinFlags * sizeof(int);
     static constexpr size_t kPerWarpFixed = 3 * kRpSlot * sizeof(int) + (kLevels ? 0 : 2 * 2 * 32 * sizeof(T));
     static constexpr size_t kPerEntry = 2 * (sizeof(int) + (kLevels ? 0 : sizeof(T)));
     // entries per buffer: what the budget leaves, a multiple of 32
-    static constexpr int kCap = (int)(((kWinSmemBudget - kFixed) / W - kPerWarpFixed) / kPerEntry) / 32 * 32;
+    static constexpr int kCap = (int)(((B - kFixed) / W - kPerWarpFixed) / kPerEntry) / 32 * 32;
     static constexpr size_t kPerWarp = kPerWarpFixed + (size_t)kCap * kPerEntry;
     static constexpr size_t kBytes = kFixed + (size_t)W * kPerWarp;
     static_assert(kCap >= 64, "staging buffers too small");
@@ -98,19 +99,19 @@ template <typename T> __device__ __forceinline__ void cpa(T* s, const T* g) {
 __device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cpa_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Rows [lo, top) of block t.
+// Rows [lo, top) of block t of the rows [row0, n).
 __device__ __forceinline__ int win_top(int n, int t) { return n - 32 * t; }
-__device__ __forceinline__ int win_lo(int n, int t) { return max(0, n - 32 * t - 32); }
+__device__ __forceinline__ int win_lo(int row0, int n, int t) { return max(row0, n - 32 * t - 32); }
 
 // One warp's staging buffers.
-template <typename T, int W> struct WinStage {
+template <typename T, int W, int B> struct WinStage {
     int* rp;   // [3][kRpSlot]
     T* inv;    // [2][32]
     T* bb;     // [2][32]
     int* col;  // [2][kCap]
     T* val;    // [2][kCap]
     __device__ WinStage(char* base) {
-        using L = WinLayout<T, W>;
+        using L = WinLayout<T, W, B>;
         rp = (int*)base;
         char* p = base + 3 * L::kRpSlot * sizeof(int);
         if constexpr (!L::kLevels) {
@@ -127,20 +128,21 @@ template <typename T, int W> struct WinStage {
 };
 
 // Copy block t's row pointers (rows lo .. top, inclusive) into rp slot `rs`.
-template <typename T, int W>
-__device__ __forceinline__ void win_stage_rp(const WinStage<T, W>& S, int rs, const int* rp, int n, int t, int lane) {
-    const int lo = win_lo(n, t), top = win_top(n, t);
-    int* d = S.rp + rs * WinLayout<T, W>::kRpSlot;
+template <typename T, int W, int B>
+__device__ __forceinline__ void win_stage_rp(const WinStage<T, W, B>& S, int rs, const int* rp, int row0, int n, int t,
+                                             int lane) {
+    const int lo = win_lo(row0, n, t), top = win_top(n, t);
+    int* d = S.rp + rs * WinLayout<T, W, B>::kRpSlot;
     for (int q = lane; q <= top - lo; q += 32) cpa4(d + q, rp + lo + q);
 }
 
 // Copy block t's entries (when they fit), reciprocal diagonal and right-hand side into data slot
 // `ds`; its row pointers are already in rp slot `rs`.
-template <typename T, int W>
-__device__ __forceinline__ void win_stage_data(const WinStage<T, W>& S, int rs, int ds, const int* col, const T* val,
-                                               const T* invd, const T* b, int n, int t, int lane) {
-    using L = WinLayout<T, W>;
-    const int lo = win_lo(n, t), top = win_top(n, t);
+template <typename T, int W, int B>
+__device__ __forceinline__ void win_stage_data(const WinStage<T, W, B>& S, int rs, int ds, const int* col, const T* val,
+                                               const T* invd, const T* b, int row0, int n, int t, int lane) {
+    using L = WinLayout<T, W, B>;
+    const int lo = win_lo(row0, n, t), top = win_top(n, t);
     const int* r = S.rp + rs * L::kRpSlot;
     const int e0 = r[0], cnt = r[top - lo] - e0;
     if (cnt <= L::kCap) {
@@ -184,12 +186,35 @@ __device__ __noinline__ T win_wait(const T* p, Ctl* ctl, int64_t budget) {
     }
 }
 
-template <typename T, int W>
-__global__ void __launch_bounds__(W * 32, 1)
-k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T* __restrict__ val,
-         const T* __restrict__ invd, const T* __restrict__ b, T* x, Ctl* ctl, int64_t budget) {
-    using L = WinLayout<T, W>;
+// The chunked level walk: CTA c walks rows [n - (c+1) rows, n - c rows) after a run-up of `warm` rows
+// below them, as if U ended there (columns at or past the run-up's end count as level 0).  Levels of
+// the run-up go to its own slice of run_up, the chunk's to x.
+struct WinChunks {
+    int rows = 0, warm = 0;
+    int* run_up = nullptr;
+};
+
+template <typename T, int W, int B = kWinSmemBudget, bool kChunk = false>
+__global__ void __launch_bounds__(W * 32, kChunk && B == kWinChunkBudget ? 4 : 1)
+k_window(int n_all, const int* __restrict__ rp, const int* __restrict__ col, const T* __restrict__ val,
+         const T* __restrict__ invd, const T* __restrict__ b, T* x, Ctl* ctl, int64_t budget, WinChunks ch) {
+    using L = WinLayout<T, W, B>;
     constexpr bool kLevels = L::kLevels;
+    static_assert(kLevels || !kChunk, "only the level walk runs in chunks");
+    // rows [row0, n); rows from `hi` up are a chunk's run-up
+    int row0 = 0, n = n_all, hi = n_all;
+    T* run_up = nullptr;
+    if constexpr (kChunk) {
+        hi = n_all - (int)blockIdx.x * ch.rows;
+        row0 = max(0, hi - ch.rows);
+        n = min(n_all, hi + ch.warm);
+        run_up = ch.run_up + (size_t)blockIdx.x * ch.warm;
+    }
+    // x of a far column; in a chunk's walk -1 (no effect, not pending) past its run-up
+    auto far_x = [&](int c) -> const T* {
+        if constexpr (kChunk) return c >= hi ? run_up + (c - hi) : x + c;
+        else return x + c;
+    };
     constexpr int RM = kWinRing - 1;
     constexpr int reach = kWinRing - 32 * (2 * W + 1);
     static_assert(reach >= 32 * (W + 1), "ring too small for W warps");
@@ -204,16 +229,16 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
     for (int q = threadIdx.x; q < kWinFlags; q += blockDim.x) dflag[q] = -1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nblk = (n + 31) >> 5;
-    const WinStage<T, W> S(win_smem + L::kFixed + (size_t)warp * L::kPerWarp);
+    const int nblk = (n - row0 + 31) >> 5;
+    const WinStage<T, W, B> S(win_smem + L::kFixed + (size_t)warp * L::kPerWarp);
     // prologue: row pointers of the warp's first two blocks, then the first block's data
     if (warp < nblk) {
-        win_stage_rp<T, W>(S, 0, rp, n, warp, lane);
-        if (warp + W < nblk) win_stage_rp<T, W>(S, 1, rp, n, warp + W, lane);
+        win_stage_rp(S, 0, rp, row0, n, warp, lane);
+        if (warp + W < nblk) win_stage_rp(S, 1, rp, row0, n, warp + W, lane);
         cpa_commit();
         cpa_wait_all();
         __syncwarp();
-        win_stage_data<T, W>(S, 0, 0, col, val, invd, b, n, warp, lane);
+        win_stage_data(S, 0, 0, col, val, invd, b, row0, n, warp, lane);
         cpa_commit();
     }
     __syncthreads();
@@ -230,12 +255,12 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
     bool nfail = false;           // a far value never arrived (not expected): the lane gives up
     auto prepare = [&](int u, int jj) {
         const int ds_u = jj & 1;
-        const int top = win_top(n, u), lo = win_lo(n, u);
+        const int top = win_top(n, u), lo = win_lo(row0, n, u);
         const int* rS = S.rp + (jj % 3) * L::kRpSlot;
         const int e0 = rS[0];
         const bool staged = rS[top - lo] - e0 <= L::kCap;
         const int i = top - 1 - lane;
-        const int far = top + reach;
+        const int far = kChunk ? min(top + reach, n) : top + reach;
         nk = e0;
         np = nacc = T(0);
         nfail = false;
@@ -272,12 +297,15 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
                 vq[q] = use[q] ? weight(kq) : T(0);
             }
 #pragma unroll
-            for (int q = 0; q < 4; ++q) xq[q] = use[q] ? win_ld<T>(x + cq[q]) : T(0);
+            for (int q = 0; q < 4; ++q) {
+                if (kChunk && use[q] && cq[q] >= n) xq[q] = T(-1);
+                else xq[q] = use[q] ? win_ld<T>(far_x(cq[q])) : T(0);
+            }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 // not expected: those blocks are done.  Wait all the same, bounded like every wait.
                 if (use[q] && !fail && WinVal<T>::is_pending(xq[q])) {
-                    xq[q] = win_wait<T>(x + cq[q], ctl, budget);
+                    xq[q] = win_wait<T>(far_x(cq[q]), ctl, budget);
                     fail = WinVal<T>::is_pending(xq[q]);
                 }
             }
@@ -337,10 +365,10 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
         __syncwarp();
         const int rs = j % 3, ds = j & 1;
         // 3. stage ahead: row pointers of block t+2W, data of block t+W; reset block t+W's ring slots
-        if (t + 2 * W < nblk) win_stage_rp<T, W>(S, (j + 2) % 3, rp, n, t + 2 * W, lane);
-        if (t + W < nblk) win_stage_data<T, W>(S, (j + 1) % 3, (j + 1) & 1, col, val, invd, b, n, t + W, lane);
+        if (t + 2 * W < nblk) win_stage_rp(S, (j + 2) % 3, rp, row0, n, t + 2 * W, lane);
+        if (t + W < nblk) win_stage_data(S, (j + 1) % 3, (j + 1) & 1, col, val, invd, b, row0, n, t + W, lane);
         cpa_commit();
-        const int top = win_top(n, t), lo = win_lo(n, t);
+        const int top = win_top(n, t), lo = win_lo(row0, n, t);
         if (t + W < nblk) {
             const int r2 = top - 32 * W - 1 - lane;
             if (r2 >= 0) vring[r2 & RM] = WinVal<T>::pending();
@@ -350,7 +378,7 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
         const int e0 = rS[0];
         const bool staged = rS[top - lo] - e0 <= L::kCap;
         const int i = top - 1 - lane;
-        const int far = top + reach;
+        const int far = kChunk ? min(top + reach, n) : top + reach;
         bool done = i < lo;
         int s = e0, k = e0, c = 0;  // a lane without a row (short last block) reads entry e0 harmlessly
         if (!done) {
@@ -395,7 +423,7 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
         // parity); stops at the first pending one
         auto walk = [&]() {
             while (k > s) {
-                const T xv = c >= far ? win_ld<T>(x + c) : vring[c & RM];
+                const T xv = kChunk && c >= n ? T(-1) : c >= far ? win_ld<T>(far_x(c)) : vring[c & RM];
                 if (WinVal<T>::is_pending(xv)) break;
                 if constexpr (kLevels) acc = max(acc, xv);
                 else if (k & 1) p2 = fma(v, xv, p2);
@@ -464,7 +492,7 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
                 // near one (rare; the far loop took the sorted case).  A finished lane's stale
                 // column reads a slot whose value is discarded.
                 T x0;
-                if (__builtin_expect(c >= far, 0)) x0 = win_ld<T>(x + c);
+                if (__builtin_expect(c >= far, 0)) x0 = kChunk && c >= n ? T(-1) : win_ld<T>(far_x(c));
                 else x0 = vring[c & RM];
                 const bool rdy = !done && !WinVal<T>::is_pending(x0);
                 if constexpr (kLevels) acc = rdy ? max(acc, x0) : acc;
@@ -528,7 +556,7 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
         }
         // 5. block t done: its rows to global x in one coalesced store; those stores, the ring
         //    stores and the reset of block t+W's slots before the flag
-        if (i >= lo) win_st<T>(x + i, xm);
+        if (i >= lo) win_st<T>(const_cast<T*>(far_x(i)), xm);
         __threadfence_block();
         __syncwarp();
         if (lane == 0) vflag[t & (kWinFlags - 1)] = t;
@@ -540,7 +568,7 @@ k_window(int n, const int* __restrict__ rp, const int* __restrict__ col, const T
         }
     }
     cpa_wait_all();  // no copy left in flight when the warp exits
-    if constexpr (kLevels) {
+    if constexpr (kLevels && !kChunk) {
         for (int o = 16; o > 0; o >>= 1) lmax = max(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
         if (lane == 0 && lmax > 0) atomicMax(&ctl->max_level, lmax);
     }
@@ -559,7 +587,7 @@ static int window_launch(int n, const int* rp, const int* col, const T* val, con
         CUDA_TRY(cudaFuncSetAttribute(k_window<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kBytes));
         configured[dev] = true;
     }
-    k_window<T, W><<<1, W * 32, L::kBytes, st>>>(n, rp, col, val, invd, b, x, ctl, budget);
+    k_window<T, W><<<1, W * 32, L::kBytes, st>>>(n, rp, col, val, invd, b, x, ctl, budget, WinChunks{});
     ++*launches;
     CUDA_TRY(cudaGetLastError());
     return 0;
@@ -610,6 +638,174 @@ int launch_window(bool f32, const SolveArgs& a) {
     return window_dispatch<double>(a.n, a.nnz, a.rp, a.col, (const double*)a.val, (const double*)a.invd,
                                    (const double*)a.b, (double*)a.x, a.ctl, a.budget, a.st, a.launches);
 }
+
+// --- levels in chunks ---------------------------------------------------------------------
+//
+// The walk of one CTA costs ~20 ns a row whatever the GPU has beside it.  Levels have a property that
+// lets many CTAs walk at once: a chunk walked after a run-up of a few hundred rows, with nothing known
+// below the run-up, gets its rows' levels up to one constant -- the longest paths have merged
+// (rank convergence of max-plus products: Maleki, Musuvathi and Mytkowicz, "Parallelizing dynamic
+// programming through rank convergence", 2014).  So:
+//   1. every chunk is walked by a CTA of its own (k_window<int, .., kChunk>);
+//   2. k_level_offsets: a chunk's constant is the difference between the two walks of the row with the
+//      highest level among the 64 rows below the chunk (the walk of the chunk they belong to and this
+//      chunk's run-up), summed from the bottom chunk up; k_level_shift adds the constants;
+//   3. k_level_sweep replaces every row's level by 1 + max_j level_j, in place, until a sweep changes
+//      nothing.  A fixed point of that rule is the level function itself (row n-1 is right, so row n-2
+//      is, ...), so the result is exact whatever the walks gave; they only have to make the sweeps few.
+// Rows whose path leaves the run-up (a row with far columns only) are what the sweeps mend: on random
+// factors of 8 entries a row 40 of 60,000 rows in two sweeps, of 4 entries 1,700 in four.
+// Measured on GB300, 8.8 entries per row, the whole analysis: 500k rows 11.1 -> 0.60 ms (the walk 85 us
+// with four CTAs an SM, offsets 24, sweeps 6 x 10), 2M rows 45 -> 0.95 ms.  Bound by the walk's rounds
+// (~750 dependent levels of a chunk and its run-up at ~110 ns).
+constexpr int kChunkMinRows = 512;    // rows of the smallest chunk
+constexpr int kChunkWarm = 1024;      // rows of the run-up (near columns within 64 rows merge in ~250)
+constexpr int kChunkMinN = 8192;
+constexpr int kChunkSweeps = 24;      // then the one-CTA walk
+constexpr int kChunkMaxCtas = 2048;   // chunks k_level_offsets takes
+
+// One CTA: off[c] of every chunk.
+__global__ void __launch_bounds__(1024) k_level_offsets(int n, int chunks, WinChunks ch, const int* __restrict__ level,
+                                                        int* __restrict__ off) {
+    __shared__ int d[kChunkMaxCtas], s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int c = warp; c < chunks; c += 32) {
+        int delta = 0;
+        if (c > 0) {
+            const int hi = n - c * ch.rows, cnt = min(64, n - hi);
+            int best = -1;
+            for (int q = lane; q < cnt; q += 32) {
+                const int r = ch.run_up[(size_t)c * ch.warm + q];
+                if (r > best) { best = r; delta = level[hi + q] - r; }
+            }
+            const int top = __reduce_max_sync(0xffffffffu, best);
+            delta = __shfl_sync(0xffffffffu, delta, __ffs(__ballot_sync(0xffffffffu, best == top)) - 1);
+        }
+        if (lane == 0) d[c] = delta;
+    }
+    __syncthreads();
+    // inclusive sums, a run of chunks per thread
+    const int per = (chunks + 1023) / 1024, c0 = threadIdx.x * per;
+    int sum = 0;
+    for (int q = 0; q < per; ++q)
+        if (c0 + q < chunks) sum += d[c0 + q];
+    int inc = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    int base = inc - sum;
+    for (int w = 0; w < warp; ++w) base += s_warp[w];
+    for (int q = 0; q < per; ++q)
+        if (c0 + q < chunks) off[c0 + q] = base += d[c0 + q];
+}
+
+__global__ void k_level_shift(int n, int rows, const int* __restrict__ off, int* __restrict__ level) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        level[i] += off[(n - 1 - i) / rows];
+}
+
+// Sweep q: state[q] counts the rows it changed; a sweep after one that changed nothing does nothing.
+// The sweep that changes nothing has seen the final levels: it leaves their maximum.
+__global__ void __launch_bounds__(256) k_level_sweep(int n, const int* __restrict__ rp, const int* __restrict__ col,
+                                                     int* level, int* state, int q) {
+    if (q > 0 && *(volatile const int*)(state + q - 1) == 0) return;
+    int changed = 0, top = 0;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int i = n - 1 - t, e = rp[i + 1];
+        int m = 0, k = rp[i] + 1;
+        for (; k + 3 < e; k += 4)
+            m = max(m, max(max(level[col[k]], level[col[k + 1]]), max(level[col[k + 2]], level[col[k + 3]])));
+        for (; k < e; ++k) m = max(m, level[col[k]]);
+        ++m;
+        if (m != level[i]) {
+            level[i] = m;
+            ++changed;
+        }
+        top = max(top, m);
+    }
+    changed = __reduce_add_sync(0xffffffffu, changed);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) {
+        if (changed) atomicAdd(state + q, changed);
+        if (top) atomicMax(state + kChunkSweeps + q, top);
+    }
+}
+
+template <int B>
+static int level_chunks_launch(int n, int chunks, const WinChunks& ch, const int* rp, const int* col, int* level,
+                               Ctl* ctl, int64_t budget, cudaStream_t st, int64_t* launches) {
+    using L = WinLayout<int, 8, B>;
+    CUDA_TRY(cudaFuncSetAttribute(k_window<int, 8, B, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kBytes));
+    k_window<int, 8, B, true><<<chunks, 8 * 32, L::kBytes, st>>>(n, rp, col, nullptr, nullptr, nullptr, level, ctl,
+                                                                  budget, ch);
+    ++*launches;
+    CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
+// Chunks: as many as are resident at once (four CTAs an SM while the rows' entries fit the small
+// staging buffers, else one), none below kChunkMinRows rows.
+static void level_chunk_shape(int n, long long nnz, int sm_count, bool* small, WinChunks* ch, int* chunks) {
+    *small = 32.0 * (double)nnz / n <= 0.9 * WinLayout<int, 8, kWinChunkBudget>::kCap;
+    const long long most = std::min<long long>(kChunkMaxCtas, (long long)sm_count * (*small ? 4 : 1));
+    const long long want = std::max(1ll, std::min<long long>(most, n / kChunkMinRows));
+    ch->rows = (int)((n + want - 1) / want + 31) / 32 * 32;
+    ch->warm = kChunkWarm;
+    *chunks = (n + ch->rows - 1) / ch->rows;
+}
+
+size_t level_chunks_scratch(int n, long long nnz, int sm_count) {
+    bool small;
+    WinChunks ch;
+    int chunks;
+    level_chunk_shape(n, nnz, sm_count, &small, &ch, &chunks);
+    return sizeof(int) * ((size_t)chunks * (ch.warm + 1) + 2 * kChunkSweeps);
+}
+
+// The levels by chunks, into level (zeroed); waits for the stream.  *max_level is left 0 when the
+// sweeps did not settle (the caller then walks the rows with one CTA, from zeroed levels).  `mem`
+// holds level_chunks_scratch bytes.
+int launch_level_chunks(int n, long long nnz, const int* rp, const int* col, int* level, void* mem, Ctl* ctl,
+                        int64_t budget, int sm_count, cudaStream_t st, int64_t* launches, int* max_level) {
+    *max_level = 0;
+    bool small;
+    WinChunks ch;
+    int chunks, rc;
+    level_chunk_shape(n, nnz, sm_count, &small, &ch, &chunks);
+    int* state = (int*)mem;
+    int* off = state + 2 * kChunkSweeps;
+    ch.run_up = off + chunks;
+    CUDA_TRY(cudaMemsetAsync(mem, 0, level_chunks_scratch(n, nnz, sm_count), st));
+    if (small) rc = level_chunks_launch<kWinChunkBudget>(n, chunks, ch, rp, col, level, ctl, budget, st, launches);
+    else rc = level_chunks_launch<kWinSmemBudget>(n, chunks, ch, rp, col, level, ctl, budget, st, launches);
+    if (rc) return rc;
+    k_level_offsets<<<1, 1024, 0, st>>>(n, chunks, ch, level, off);
+    k_level_shift<<<sm_count * 4, 256, 0, st>>>(n, ch.rows, off, level);
+    *launches += 2;
+    int host[2 * kChunkSweeps];
+    const int blocks = std::min((n + 255) / 256, sm_count * 8);
+    for (int q = 0; q < kChunkSweeps;) {
+        const int end = q == 0 ? 6 : kChunkSweeps;  // most matrices settle within the first few
+        for (; q < end; ++q) k_level_sweep<<<blocks, 256, 0, st>>>(n, rp, col, level, state, q), ++*launches;
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaMemcpyAsync(host, state, sizeof(host), cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        for (int u = 0; u < q; ++u)
+            if (host[u] == 0) {
+                *max_level = host[kChunkSweeps + u];
+                return 0;
+            }
+    }
+    return 0;
+}
+
+// Rows from which the chunks are tried, and the row length up to which: a chunk and its run-up cost
+// the one-CTA walk's time for ~2,000 rows (40 us) and the sweeps a few launches, against 20 ns a row;
+// long rows have no near window to merge in (and are the supernodal solve's).
+bool level_chunks_apply(int n, long long nnz) { return n >= kChunkMinN && (double)nnz <= 64.0 * n; }
 
 int launch_window_levels(int n, long long nnz, const int* rp, const int* col, int* level, Ctl* ctl, int64_t budget,
                          cudaStream_t st, int64_t* launches) {
