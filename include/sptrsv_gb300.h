@@ -91,7 +91,8 @@ enum sptrsv_kernel_kind {
     SPTRSV_K_TRANSPOSE = 12,   /* column-major <-> row-major */
     SPTRSV_K_PULL_BLOCK = 13,  /* sync-free CSR pull, shared-memory blocks */
     SPTRSV_K_SUPERNODAL = 14,  /* supernode panel products (FP64, or BF16x3 tensor cores) */
-    SPTRSV_K_WINDOW = 15       /* sync-free CSR pull by one CTA over a shared-memory ring */
+    SPTRSV_K_WINDOW = 15,      /* sync-free CSR pull by one CTA over a shared-memory ring */
+    SPTRSV_K_SETTLE = 16       /* FP64 sweeps until the solution stands still */
 };
 
 typedef struct sptrsv_opts {

@@ -256,6 +256,25 @@ static bool auto_window(double mean_len) {
     return w < 0 ? mean_len <= 90.0 : w == 1;
 }
 
+// Whether FP64 AUTO tries the sweeps (settle.cu) before the exact kernel: when the sweeps of a
+// contracting matrix take less than 0.7 of the exact kernel's time (a matrix that does not contract
+// costs nine of them on top).  Measured on GB300, 8.8 entries a row: 24-31 sweeps of 11 us + 4 us per
+// million entries and columns; the exact kernels take 0.19 us a level with one right-hand side
+// (10k rows 332 us, sweeps 334; 50k rows 1.7 ms, sweeps 0.42) and 2 us with several (200k rows x 8
+// 70 ms, sweeps 1.95).  Tiles of long rows do not fit shared memory.
+bool Handle::settle_pays(int rhs) const {
+    const double depth = levels_ready ? (double)max_level : depth_est;
+    const double sweeps_us = 28.0 * (11.0 + 4.0e-6 * (double)nnz * rhs);
+    return mean_len <= kSettleMaxLen && sweeps_us < 0.7 * (rhs == 1 ? 0.19 : 2.0) * depth;
+}
+
+// The exact sync-free kernel of FP64 AUTO: for one RHS the window or the block kernel (auto_window),
+// for several the block kernel once per column on long rows, else the RHS-tiled warp kernel.
+int Handle::exact_schedule(int rhs) const {
+    if (rhs == 1) return auto_window(mean_len) ? SPTRSV_SCHED_SYNCFREE_WINDOW : SPTRSV_SCHED_SYNCFREE_BLOCK;
+    return mean_len >= kBlockPerColumnLen ? SPTRSV_SCHED_SYNCFREE_BLOCK : SPTRSV_SCHED_SYNCFREE_WARP;
+}
+
 // Schedule choice from the analysis features (the autotuner overrides it).
 sptrsv_opts Handle::resolve(const sptrsv_opts* o, int rhs) const {
     sptrsv_opts r;
@@ -287,13 +306,10 @@ sptrsv_opts Handle::resolve(const sptrsv_opts* o, int rhs) const {
         } else if (r.precision == SPTRSV_PREC_MIXED) {
             r.schedule = SPTRSV_SCHED_JACOBI;
         } else {
-            // wide, shallow DAGs: one grid barrier per level is cheap; otherwise the block
-            // sync-free kernel for one RHS (and, once per column, for several RHS on long rows)
-            // and the RHS-tiled warp kernel for several RHS on short rows
+            // wide, shallow DAGs: one grid barrier per level is cheap; deep ones: sweeps where they
+            // pay, else the exact sync-free kernel
             if (levels_ready && width >= 2048.0 && max_level <= 2000) r.schedule = SPTRSV_SCHED_LEVELSET;
-            else if (rhs == 1) r.schedule = auto_window(mean_len) ? SPTRSV_SCHED_SYNCFREE_WINDOW : SPTRSV_SCHED_SYNCFREE_BLOCK;
-            else if (mean_len >= kBlockPerColumnLen) r.schedule = SPTRSV_SCHED_SYNCFREE_BLOCK;
-            else r.schedule = SPTRSV_SCHED_SYNCFREE_WARP;
+            else r.schedule = settle_pays(rhs) ? kSchedSettle : exact_schedule(rhs);
         }
     }
     if (r.precision == SPTRSV_PREC_MIXED) {
@@ -348,6 +364,8 @@ int Handle::prepare(const sptrsv_opts& o, int rhs, int layout) {
         if ((rc = grow(d32b, sizeof(float) * nr))) return rc;
         if ((rc = grow(norms, sizeof(double) * 2 * (size_t)rhs))) return rc;
     }
+    if (o.schedule == kSchedSettle)
+        if ((rc = grow(settle, sizeof(int) * kSettleSweeps))) return rc;
     if (o.schedule == SPTRSV_SCHED_SYNCFREE_CSC && o.precision == SPTRSV_PREC_FP64) {
         if ((rc = build_csc())) return rc;
         if ((rc = grow(indeg_work, sizeof(int) * (size_t)n))) return rc;
@@ -398,6 +416,17 @@ int Handle::enqueue(const sptrsv_opts& o, const double* b, double* x, int rhs, i
     a.launches = &launches;
     if (o.precision == SPTRSV_PREC_FP64) {
         switch (o.schedule) {
+            case kSchedSettle:
+                if ((rc = launch_settle(a, settle.as<int>()))) return rc;
+                if ((rc = mark(SPTRSV_K_SETTLE))) return rc;
+                // the exact kernel, for a matrix whose sweeps did not contract
+                switch (exact_schedule(rhs)) {
+                    case SPTRSV_SCHED_SYNCFREE_WINDOW: rc = launch_window(false, a); break;
+                    case SPTRSV_SCHED_SYNCFREE_BLOCK: rc = launch_bsf(false, a); break;
+                    default: rc = launch_pull_warp(false, a, o.rows_per_warp, o.rhs_tile);
+                }
+                if (rc || (rc = mark(rhs == 1 ? SPTRSV_K_WINDOW : SPTRSV_K_PULL_WARP))) return rc;
+                break;
             case SPTRSV_SCHED_SYNCFREE_THREAD:
                 if (rhs == 1) {
                     if ((rc = launch_fill_pending(false, xrm, (size_t)n * rhs, st, &launches))) return rc;
@@ -778,6 +807,7 @@ int Handle::solve(const sptrsv_opts* o_in, const double* b, double* x, int rhs, 
     if (!analysed) return SPTRSV_ERR_NO_ANALYSIS;
     if (rhs < 1 || !b || !x || (layout != SPTRSV_COL_MAJOR && layout != SPTRSV_ROW_MAJOR)) return SPTRSV_ERR_INVALID_ARG;
     if ((size_t)n * rhs > (size_t)0x7fffffff) return SPTRSV_ERR_TOO_LARGE;
+    if (o_in && o_in->schedule == kSchedSettle) return SPTRSV_ERR_UNSUPPORTED;
     sptrsv_opts o = resolve(o_in, rhs);
     if (o.precision == SPTRSV_PREC_MIXED && rhs > 1024) return SPTRSV_ERR_UNSUPPORTED;
     int rc;
@@ -915,7 +945,7 @@ Handle::~Handle() {
     for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
     if (prof0) cudaEventDestroy(prof0);
     DevBuf* bufs[] = {&own_rp, &own_col, &own_val, &val32, &invd, &invd32, &in_degree, &levels, &level_ptr,
-                      &level_rows, &stats, &csc_ptr, &csc_row, &csc_val, &scratch, &xw, &bw, &r32, &d32a, &d32b,
+                      &level_rows, &stats, &csc_ptr, &csc_row, &csc_val, &scratch, &settle, &xw, &bw, &r32, &d32a, &d32b,
                       &norms, &indeg_work, &left, &db, &dx, &flush, &offdiag, &roff, &jmeta, &jbase, &sell, &sell_perm, &sell_len, &sell_ptr,
                       &sn_start, &sn_m, &sn_roff, &sn_rect, &sn_goff, &sn_ld, &sn_colbase, &sn_outbase, &sn_items,
                       &sn_G, &sn_Ghi, &sn_Glo, &sn_pan, &sn_pitems, &sn_pcnt, &sn_ppart, &sn_gtc, &sn_tcrec, &sn_ghl, &sn_gexp, &tune_b, &tune_x};

@@ -32,6 +32,10 @@ constexpr double kBlockPerColumnLen = 64.0;
 // 0.253 / 0.147 / 0.109 / 0.081 ms at 64 / 128 / 192 / 256 rows).
 constexpr int kAutoChunkRows = 256;
 
+// FP64 AUTO's schedule for deep DAGs, not one a caller can name: settle.cu's sweeps, with the exact
+// AUTO kernel behind them.
+constexpr int kSchedSettle = 100;
+
 struct GraphKey {
     sptrsv_opts o;
     const double* b;
@@ -120,7 +124,7 @@ struct Handle {
     bool have_offdiag = false;
 
     // work
-    DevBuf scratch, xw, bw, r32, d32a, d32b, norms, indeg_work, left, db, dx, flush;
+    DevBuf scratch, settle, xw, bw, r32, d32a, d32b, norms, indeg_work, left, db, dx, flush;
     unsigned flush_byte = 1;
     bool last_mixed = false;
     bool last_cond = false;       // the last solve ran the conditional (device-looped) graph
@@ -150,6 +154,8 @@ struct Handle {
     int analyse();
     int ensure_levels();
     int build_csc();
+    bool settle_pays(int rhs) const;
+    int exact_schedule(int rhs) const;
     sptrsv_opts resolve(const sptrsv_opts* o, int rhs) const;
     int prepare(const sptrsv_opts& o, int rhs, int layout);
     int enqueue(const sptrsv_opts& o, const double* b, double* x, int rhs, int layout);

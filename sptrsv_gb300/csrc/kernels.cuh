@@ -86,6 +86,13 @@ int launch_level_chunks(int n, long long nnz, const int* rp, const int* col, int
 int launch_transpose(bool to_row_major, const double* src, double* dst, int n, int rhs, cudaStream_t st,
                      int64_t* launches);
 
+// settle.cu: FP64 sweeps in place until the solution stands still; sets ctl->done (and prepares the
+// exact kernel launched behind it: x pending and rows to claim only when it is not set).  `worst`:
+// kSettleSweeps ints of device memory.
+constexpr int kSettleSweeps = 64;
+constexpr double kSettleMaxLen = 20.0;  // mean entries per row
+int launch_settle(const SolveArgs& a, int* worst);
+
 // supernodal.cu -- the panel work list and dense panels of a supernode partition
 struct SnArgs {
     int nitems;

@@ -1,0 +1,321 @@
+// settle.cu -- the FP64 solve of a deep DAG by sweeps that run until the solution stands still.
+//
+// Substitution is the only fixed point of x_i <- (b_i - sum_j U_ij x_j) / U_ii: row n-1 has no other
+// value, so row n-2 has none, and so on up.  Sweeping that rule over all rows at once therefore
+// computes what the exact kernels compute, from any start and in any order, once the sweeps stand
+// still; they do after a few dozen when U's off-diagonals are small against its diagonal, instead of
+// after as many dependent hops as the DAG has levels.  A sweep reads U once at bandwidth, a hop costs
+// 0.2 us on one CTA.  A matrix whose sweeps do not contract is given up after a few of them (see
+// settle_hopeless) and solved by the exact kernel launched behind this one, which returns at once
+// when this one has finished (ctl->done).
+//
+// When it stands still: every row's new value differs from the one it replaces by less than 2^-50 of
+// the largest of |x_i|, |b_i / U_ii| and the terms |U_ij x_j / U_ii| it is formed from.  That is the
+// size of the rounding error substitution itself may make in forming x_i (k + 1 half-ulps of the sum
+// of k terms; eight terms a row), so the result is substitution's with local errors of the same size,
+// and what is left after the last sweep has contracted once more.  Measured against 64-bit references
+// at 10k to 2M rows: 1.1e-16 in norm (the exact kernels: 1.1e-16 to 1.6e-16) and at most 1e-15 of the
+// root mean square, with bounds of 2^-52 to 2^-49 alike.  (Waiting for equal bits takes the sweeps of the
+// slowest rounding flip: twice as many.)
+//
+// Sweep order.  Each warp owns a contiguous run of rows and walks it upwards from its bottom, 32 rows
+// a tile (lane per row; 32 / NC rows for NC right-hand sides), writing x in place: a row sees this
+// sweep's values of everything below it in the run, so only columns inside the tile, across the run's
+// lower edge and far away are one sweep old.  Those inside the tile are a quarter of a 64-column band
+// and cost the most sweeps, so with one right-hand side a tile's changes are folded in once more
+// before they are written (k_settle, "second look"): half the sweeps for a third more arithmetic.
+//
+// Bound by the FP64 pipe (57 % active by ncu at 500k rows; 2 FMAs a clock and SM, and a tile takes its
+// longest row's count: 1.9 times the mean of 7.6 off-diagonals) and, below ~200k rows, by the chain of
+// loads and FMAs through a tile.  Measured on GB300, 8.8 entries a row: 2M rows 68 -> 3.1 ms (24
+// sweeps), 200k rows 6.9 -> 0.60 ms (31), 50k rows 1.7 -> 0.42 ms (28); 200k rows x 8 columns 70 ->
+// 1.95 ms (33).
+//
+// One cooperative launch runs all sweeps, with a grid barrier after each; x of other warps' rows may
+// be read old or new within a sweep, and is new after the barrier.
+#include <algorithm>
+#include <cmath>
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace sptrsv {
+
+constexpr int kSetWarps = 8;
+constexpr size_t kSetSmem = 220 * 1024;
+// Tiles of the shortest run: longer runs take fewer sweeps (fewer rows see a neighbour's old values),
+// shorter ones spread further: 10k rows 325 / 392 / 514 us at 1 / 2 / 4 tiles, 60k rows x 16 columns
+// 1776 / 1538 / 1586 us.
+constexpr int kSetMinTiles = 2;
+constexpr int kSetPending = 5000;  // offset of a sweep's record: 0 = nothing changed
+constexpr int kSetStill = kSetPending - 51;  // changes below 2^-50 (the exponents are floors)
+
+struct SettleArgs {
+    int n, rhs;
+    const int* rp;
+    const int* col;
+    const double* val;
+    const double* invd;
+    const double* b;
+    double* x;
+    Ctl* ctl;
+    int* worst;  // kSettleSweeps records: the largest change of each sweep, as an exponent
+    int64_t budget;
+    int tiles;  // tiles per warp
+    int cap;    // staged entries of a tile; a tile with more is read from global memory
+};
+
+template <int NC> struct SetShape {
+    static constexpr int kRows = 32 / NC;  // rows of a tile
+};
+
+// Bytes of a warp's buffers: two tiles of `cap` staged entries (columns and values), one tile's x at
+// every entry (cap * NC), the tile's changes.
+__host__ __device__ __forceinline__ size_t set_warp_bytes(int cap, int nc) {
+    return (size_t)cap * (2 * 12 + 8 * nc) + 32 * 8;
+}
+
+__device__ __forceinline__ int d_exp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+
+// After sweep p (from 0): whether to leave the matrix to the exact kernel.  From the ninth sweep on the
+// largest change has to lose at least a bit a sweep over the last four, until it is within 2^-40 of
+// its row's size, where single rows decide it.
+__device__ __forceinline__ bool settle_hopeless(const int* worst, int p) {
+    if (p < 8) return false;
+    const int now = ld_relaxed(worst + p), then = ld_relaxed(worst + p - 4);
+    return now > kSetPending - 40 && now > then - 4;
+}
+
+__device__ __forceinline__ void set_cp4(void* s, const void* g) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(s);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(a), "l"(g) : "memory");
+}
+__device__ __forceinline__ void set_cp8(void* s, const void* g) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(s);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(g) : "memory");
+}
+
+// x changes within the launch, so never the read-only path: a warp's own run through L1 (its stores
+// update it), other rows from L2, where this sweep's values are.
+__device__ __forceinline__ double set_ld(const double* p, bool own) {
+    double v;
+    if (own) asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    else asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+
+template <int NC>
+__global__ void __launch_bounds__(kSetWarps * 32, 2) k_settle(SettleArgs A) {
+    constexpr int R = SetShape<NC>::kRows;
+    extern __shared__ __align__(16) char set_smem[];
+    __shared__ int s_worst;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = lane / NC, j0 = lane % NC;
+    const int n = A.n, m = A.rhs, cap = A.cap;
+    char* base = set_smem + warp * set_warp_bytes(cap, NC);
+    double* sv = (double*)base;            // [2][cap] values
+    double* sx = sv + 2 * cap;             // [cap][NC] x at the tile's entries
+    double* dl = sx + cap * NC;            // [32] the tile's changes
+    int* sc = (int*)(dl + 32);             // [2][cap] columns
+    const int ntiles = (n + R - 1) / R;
+    const int t0 = min((int)(blockIdx.x * kSetWarps + warp) * A.tiles, ntiles), t1 = min(t0 + A.tiles, ntiles);
+    const int run_top = n - R * t0;
+
+    // x = D^-1 b
+    for (int t = t0; t < t1; ++t) {
+        const int top = n - R * t, lo = max(0, top - R), i = lo + r;
+        if (i < top)
+            for (int j = j0; j < m; j += NC) A.x[(size_t)i * m + j] = A.b[(size_t)i * m + j] * A.invd[i];
+    }
+    if (!grid_barrier(A.ctl, gridDim.x, A.budget)) return;
+
+    struct Rows { int e0, e1, s, e; };
+    auto rows_of = [&](int t) {
+        Rows q{0, 0, 0, 0};
+        if (t < t1) {
+            const int top = n - R * t, lo = max(0, top - R);
+            q.e0 = A.rp[lo];
+            q.e1 = A.rp[top];
+            if (lo + r < top) {
+                q.s = A.rp[lo + r] + 1;
+                q.e = A.rp[lo + r + 1];
+            }
+        }
+        return q;
+    };
+    auto stage = [&](const Rows& q, int buf) {
+        const int cnt = q.e1 - q.e0;
+        if (cnt <= cap)
+            for (int k = lane; k < cnt; k += 32) {
+                set_cp4(sc + buf * cap + k, A.col + q.e0 + k);
+                set_cp8(sv + buf * cap + k, A.val + q.e0 + k);
+            }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+
+    for (int p = 0; p < kSettleSweeps; ++p) {
+        if (threadIdx.x == 0) s_worst = 0;
+        __syncthreads();
+        int worst = 0;
+        Rows cur = rows_of(t0);
+        stage(cur, 0);
+        Rows nxt = rows_of(t0 + 1);
+        for (int t = t0; t < t1; ++t) {
+            const int buf = (t - t0) & 1;
+            const int top = n - R * t, lo = max(0, top - R), i = lo + r;
+            stage(nxt, buf ^ 1);
+            const Rows after = rows_of(t + 2);
+            const bool staged = cur.e1 - cur.e0 <= cap;
+            const double* pv = sv + buf * cap - cur.e0;
+            const int* pc = sc + buf * cap - cur.e0;
+            const double di = i < top ? A.invd[i] : 0.0;
+            for (int jb = 0; jb < m; jb += NC) {
+                const int j = jb + j0;
+                const bool mine = i < top && j < m;
+                const size_t at = mine ? (size_t)i * m + j : 0;
+                // the row's sum apart from b_i: its roundings are those of the smaller terms
+                double acc = 0.0, bi = 0.0, old = 0.0;
+                if (mine) {
+                    bi = A.b[at];
+                    old = set_ld(A.x + at, true);
+                }
+                const int eb = d_exp(bi);
+                if (jb == 0) {
+                    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+                    __syncwarp();
+                }
+                if (staged) {
+                    // x at every entry, all of a lane's loads in flight together (a diagonal's is not used)
+                    const int cnt = (cur.e1 - cur.e0) * NC;
+                    for (int q0 = 0; q0 < cnt; q0 += 32 * 8) {
+                        double xv[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const int q = q0 + lane + 32 * u;
+                            if (q < cnt) {
+                                const int c = sc[buf * cap + q / NC];
+                                if (jb + q % NC < m) xv[u] = set_ld(A.x + (size_t)c * m + jb + q % NC, c < run_top);
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const int q = q0 + lane + 32 * u;
+                            if (q < cnt) sx[q] = xv[u];
+                        }
+                    }
+                    __syncwarp();
+                }
+                unsigned em = 0;  // largest sum of the exponents of a term's factors, in the exponent's place
+                int inside = 0;   // entries with their column in this tile
+                if (mine) {
+                    const double* px = sx - (size_t)cur.e0 * NC + j0;
+                    for (int k = cur.s; k < cur.e; ++k) {
+                        const int c = staged ? pc[k] : __ldg(A.col + k);
+                        const double v = staged ? pv[k] : __ldg(A.val + k);
+                        const double xv = staged ? px[(size_t)k * NC] : set_ld(A.x + (size_t)c * m + j, c < run_top);
+                        acc = fma(v, xv, acc);
+                        em = max(em, ((unsigned)__double2hiint(v) & 0x7ff00000u) +
+                                         ((unsigned)__double2hiint(xv) & 0x7ff00000u));
+                        inside += c < top;
+                    }
+                }
+                double y = (bi - acc) * di;
+                if constexpr (NC == 1) {
+                    // second look: the tile's own changes, once
+                    // (no change is zero for infinities too)
+                    dl[lane] = mine && __double_as_longlong(y) != __double_as_longlong(old) ? y - old : 0.0;
+                    __syncwarp();
+                    if (mine) {
+                        for (int k = cur.s; inside > 0; ++k) {
+                            const int c = staged ? pc[k] : __ldg(A.col + k);
+                            if (c < top) {
+                                acc = fma(staged ? pv[k] : __ldg(A.val + k), dl[c - lo], acc);
+                                --inside;
+                            }
+                        }
+                        y = (bi - acc) * di;
+                    }
+                }
+                if (mine && __double_as_longlong(y) != __double_as_longlong(old)) {
+                    const int ei = d_exp(di) - 1023;
+                    const int size = max(d_exp(y), max(eb, (int)(em >> 20) - 1023) + ei);
+                    const int gap = d_exp(y - old) - size;
+                    worst = max(worst, gap + kSetPending);
+                    A.x[at] = y;
+                }
+                __syncwarp();  // sx and dl are read before they are written again
+            }
+            __syncwarp();  // the staged entries are read, the tile's x written, before the next tile
+            cur = nxt;
+            nxt = after;
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        worst = __reduce_max_sync(0xffffffffu, worst);
+        if (lane == 0 && worst > 0) atomicMax(&s_worst, worst);
+        __syncthreads();
+        if (threadIdx.x == 0 && s_worst > 0) atomicMax(A.worst + p, s_worst);
+        if (!grid_barrier(A.ctl, gridDim.x, A.budget)) return;
+        if (ld_relaxed(A.worst + p) <= kSetStill) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                A.ctl->done = 1;
+                A.ctl->steps = p + 1;
+            }
+            return;
+        }
+        if (settle_hopeless(A.worst, p)) return;
+    }
+}
+
+// Prepares the exact kernel behind k_settle: x pending when it has to run, no row left to claim when
+// it has not.
+__global__ void k_settle_gate(double* x, size_t count, Ctl* ctl) {
+    if (*(volatile const int*)&ctl->done) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->ticket = 0xF0000000u;
+        return;
+    }
+    const double v = Pend<double>::value();
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) x[k] = v;
+}
+
+template <int NC>
+static int settle_t(const SolveArgs& a, int* worst) {
+    constexpr int R = SetShape<NC>::kRows;
+    // staged entries: the mean tile and four deviations of a Poisson count, if shared memory holds it
+    const double mean = R * (double)a.nnz / a.n;
+    const int fit = (int)((kSetSmem / kSetWarps - 256) / (24 + 8 * NC));
+    const int cap = std::min(fit, (int)(mean + 4.0 * std::sqrt(mean)) + 15) / 8 * 8;
+    const size_t bytes = kSetWarps * set_warp_bytes(cap, NC);
+    const void* fn = (const void*)k_settle<NC>;
+    CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    int per_sm = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSetWarps * 32, bytes));
+    if (per_sm < 1) return SPTRSV_ERR_UNSUPPORTED;
+    const int ntiles = (a.n + R - 1) / R;
+    const int warps = std::max(1, std::min(per_sm * a.sm_count * kSetWarps, ntiles / kSetMinTiles));
+    SettleArgs s{a.n, a.rhs, a.rp, a.col, (const double*)a.val, (const double*)a.invd, (const double*)a.b, (double*)a.x,
+                 a.ctl, worst, a.budget, (ntiles + warps - 1) / warps, cap};
+    const int grid = ((ntiles + s.tiles - 1) / s.tiles + kSetWarps - 1) / kSetWarps;
+    void* args[] = {(void*)&s};
+    CUDA_TRY(cudaLaunchCooperativeKernel(fn, grid, kSetWarps * 32, args, bytes, a.st));
+    ++*a.launches;
+    return 0;
+}
+
+// `worst`: kSettleSweeps ints of device memory.
+int launch_settle(const SolveArgs& a, int* worst) {
+    CUDA_TRY(cudaMemsetAsync(worst, 0, sizeof(int) * kSettleSweeps, a.st));
+    int rc;
+    if (a.rhs == 1) rc = settle_t<1>(a, worst);
+    else if (a.rhs == 2) rc = settle_t<2>(a, worst);
+    else if (a.rhs <= 4) rc = settle_t<4>(a, worst);
+    else if (a.rhs <= 8) rc = settle_t<8>(a, worst);
+    else if (a.rhs <= 16) rc = settle_t<16>(a, worst);
+    else rc = settle_t<32>(a, worst);
+    if (rc) return rc;
+    const size_t count = (size_t)a.n * a.rhs;
+    k_settle_gate<<<(int)std::min<size_t>((count + 255) / 256, 2048), 256, 0, a.st>>>((double*)a.x, count, a.ctl);
+    ++*a.launches;
+    CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
+}  // namespace sptrsv
