@@ -13,84 +13,182 @@
 //    level into num_threads tasks, one device thread per level, same integer arithmetic.
 //  * CSR -> CSC transpose (utils.cpp:128-159): stable radix sort of the entries by column,
 //    so each column lists its rows in ascending order and the diagonal lands last.
+#include <algorithm>
 #include "common.cuh"
 #include "kernels.cuh"
 
 namespace sptrsv {
-
-__global__ void k_validate(int n, int nnz, const int* __restrict__ rp, const int* __restrict__ col,
-                           const double* __restrict__ val, int* __restrict__ in_degree, double* __restrict__ invd,
-                           float* __restrict__ invd32, Ctl* ctl) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int s = rp[i], e = rp[i + 1];
-        if ((i == 0 && s != 0) || e < s || e > nnz || s < 0) {
-            record_error(ctl, SPTRSV_ERR_ROW_PTR);
-            in_degree[i] = 0;
-            continue;
-        }
-        in_degree[i] = e - s;
-        if (e == s || col[s] != i) {
-            record_error(ctl, SPTRSV_ERR_MISSING_DIAG);
-            continue;
-        }
-        const double d = val[s];
-        if (d == 0.0 || !isfinite(d)) record_error(ctl, SPTRSV_ERR_ZERO_PIVOT);
-        invd[i] = 1.0 / d;
-        invd32[i] = (float)(1.0 / d);
-        for (int k = s + 1; k < e; ++k) {
-            const int c = col[k];
-            if (c < 0 || c >= n) { record_error(ctl, SPTRSV_ERR_COL_RANGE); break; }
-            if (c <= i) { record_error(ctl, SPTRSV_ERR_NOT_UPPER); break; }
-        }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && rp[n] != nnz) record_error(ctl, SPTRSV_ERR_ROW_PTR);
-}
 
 __global__ void k_to_f32(size_t count, const double* __restrict__ a, float* __restrict__ b) {
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x)
         b[k] = (float)a[k];
 }
 
-// Per-row dominance ratio sum_j |U_ij| / |U_ii| (reduced to its maximum) and the sum of
-// squared row lengths, used to choose schedules.
-// Per-matrix statistics: max_i sum|off| / |diag|, sum of squared row lengths, the sum over rows
-// of 1 / (distance to the row's nearest dependency), which is about the depth of the DAG when
-// dependencies chain through their nearest columns (the levels themselves take a DAG traversal),
-// and the number of rows that are not one contiguous column range from the diagonal (zero for a
-// banded factor stored with its explicit zeros: a skyline matrix).
-__global__ void k_row_stats(int n, const int* __restrict__ rp, const int* __restrict__ col,
-                            const double* __restrict__ val, unsigned long long* max_ratio_bits,
-                            unsigned long long* sum_len2, double* depth_sum, unsigned long long* gapped_rows) {
-    double mr = 0.0, dep = 0.0;
-    unsigned long long l2 = 0, gapped = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int s = rp[i], e = rp[i + 1];
-        double off = 0.0;
-        int near = n;
-        bool contiguous = true;
-        for (int k = s + 1; k < e; ++k) {
-            off += fabs(val[k]);
-            near = min(near, col[k] - i);
-            contiguous &= col[k] == i + (k - s);
+// The checks, the reciprocal diagonal and the matrix's statistics in one pass over U:
+//   stats[0] max_i sum_j |U_ij| / |U_ii| (bits), stats[1] sum of squared row lengths, stats[2] the sum
+//   over rows of 1 / (distance to the row's nearest dependency), which is about the depth of the DAG
+//   when dependencies chain through their nearest columns (the levels themselves take a DAG traversal),
+//   stats[3] the number of rows that are not one contiguous column range from the diagonal (zero for a
+//   banded factor stored with its explicit zeros: a skyline matrix).
+// Rows go 32 a tile.  Short ones (kLong = false): a warp per tile copies the tile's entries to shared
+// memory in order and each lane walks its own row there.  Long ones (mean above kRowsLong): a block of
+// eight warps per tile, each walking four rows, 32 entries a step.  Either way one lane finishes each
+// row: divisions are FP64 chains of ~10 operations at 2 a clock and SM, so a row makes one (its
+// reciprocal) and a lane one more at its end (the ratio of its worst row).  Measured on GB300 against
+// separate passes of a lane per row: 500k rows of 8.8 entries 64 -> 41 us (bound by the FP64 sums and
+// divisions), the 20^3 dissection factor (8,000 rows of 185 entries) 368 -> 31 us.
+constexpr int kRowsWarps = 4, kRowsCap = 512, kRowsLongWarps = 8;
+constexpr double kRowsLong = 14.0;  // tiles of longer rows would not fit kRowsCap
+
+// What a walk finds out about a row.
+struct RowFacts {
+    double off = 0.0;  // sum of the off-diagonals' sizes
+    int near;          // distance to the nearest column
+    bool contiguous = true;
+    int err = 0;
+};
+
+__device__ __forceinline__ void look(RowFacts& f, int n, int row, int at, int c, double v) {
+    if (!f.err) {
+        if (c < 0 || c >= n) f.err = SPTRSV_ERR_COL_RANGE;
+        else if (c <= row) f.err = SPTRSV_ERR_NOT_UPPER;
+    }
+    f.near = min(f.near, c - row);
+    f.contiguous &= c == row + at;
+    f.off += fabs(v);
+}
+
+template <bool kLong>
+__global__ void __launch_bounds__((kLong ? kRowsLongWarps : kRowsWarps) * 32)
+k_check_rows(int n, int nnz, const int* __restrict__ rp, const int* __restrict__ col, const double* __restrict__ val,
+             int* __restrict__ in_degree, double* __restrict__ invd, float* __restrict__ invd32,
+             unsigned long long* stats, Ctl* ctl) {
+    constexpr int W = kLong ? kRowsLongWarps : kRowsWarps;
+    __shared__ int s_col[kLong ? 1 : W][kRowsCap];
+    __shared__ double s_val[kLong ? 1 : W][kRowsCap];
+    __shared__ struct { double off; int near; bool contiguous; int err; } s_row[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double worst = 0.0, worst_off = 0.0, worst_d = 1.0;  // the lane's row of the largest off / |d|
+    float depth = 0.f;
+    unsigned long long len2 = 0, gapped = 0;
+    const int first = kLong ? blockIdx.x : blockIdx.x * W + w, step = kLong ? gridDim.x : gridDim.x * W;
+    for (int t = first; (long long)t * 32 < n; t += step) {
+        const int r0 = t * 32, i = r0 + lane;
+        const bool owner = !kLong || w == 0;  // the warp that finishes the tile's rows
+        int s = 0, e = 0, bad = 0;
+        if (i < n) {
+            s = rp[i];
+            e = rp[i + 1];
+            if ((i == 0 && s != 0) || e < s || e > nnz || s < 0) bad = SPTRSV_ERR_ROW_PTR;
+            if (owner) in_degree[i] = bad ? 0 : e - s;
         }
-        const double r = off / fabs(val[s]);
-        mr = fmax(mr, r);
-        if (e > s + 1) dep += 1.0 / (double)near;
-        gapped += contiguous ? 0ull : 1ull;
-        l2 += (unsigned long long)(e - s) * (unsigned long long)(e - s);
+        if (__any_sync(0xffffffffu, bad)) {  // no entry of these rows is read (every warp of a block agrees)
+            if (bad && owner) record_error(ctl, bad);
+            continue;
+        }
+        RowFacts f;
+        f.near = n;
+        double d = 1.0;
+        if constexpr (kLong) {
+            for (int q = w; q < min(32, n - r0); q += W) {
+                const int rs = __shfl_sync(0xffffffffu, s, q), re = __shfl_sync(0xffffffffu, e, q), row = r0 + q;
+                RowFacts g;
+                g.near = n;
+#pragma unroll 4
+                for (int k = rs + 1 + lane; k < re; k += 32) look(g, n, row, k - rs, col[k], val[k]);
+                g.off = warp_sum(g.off);
+                g.near = __reduce_min_sync(0xffffffffu, g.near);
+                const bool all = __all_sync(0xffffffffu, g.contiguous);
+                g.err = __reduce_min_sync(0xffffffffu, g.err);  // statuses are negative
+                if (lane == 0) {
+                    s_row[q].off = g.off;
+                    s_row[q].near = g.near;
+                    s_row[q].contiguous = all;
+                    s_row[q].err = g.err;
+                }
+            }
+            __syncthreads();
+            if (owner && i < n) {
+                f.off = s_row[lane].off;
+                f.near = s_row[lane].near;
+                f.contiguous = s_row[lane].contiguous;
+                f.err = s_row[lane].err;
+                if (e == s || col[s] != i) f.err = SPTRSV_ERR_MISSING_DIAG;
+                else d = val[s];
+            }
+            __syncthreads();
+        } else {
+            const int E0 = __shfl_sync(0xffffffffu, s, 0), E1 = __shfl_sync(0xffffffffu, e, min(31, n - 1 - r0));
+            const bool staged = E1 - E0 <= kRowsCap;
+            if (staged)
+                for (int q = lane; q < E1 - E0; q += 32) {
+                    s_col[w][q] = col[E0 + q];
+                    s_val[w][q] = val[E0 + q];
+                }
+            __syncwarp();
+            const int* c = staged ? s_col[w] - E0 : col;
+            const double* v = staged ? s_val[w] - E0 : val;
+            if (i < n) {
+                if (e == s || c[s] != i) f.err = SPTRSV_ERR_MISSING_DIAG;
+                else {
+                    d = v[s];
+                    for (int k = s + 1; k < e; ++k) look(f, n, i, k - s, c[k], v[k]);
+                }
+            }
+            __syncwarp();
+        }
+        if (!owner || i >= n) continue;
+        if (f.err != SPTRSV_ERR_MISSING_DIAG && (d == 0.0 || !isfinite(d))) f.err = SPTRSV_ERR_ZERO_PIVOT;
+        if (f.err) {
+            record_error(ctl, f.err);
+            continue;
+        }
+        const double inv = 1.0 / d;
+        invd[i] = inv;
+        invd32[i] = (float)inv;
+        const double r = f.off * fabs(inv);
+        if (r > worst) {
+            worst = r;
+            worst_off = f.off;
+            worst_d = fabs(d);
+        }
+        if (e > s + 1) depth += 1.f / (float)f.near;
+        gapped += f.contiguous ? 0ull : 1ull;
+        len2 += (unsigned long long)(e - s) * (unsigned long long)(e - s);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        mr = fmax(mr, __shfl_xor_sync(0xffffffffu, mr, o));
-        dep += __shfl_xor_sync(0xffffffffu, dep, o);
-        l2 += __shfl_xor_sync(0xffffffffu, l2, o);
-        gapped += __shfl_xor_sync(0xffffffffu, gapped, o);
+    __syncwarp();
+    if (!kLong || w == 0) {
+        double mr = worst_off / worst_d, dep = (double)depth;
+        for (int o = 16; o > 0; o >>= 1) {
+            mr = fmax(mr, __shfl_xor_sync(0xffffffffu, mr, o));
+            dep += __shfl_xor_sync(0xffffffffu, dep, o);
+            len2 += __shfl_xor_sync(0xffffffffu, len2, o);
+            gapped += __shfl_xor_sync(0xffffffffu, gapped, o);
+        }
+        if (lane == 0) {
+            atomicMax(stats, (unsigned long long)__double_as_longlong(mr));  // mr >= 0: bit order = value order
+            atomicAdd(stats + 1, len2);
+            atomicAdd(reinterpret_cast<double*>(stats + 2), dep);
+            atomicAdd(stats + 3, gapped);
+        }
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(max_ratio_bits, (unsigned long long)__double_as_longlong(mr));  // mr >= 0: bit order = value order
-        atomicAdd(sum_len2, l2);
-        atomicAdd(depth_sum, dep);
-        atomicAdd(gapped_rows, gapped);
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0 && rp[n] != nnz) record_error(ctl, SPTRSV_ERR_ROW_PTR);
+}
+
+int launch_check_rows(int n, int nnz, const int* rp, const int* col, const double* val, int* in_degree, double* invd,
+                      float* invd32, unsigned long long* stats, Ctl* ctl, int sm_count, cudaStream_t st,
+                      int64_t* launches) {
+    CUDA_TRY(cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), st));
+    const int tiles = (n + 31) / 32;
+    if ((double)nnz > kRowsLong * n)
+        k_check_rows<true><<<std::min(tiles, sm_count * 8), kRowsLongWarps * 32, 0, st>>>(n, nnz, rp, col, val, in_degree,
+                                                                                       invd, invd32, stats, ctl);
+    else
+        k_check_rows<false><<<std::min((tiles + kRowsWarps - 1) / kRowsWarps, sm_count * 8), kRowsWarps * 32, 0, st>>>(
+            n, nnz, rp, col, val, in_degree, invd, invd32, stats, ctl);
+    ++*launches;
+    CUDA_TRY(cudaGetLastError());
+    return 0;
 }
 
 // levels: warp per row, rows claimed in reverse order through ctl->ticket2.
@@ -227,17 +325,16 @@ int scan_partials_needed(int count) { return (count + kScanTile - 1) / kScanTile
 
 // ---------------------------------------------------------------------------------------
 // Stable LSD radix sort of (key, idx) pairs, 8-bit digits; one warp per tile, tiles in order.
-constexpr int kRadixTile = 4096;  // items per warp-tile
 constexpr int kRadixWarps = 4;    // warps per block
 
-__global__ void k_radix_hist(const unsigned* __restrict__ keys, int count, int shift, int ntiles, int* __restrict__ hist) {
+__global__ void k_radix_hist(const unsigned* __restrict__ keys, int count, int shift, int ntiles, int per, int* __restrict__ hist) {
     __shared__ int cnt[kRadixWarps][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int tile = blockIdx.x * kRadixWarps + w;
     for (int d = lane; d < 256; d += 32) cnt[w][d] = 0;
     __syncwarp();
     if (tile < ntiles) {
-        const int beg = tile * kRadixTile, end = min(count, beg + kRadixTile);
+        const int beg = tile * per, end = min(count, beg + per);
         for (int k = beg + lane; k < end; k += 32) atomicAdd(&cnt[w][(keys[k] >> shift) & 255u], 1);
     }
     __syncwarp();
@@ -246,7 +343,7 @@ __global__ void k_radix_hist(const unsigned* __restrict__ keys, int count, int s
 }
 
 __global__ void k_radix_scatter(const unsigned* __restrict__ keys, const int* __restrict__ idx, int count, int shift,
-                                int ntiles, const int* __restrict__ offs, unsigned* __restrict__ keys_out,
+                                int ntiles, int per, const int* __restrict__ offs, unsigned* __restrict__ keys_out,
                                 int* __restrict__ idx_out) {
     __shared__ int cnt[kRadixWarps][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -254,7 +351,7 @@ __global__ void k_radix_scatter(const unsigned* __restrict__ keys, const int* __
     if (tile >= ntiles) return;
     for (int d = lane; d < 256; d += 32) cnt[w][d] = offs[d * ntiles + tile];
     __syncwarp();
-    const int beg = tile * kRadixTile, end = min(count, beg + kRadixTile);
+    const int beg = tile * per, end = min(count, beg + per);
     const unsigned lt = (1u << lane) - 1u;
     for (int k0 = beg; k0 < end; k0 += 32) {
         const int k = k0 + lane;
@@ -277,13 +374,23 @@ __global__ void k_radix_scatter(const unsigned* __restrict__ keys, const int* __
     }
 }
 
+// Items of a warp's tile: a warp takes them 32 at a time in order, so a long tile is a long chain (4,096
+// items 88 us a pass on GB300 whatever the count), a short one costs 1 KB of histogram to scan.  Enough
+// tiles for 16 warps an SM, between 256 items (500k keys: 88 -> 13 us) and 4,096.
+static int radix_tile(int count) { return std::min(4096, std::max(256, (count / (152 * 16) + 255) / 256 * 256)); }
+
+// Scratch bytes of a sort of `count` keys.
+size_t sort_scratch(int count) {
+    const int per = radix_tile(count), ntiles = (count + per - 1) / per;
+    return ((size_t)3 * count + (size_t)256 * ntiles + 1 + scan_partials_needed(256 * ntiles)) * sizeof(int) + 8 * 256;
+}
+
 // Sorts keys (count items, values < 2^key_bits) stably; writes the permutation into
-// perm (perm[p] = original index of the p-th smallest).  Needs scratch:
-// 2*count unsigned/int + 256*ntiles + scan partials.
+// perm (perm[p] = original index of the p-th smallest).  Takes sort_scratch(count) bytes of scratch.
 int stable_sort_perm(const unsigned* keys_in, int count, int key_bits, int* perm, Scratch& scr, cudaStream_t st,
                      int64_t* launches) {
     if (count <= 0) return 0;
-    const int ntiles = (count + kRadixTile - 1) / kRadixTile;
+    const int per = radix_tile(count), ntiles = (count + per - 1) / per;
     const int nblocks = (ntiles + kRadixWarps - 1) / kRadixWarps;
     unsigned* ka = scr.take<unsigned>(count);
     unsigned* kb = scr.take<unsigned>(count);
@@ -301,13 +408,13 @@ int stable_sort_perm(const unsigned* keys_in, int count, int key_bits, int* perm
     int* iouts[2] = {(passes % 2 == 1) ? ib : ia, (passes % 2 == 1) ? ia : ib};
     for (int p = 0; p < passes; ++p) {
         const int shift = 8 * p;
-        k_radix_hist<<<nblocks, 32 * kRadixWarps, 0, st>>>(kin, count, shift, ntiles, hist);
+        k_radix_hist<<<nblocks, 32 * kRadixWarps, 0, st>>>(kin, count, shift, ntiles, per, hist);
         ++*launches;
         int rc = scan_exclusive(hist, hist, hist_n, part, st, launches);
         if (rc) return rc;
         unsigned* ko = kouts[p & 1];
         int* io = iouts[p & 1];
-        k_radix_scatter<<<nblocks, 32 * kRadixWarps, 0, st>>>(kin, iin, count, shift, ntiles, hist, ko, io);
+        k_radix_scatter<<<nblocks, 32 * kRadixWarps, 0, st>>>(kin, iin, count, shift, ntiles, per, hist, ko, io);
         ++*launches;
         kin = ko;
         iin = io;

@@ -84,6 +84,7 @@ void Handle::drop_matrix() {
     levels_ready = false;
     have_csc = false;
     have_offdiag = false;
+    have_val32 = false;
     have_supernodes = false;
     auto_supernodes = false;
     skyline = false;
@@ -101,27 +102,15 @@ int Handle::analyse() {
     if ((rc = in_degree.ensure(sizeof(int) * (size_t)n))) return rc;
     if ((rc = invd.ensure(sizeof(double) * (size_t)n))) return rc;
     if ((rc = invd32.ensure(sizeof(float) * (size_t)n))) return rc;
-    if ((rc = val32.ensure(sizeof(float) * (size_t)nnz))) return rc;
     if ((rc = levels.ensure(sizeof(int) * (size_t)n))) return rc;
     if ((rc = stats.ensure(4 * sizeof(unsigned long long)))) return rc;
-    const int sgrid = sm_count * 4;
-    k_validate<<<sgrid, 256, 0, st>>>(n, nnz, rp, col, val, in_degree.as<int>(), invd.as<double>(),
-                                      invd32.as<float>(), ctl);
-    ++launches;
-    CUDA_TRY(cudaGetLastError());
-    if ((rc = read_ctl(&c))) return rc;
-    if (c.status) return c.status;
-    k_to_f32<<<sgrid, 256, 0, st>>>((size_t)nnz, val, val32.as<float>());
-    CUDA_TRY(cudaMemsetAsync(stats.p, 0, 4 * sizeof(unsigned long long), st));
-    k_row_stats<<<sgrid, 256, 0, st>>>(n, rp, col, val, stats.as<unsigned long long>(),
-                                       stats.as<unsigned long long>() + 1,
-                                       reinterpret_cast<double*>(stats.as<unsigned long long>() + 2),
-                                       stats.as<unsigned long long>() + 3);
-    launches += 2;
-    CUDA_TRY(cudaGetLastError());
+    if ((rc = launch_check_rows(n, nnz, rp, col, val, in_degree.as<int>(), invd.as<double>(), invd32.as<float>(),
+                                stats.as<unsigned long long>(), ctl, sm_count, st, &launches)))
+        return rc;
     unsigned long long hs[4];
     CUDA_TRY(cudaMemcpyAsync(hs, stats.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    if ((rc = read_ctl(&c))) return rc;
+    if (c.status) return c.status;
     double mr;
     memcpy(&mr, &hs[0], sizeof(double));
     max_ratio = mr;
@@ -182,8 +171,7 @@ int Handle::ensure_levels() {
     // level buckets: counts -> level_ptr; stable radix sort of level keys -> level_rows
     if ((rc = level_ptr.ensure(sizeof(int) * (size_t)(max_level + 2)))) return rc;
     if ((rc = level_rows.ensure(sizeof(int) * (size_t)n))) return rc;
-    const size_t need = (size_t)4 * n * sizeof(int) + (size_t)(max_level + 2) * sizeof(int) +
-                        (size_t)256 * ((n + 4095) / 4096 + 1) * sizeof(int) * 2 + (1 << 20);
+    const size_t need = sort_scratch(n) + (size_t)(max_level + 2 + scan_partials_needed(max_level + 1)) * sizeof(int) + 4096;
     if ((rc = scratch.ensure(need))) return rc;
     Scratch scr{(char*)scratch.p, scratch.cap, 0};
     int* cnt = scr.take<int>(max_level + 2);
@@ -219,8 +207,7 @@ int Handle::build_csc() {
     if ((rc = csc_ptr.ensure(sizeof(int) * (size_t)(n + 1)))) return rc;
     if ((rc = csc_row.ensure(sizeof(int) * (size_t)nnz))) return rc;
     if ((rc = csc_val.ensure(sizeof(double) * (size_t)nnz))) return rc;
-    const size_t need = (size_t)5 * nnz * sizeof(int) + (size_t)(n + 2) * sizeof(int) +
-                        (size_t)256 * ((nnz + 4095) / 4096 + 1) * sizeof(int) * 2 + (1 << 20);
+    const size_t need = sort_scratch(nnz) + ((size_t)2 * nnz + n + 2 + scan_partials_needed(n)) * sizeof(int) + 4096;
     if ((rc = scratch.ensure(need))) return rc;
     Scratch scr{(char*)scratch.p, scratch.cap, 0};
     int* erow = scr.take<int>(nnz);
@@ -359,6 +346,15 @@ int Handle::prepare(const sptrsv_opts& o, int rhs, int layout) {
     if (o.precision == SPTRSV_PREC_MIXED) {
         if (o.inner == SPTRSV_SCHED_JACOBI && rhs == 1)
             if ((rc = ensure_offdiag())) return rc;
+        if (!have_val32 && !(o.inner == SPTRSV_SCHED_JACOBI && rhs == 1 && mean_len <= kShortRowLen)) {
+            // the FP32 values, where the inner solve reads them (the Jacobi sweeps of one right-hand side
+            // on short rows have their own layout)
+            if ((rc = val32.ensure(sizeof(float) * (size_t)nnz))) return rc;
+            k_to_f32<<<sm_count * 4, 256, 0, st>>>((size_t)nnz, val, val32.as<float>());
+            ++launches;
+            CUDA_TRY(cudaGetLastError());
+            have_val32 = true;
+        }
         if ((rc = grow(r32, sizeof(float) * nr))) return rc;
         if ((rc = grow(d32a, sizeof(float) * nr))) return rc;
         if ((rc = grow(d32b, sizeof(float) * nr))) return rc;

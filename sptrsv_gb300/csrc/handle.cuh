@@ -122,6 +122,7 @@ struct Handle {
     long long sn_prows = 0;
     bool have_supernodes = false;
     bool have_offdiag = false;
+    bool have_val32 = false;  // val32 holds the FP32 values (built when a mixed solve reads them)
 
     // work
     DevBuf scratch, settle, xw, bw, r32, d32a, d32b, norms, indeg_work, left, db, dx, flush;

@@ -26,12 +26,10 @@ struct Scratch {
 __global__ void k_narrow_rp(int count, const int64_t* in, int* out, Ctl* ctl);
 
 // analysis.cu
-__global__ void k_validate(int n, int nnz, const int* rp, const int* col, const double* val, int* in_degree,
-                           double* invd, float* invd32, Ctl* ctl);
+int launch_check_rows(int n, int nnz, const int* rp, const int* col, const double* val, int* in_degree, double* invd,
+                      float* invd32, unsigned long long* stats, Ctl* ctl, int sm_count, cudaStream_t st,
+                      int64_t* launches);
 __global__ void k_to_f32(size_t count, const double* a, float* b);
-__global__ void k_row_stats(int n, const int* rp, const int* col, const double* val,
-                            unsigned long long* max_ratio_bits, unsigned long long* sum_len2, double* depth_sum,
-                            unsigned long long* gapped_rows);
 __global__ void k_levels(int n, const int* rp, const int* col, int* level, Ctl* ctl, int64_t budget);
 __global__ void k_level_hist(int n, const int* level, int* cnt);
 __global__ void k_level_tasks(int max_level, const int* lptr, const int* lrows, const int* rp, int T, int* tasks);
@@ -44,6 +42,7 @@ __global__ void k_validate_csc(int n, int nnz, const int* cp, const int* crow, c
                                Ctl* ctl);
 int scan_exclusive(const int* in, int* out, int count, int* part_scratch, cudaStream_t st, int64_t* launches);
 int scan_partials_needed(int count);
+size_t sort_scratch(int count);
 int stable_sort_perm(const unsigned* keys_in, int count, int key_bits, int* perm, Scratch& scr, cudaStream_t st,
                      int64_t* launches);
 
@@ -107,6 +106,8 @@ struct SnArgs {
 };
 
 // refine.cu
+// Mean entries per row up to which the sweeps of one right-hand side use the off-diagonals' own layouts.
+constexpr double kShortRowLen = 14.0;
 struct RefineArgs {
     int n, nnz, rhs;
     const int* rp;

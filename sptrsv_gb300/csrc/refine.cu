@@ -1092,7 +1092,7 @@ static int lpr_for(int n, int nnz) {
     return 32;
 }
 // warp tiles pay off while a 32-row tile usually fits the stage
-static bool short_rows(const RefineArgs& a) { return a.rhs == 1 && (double)a.nnz / a.n <= 14.0; }
+static bool short_rows(const RefineArgs& a) { return a.rhs == 1 && (double)a.nnz / a.n <= kShortRowLen; }
 static bool use_tiles(const RefineArgs& a) { return short_rows(a) && a.off; }
 
 static int stream_grid(int sm_count) { return sm_count * 8; }

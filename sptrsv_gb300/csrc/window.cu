@@ -669,19 +669,29 @@ __global__ void __launch_bounds__(1024) k_level_offsets(int n, int chunks, WinCh
                                                         int* __restrict__ off) {
     __shared__ int d[kChunkMaxCtas], s_warp[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c = warp; c < chunks; c += 32) {
-        int delta = 0;
-        if (c > 0) {
-            const int hi = n - c * ch.rows, cnt = min(64, n - hi);
-            int best = -1;
-            for (int q = lane; q < cnt; q += 32) {
-                const int r = ch.run_up[(size_t)c * ch.warm + q];
-                if (r > best) { best = r; delta = level[hi + q] - r; }
+    // four chunks a time, all their loads in flight together
+    for (int c0 = warp; c0 < chunks; c0 += 128) {
+        int r[4][2], l[4][2];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = c0 + 32 * u, hi = n - c * ch.rows;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const bool in = c > 0 && c < chunks && hi + lane + 32 * q < n;
+                r[u][q] = in ? ch.run_up[(size_t)c * ch.warm + lane + 32 * q] : -1;
+                l[u][q] = in ? level[hi + lane + 32 * q] : -1;
             }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = c0 + 32 * u;
+            const bool second = r[u][1] > r[u][0];
+            const int best = second ? r[u][1] : r[u][0];
+            int delta = second ? l[u][1] - r[u][1] : l[u][0] - r[u][0];
             const int top = __reduce_max_sync(0xffffffffu, best);
             delta = __shfl_sync(0xffffffffu, delta, __ffs(__ballot_sync(0xffffffffu, best == top)) - 1);
+            if (lane == 0 && c < chunks) d[c] = delta;
         }
-        if (lane == 0) d[c] = delta;
     }
     __syncthreads();
     // inclusive sums, a run of chunks per thread
