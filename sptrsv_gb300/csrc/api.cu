@@ -943,7 +943,7 @@ Handle::~Handle() {
     DevBuf* bufs[] = {&own_rp, &own_col, &own_val, &val32, &invd, &invd32, &in_degree, &levels, &level_ptr,
                       &level_rows, &stats, &csc_ptr, &csc_row, &csc_val, &scratch, &settle, &xw, &bw, &r32, &d32a, &d32b,
                       &norms, &indeg_work, &left, &db, &dx, &flush, &offdiag, &roff, &jmeta, &jbase, &sell, &sell_perm, &sell_len, &sell_ptr,
-                      &sn_start, &sn_m, &sn_roff, &sn_rect, &sn_goff, &sn_ld, &sn_colbase, &sn_outbase, &sn_items,
+                      &sn_start, &sn_m, &sn_roff, &sn_rect, &sn_goff, &sn_ld, &sn_tasks, &sn_outbase, &sn_items,
                       &sn_G, &sn_Ghi, &sn_Glo, &sn_pan, &sn_pitems, &sn_pcnt, &sn_ppart, &sn_gtc, &sn_tcrec, &sn_ghl, &sn_gexp, &tune_b, &tune_x};
     for (DevBuf* b : bufs) b->release();
     if (ctl) cudaFree(ctl);

@@ -108,7 +108,7 @@ struct Handle {
     DevBuf sell, sell_perm, sell_len, sell_ptr;  // SELL-32-256 copy of the off-diagonals
     int sell_nslices = 0;
     // supernode partition and its dense panels (supernodal.cu)
-    DevBuf sn_start, sn_m, sn_roff, sn_rect, sn_goff, sn_ld, sn_colbase, sn_outbase, sn_items, sn_G, sn_Ghi, sn_Glo;
+    DevBuf sn_start, sn_m, sn_roff, sn_rect, sn_goff, sn_ld, sn_tasks, sn_outbase, sn_items, sn_G, sn_Ghi, sn_Glo;
     int sn_count = 0, sn_nitems = 0;
     // the FP64 solve's 64-row panels split into column blocks (panels64.cu): panel records,
     // (panel, block) items, per-panel completion counters, partial sums (sn_prows per column)

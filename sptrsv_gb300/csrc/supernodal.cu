@@ -40,41 +40,57 @@ constexpr int kNc = 32;        // right-hand-side columns per pass
 //     factor stored with its explicit zeros); a row that ends inside the triangle leaves zeros
 //     there, the rectangle is the contiguous range b..b+m-1 with m the longest row's reach past b,
 //     and shorter rows read zero in it.
-// Records the rectangle width and the layout (0 exact, 1 skyline).
-__global__ void k_sn_check(int S, const int* __restrict__ sstart, const int* __restrict__ rp,
-                           const int* __restrict__ col, int* __restrict__ m_out, int* __restrict__ kind_out,
-                           Ctl* ctl) {
-    for (int s = blockIdx.x; s < S; s += gridDim.x) {
-        const int a = sstart[s], b = sstart[s + 1], w = b - a;
-        const int m = rp[a + 1] - rp[a] - w;
-        bool exact = m >= 0;
-        const int* rect0 = col + rp[a] + w;
-        for (int t = 0; t < w && exact; ++t) {
-            const int i = a + t, base = rp[i];
-            if (rp[i + 1] - base != (w - t) + m) { exact = false; break; }
-            bool bad = false;
-            for (int q = threadIdx.x; q < w - t; q += blockDim.x) bad |= col[base + q] != i + q;
-            for (int q = threadIdx.x; q < m; q += blockDim.x) bad |= col[base + (w - t) + q] != rect0[q];
-            if (__syncthreads_or(bad)) exact = false;
+// Every row is looked at by itself: a block takes 32 rows of a chunk, a warp four of them.  flags[s]
+// collects what some row rules out (1 the exact layout, 2 the skyline), reach[s] the skyline's m.
+// (One block per chunk walking its rows in turn, a block vote per row, took 445 us on the 20^3
+// dissection factor's 8,000 rows; this takes 26.)
+constexpr int kCheckRows = 32;
+
+__global__ void __launch_bounds__(256) k_sn_check(const int* __restrict__ sstart, const int* __restrict__ rp,
+                                                  const int* __restrict__ col, int* __restrict__ reach,
+                                                  int* __restrict__ flags) {
+    const int s = blockIdx.x, a = sstart[s], w = sstart[s + 1] - a;
+    const int lane = threadIdx.x & 31, t_end = min(w, (int)(blockIdx.y + 1) * kCheckRows);
+    const int m = rp[a + 1] - rp[a] - w;
+    const int* rect0 = col + rp[a] + w;
+    int ruled = m < 0 ? 1 : 0, far = 0;
+    for (int t = blockIdx.y * kCheckRows + (threadIdx.x >> 5); t < t_end; t += 8) {
+        const int i = a + t, base = rp[i], len = rp[i + 1] - base;
+        const int tri = min(w - t, len);
+        const bool same = len == (w - t) + m;  // as long as the exact layout has it
+        far = max(far, len - (w - t));
+        bool gap = false, off = false;
+#pragma unroll 4
+        for (int q = lane; q < tri; q += 32) gap |= col[base + q] != i + q;
+        if (gap || !same) ruled |= 1;
+#pragma unroll 4
+        for (int q = tri + lane; q < len; q += 32) {
+            const int c = col[base + q];
+            gap |= c != i + q;
+            off |= same && c != rect0[q - tri];
         }
-        if (exact) {
-            if (threadIdx.x == 0) { m_out[s] = m; kind_out[s] = 0; }
-            continue;
-        }
-        bool sky = true;
-        int msky = 0;
-        for (int t = 0; t < w && sky; ++t) {
-            const int i = a + t, base = rp[i], len = rp[i + 1] - base;
-            if (len < 1) { sky = false; break; }
-            msky = max(msky, len - (w - t));
-            bool bad = false;
-            for (int q = threadIdx.x; q < len; q += blockDim.x) bad |= col[base + q] != i + q;
-            if (__syncthreads_or(bad)) sky = false;
-        }
-        if (threadIdx.x == 0) {
-            m_out[s] = sky ? msky : 0;
+        ruled |= (gap ? 2 : 0) | (off ? 1 : 0);
+    }
+    ruled = __reduce_or_sync(0xffffffffu, ruled);
+    if (lane == 0) {
+        if (ruled) atomicOr(flags + s, ruled);
+        if (far > 0) atomicMax(reach + s, far);
+    }
+}
+
+// The rectangle width and the layout (0 exact, 1 skyline) of every chunk.
+__global__ void k_sn_kind(int S, const int* __restrict__ sstart, const int* __restrict__ rp,
+                          const int* __restrict__ reach, const int* __restrict__ flags, int* __restrict__ m_out,
+                          int* __restrict__ kind_out, Ctl* ctl) {
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
+        const int a = sstart[s], f = flags[s];
+        if (f & 1) {
+            m_out[s] = (f & 2) ? 0 : reach[s];
             kind_out[s] = 1;
-            if (!sky) record_error(ctl, SPTRSV_ERR_SUPERNODES);
+            if (f & 2) record_error(ctl, SPTRSV_ERR_SUPERNODES);
+        } else {
+            m_out[s] = rp[a + 1] - rp[a] - (sstart[s + 1] - a);
+            kind_out[s] = 0;
         }
     }
 }
@@ -93,40 +109,99 @@ __global__ void k_sn_rectcols(int S, const int* __restrict__ sstart, const int* 
     }
 }
 
-// Column j of T_s^{-1} by back substitution, one warp per (supernode, column); written into the
-// first w columns of G_s (row-major, leading dimension ld).
-__global__ void __launch_bounds__(256) k_sn_tinv(int S, const int* __restrict__ sstart, const int* __restrict__ rp,
+// T_s^{-1} into the first w columns of G_s (row-major, leading dimension ld), in blocks of 32 rows:
+// k_sn_dinv inverts the diagonal blocks D_I, then k_sn_tinv builds eight columns a block upwards,
+//     X_I = -D_I sum_{K > I} T_IK X_K,
+// a thread per (row, column) of X_I.  w^3 / 6 FP64 FMAs a chunk bound it (2 a clock and SM); a warp per
+// column substituting row by row, as before, spent five shuffle-and-add steps and a division on each of
+// its w^2 / 2 rows instead.  Measured on GB300, 20^3 dissection factor: 743 -> 42 + 106 us.
+constexpr int kInvB = 32;    // rows of a block
+constexpr int kInvCols = 8;  // columns of a CTA
+
+// T[r][c] of the chunk from row a, c >= r; a skyline row may end inside the triangle.
+__device__ __forceinline__ double sn_t(const int* __restrict__ rp, const double* __restrict__ val, int a, int r, int c) {
+    const int base = rp[a + r] + (c - r);
+    return base < rp[a + r + 1] ? val[base] : 0.0;
+}
+
+// A warp per diagonal block, a lane per column j of its inverse, upwards from row j: x_r = -acc_r / T_rr
+// (1 / T_jj at r = j), then acc_i += T_ir x_r for every row i above, the sums in registers.  An FP64
+// operation holds its SM quarter's pipe for 64 cycles, so operations are counted: one reciprocal per
+// lane for all 32 rows instead of 32 divisions of ~14 operations.
+__global__ void __launch_bounds__(128) k_sn_dinv(const int* __restrict__ sstart, const int* __restrict__ rp,
                                                  const double* __restrict__ val, const long long* __restrict__ goff,
-                                                 const int* __restrict__ ld, const int* __restrict__ colbase,
-                                                 int ncols, double* __restrict__ G) {
-    __shared__ double xs[8][kSnMaxW];
+                                                 const int* __restrict__ ld, double* __restrict__ G) {
+    __shared__ double s_t[4][kInvB][kInvB + 1];
     const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
-    for (int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < ncols; task += (gridDim.x * blockDim.x) >> 5) {
-        // task -> (s, j) through the per-supernode column offsets
-        int lo = 0, hi = S - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (colbase[mid] <= task) lo = mid; else hi = mid - 1;
+    const int s = blockIdx.x, blk = blockIdx.y * 4 + wv;
+    const int a = sstart[s], w = sstart[s + 1] - a, r0 = blk * kInvB, nb = min(kInvB, w - r0);
+    if (nb <= 0) return;
+    double(*T)[kInvB + 1] = s_t[wv];
+    // rows past a short block are the identity's
+#pragma unroll 8
+    for (int r = 0; r < kInvB; ++r)
+        T[r][lane] = lane >= r && lane < nb ? sn_t(rp, val, a, r0 + r, r0 + lane) : (r == lane ? 1.0 : 0.0);
+    __syncwarp();
+    const double inv = 1.0 / T[lane][lane];
+    double acc[kInvB];
+#pragma unroll
+    for (int r = 0; r < kInvB; ++r) acc[r] = 0.0;
+    double* g = G + goff[s] + (size_t)r0 * ld[s] + r0;
+#pragma unroll
+    for (int r = kInvB - 1; r >= 0; --r) {
+        const double inv_r = __shfl_sync(0xffffffffu, inv, r);
+        const double x = lane < r ? 0.0 : lane == r ? inv : -acc[r] * inv_r;
+#pragma unroll
+        for (int i = 0; i < r; ++i) acc[i] = fma(T[i][r], x, acc[i]);
+        if (r < nb && lane < nb) g[(size_t)r * ld[s] + lane] = x;
+    }
+}
+
+// tasks: (chunk, block of columns), one a CTA, the longest columns of a chunk first.
+__global__ void __launch_bounds__(kInvB * kInvCols) k_sn_tinv(const int2* __restrict__ tasks,
+                                                               const int* __restrict__ sstart,
+                                                               const int* __restrict__ rp,
+                                                               const double* __restrict__ val,
+                                                               const long long* __restrict__ goff,
+                                                               const int* __restrict__ ld, double* __restrict__ G) {
+    __shared__ double X[kSnMaxW][kInvCols];
+    __shared__ double M[kInvB][kInvCols];
+    const int s = tasks[blockIdx.x].x, a = sstart[s], w = sstart[s + 1] - a, j0 = tasks[blockIdx.x].y * kInvCols;
+    const int r = threadIdx.x / kInvCols, jj = threadIdx.x % kInvCols, j = j0 + jj;
+    const size_t L = ld[s];
+    double* g = G + goff[s];
+    const int jb = j0 / kInvB, top = min(w, (jb + 1) * kInvB);  // the columns' diagonal block; no rows past it
+    for (int I = jb; I >= 0; --I) {
+        const int row = I * kInvB + r;
+        const bool in = row < top && j < w;
+        double v = 0.0;
+        if (I == jb) {
+            if (in && row <= j) v = g[(size_t)row * L + j];  // k_sn_dinv's
+        } else {
+            // M = sum_{K > I} T_IK X_K, four chains
+            double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;
+            const int base = rp[a + row] - row, end = min(top, rp[a + row + 1] - base);  // T[row][c] = val[base + c]
+            int c = (I + 1) * kInvB;
+            for (; c + 3 < end; c += 4) {
+                m0 = fma(val[base + c], X[c][jj], m0);
+                m1 = fma(val[base + c + 1], X[c + 1][jj], m1);
+                m2 = fma(val[base + c + 2], X[c + 2][jj], m2);
+                m3 = fma(val[base + c + 3], X[c + 3][jj], m3);
+            }
+            for (; c < end; ++c) m0 = fma(val[base + c], X[c][jj], m0);
+            M[r][jj] = (m0 + m1) + (m2 + m3);
+            __syncthreads();
+            double d0 = 0.0, d1 = 0.0;
+            const double* d = g + (size_t)row * L + I * kInvB;  // row r of D_I: columns r .. 31
+            for (int q = r; q < kInvB; q += 2) {
+                d0 = fma(d[q], M[q][jj], d0);
+                if (q + 1 < kInvB) d1 = fma(d[q + 1], M[q + 1][jj], d1);
+            }
+            v = -(d0 + d1);
+            if (in) g[(size_t)row * L + j] = v;
         }
-        const int s = lo, j = task - colbase[s];
-        const int a = sstart[s], w = sstart[s + 1] - a;
-        double* x = xs[wv];
-        // T[r][c] = val[rp[a+r] + (c - r)]  (c >= r)
-        if (lane == 0) x[j] = 1.0 / val[rp[a + j]];
-        __syncwarp();
-        for (int r = j - 1; r >= 0; --r) {
-            const int base = rp[a + r] - r;
-            const int lim = min(j, rp[a + r + 1] - base - 1);  // a skyline row may end inside the triangle
-            double sum = 0.0;
-            for (int c = r + 1 + lane; c <= lim; c += 32) sum = fma(val[base + c], x[c], sum);
-            sum = warp_sum(sum);
-            if (lane == 0) x[r] = -sum / val[rp[a + r]];
-            __syncwarp();
-        }
-        double* g = G + goff[s];
-        const int L = ld[s];
-        for (int r = lane; r < w; r += 32) g[(size_t)r * L + j] = r <= j ? x[r] : 0.0;
-        __syncwarp();
+        if (row < kSnMaxW) X[row][jj] = v;
+        __syncthreads();
     }
 }
 
@@ -309,12 +384,18 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
     }
     const int S = (int)ss.size() - 1;
     int rc;
-    if ((rc = sn_start.ensure(sizeof(int) * (S + 1))) || (rc = sn_m.ensure(sizeof(int) * 2 * S))) return rc;
+    if ((rc = sn_start.ensure(sizeof(int) * (S + 1))) || (rc = sn_m.ensure(sizeof(int) * 4 * S))) return rc;
     CUDA_TRY(cudaMemcpyAsync(sn_start.p, ss.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice, st));
     if ((rc = reset_ctl())) return rc;
-    k_sn_check<<<std::min(S, sm_count * 8), 128, 0, st>>>(S, sn_start.as<int>(), rp, col, sn_m.as<int>(),
-                                                         sn_m.as<int>() + S, ctl);
-    ++launches;
+    int wmax = 0;
+    for (int q = 0; q < S; ++q) wmax = std::max(wmax, ss[q + 1] - ss[q]);
+    // sn_m: rectangle widths, layouts, and the checks' reach and flags
+    int* reach = sn_m.as<int>() + 2 * (size_t)S;
+    CUDA_TRY(cudaMemsetAsync(reach, 0, sizeof(int) * 2 * S, st));
+    k_sn_check<<<dim3(S, (wmax + kCheckRows - 1) / kCheckRows), 256, 0, st>>>(sn_start.as<int>(), rp, col, reach, reach + S);
+    k_sn_kind<<<std::min((S + 255) / 256, sm_count), 256, 0, st>>>(S, sn_start.as<int>(), rp, reach, reach + S,
+                                                                   sn_m.as<int>(), sn_m.as<int>() + S, ctl);
+    launches += 2;
     CUDA_TRY(cudaGetLastError());
     Ctl c{};
     if ((rc = read_ctl(&c))) return rc;
@@ -322,7 +403,7 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
     std::vector<int> m(S);
     CUDA_TRY(cudaMemcpy(m.data(), sn_m.p, sizeof(int) * S, cudaMemcpyDeviceToHost));
     // per-chunk offsets (host bookkeeping over S entries)
-    std::vector<int> roffh(S + 1, 0), ldh(S), colbase(S + 1, 0);
+    std::vector<int> roffh(S + 1, 0), ldh(S);
     std::vector<long long> goffh(S + 1, 0), outbase(S + 1, 0);
     std::vector<int> item_s, item_p;
     for (int s = 0; s < S; ++s) {
@@ -331,9 +412,11 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
         ldh[s] = (w + m[s] + 15) & ~15;
         const int wpad = (w + 15) & ~15;
         goffh[s + 1] = goffh[s] + (long long)wpad * ldh[s];
-        colbase[s + 1] = colbase[s] + w;
         outbase[s + 1] = outbase[s] + (long long)w * m[s];
     }
+    std::vector<int2> inv;
+    for (int s = 0; s < S; ++s)
+        for (int q = (ss[s + 1] - ss[s] + kInvCols - 1) / kInvCols - 1; q >= 0; --q) inv.push_back(make_int2(s, q));
     for (int s = S - 1; s >= 0; --s) {
         const int w = ss[s + 1] - ss[s];
         for (int p = 0; p * kPanel < w; ++p) { item_s.push_back(s); item_p.push_back(p); }
@@ -341,14 +424,14 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
     const long long gtot = goffh[S];
     if ((rc = sn_roff.ensure(sizeof(int) * (S + 1))) || (rc = sn_rect.ensure(sizeof(int) * ((size_t)roffh[S] + 1))) ||
         (rc = sn_goff.ensure(sizeof(long long) * (S + 1))) || (rc = sn_ld.ensure(sizeof(int) * S)) ||
-        (rc = sn_colbase.ensure(sizeof(int) * (S + 1))) || (rc = sn_outbase.ensure(sizeof(long long) * (S + 1))) ||
+        (rc = sn_tasks.ensure(sizeof(int2) * inv.size())) || (rc = sn_outbase.ensure(sizeof(long long) * (S + 1))) ||
         (rc = sn_items.ensure(sizeof(int) * 2 * item_s.size())) || (rc = sn_G.ensure(sizeof(double) * (size_t)gtot)) ||
         (rc = sn_Ghi.ensure(2 * (size_t)gtot)) || (rc = sn_Glo.ensure(2 * (size_t)gtot)))
         return rc;
     CUDA_TRY(cudaMemcpyAsync(sn_roff.p, roffh.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(sn_goff.p, goffh.data(), sizeof(long long) * (S + 1), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(sn_ld.p, ldh.data(), sizeof(int) * S, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(sn_colbase.p, colbase.data(), sizeof(int) * (S + 1), cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(sn_tasks.p, inv.data(), sizeof(int2) * inv.size(), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(sn_outbase.p, outbase.data(), sizeof(long long) * (S + 1), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(sn_items.p, item_s.data(), sizeof(int) * item_s.size(), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(sn_items.as<int>() + item_s.size(), item_p.data(), sizeof(int) * item_p.size(),
@@ -356,9 +439,11 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
     CUDA_TRY(cudaMemsetAsync(sn_G.p, 0, sizeof(double) * (size_t)gtot, st));
     k_sn_rectcols<<<std::min(S, sm_count * 8), 128, 0, st>>>(S, sn_start.as<int>(), rp, col, sn_roff.as<int>(),
                                                             sn_m.as<int>() + S, sn_rect.as<int>());
-    k_sn_tinv<<<sm_count * 8, 256, 0, st>>>(S, sn_start.as<int>(), rp, val, sn_goff.as<long long>(), sn_ld.as<int>(),
-                                            sn_colbase.as<int>(), colbase[S], sn_G.as<double>());
-    launches += 2;
+    k_sn_dinv<<<dim3(S, (wmax + 4 * kInvB - 1) / (4 * kInvB)), 128, 0, st>>>(
+        sn_start.as<int>(), rp, val, sn_goff.as<long long>(), sn_ld.as<int>(), sn_G.as<double>());
+    k_sn_tinv<<<(unsigned)inv.size(), kInvB * kInvCols, 0, st>>>(
+        sn_tasks.as<int2>(), sn_start.as<int>(), rp, val, sn_goff.as<long long>(), sn_ld.as<int>(), sn_G.as<double>());
+    launches += 3;
     if (outbase[S] > 0) {
         k_sn_w<<<sm_count * 16, 256, 0, st>>>(S, sn_start.as<int>(), rp, val, sn_goff.as<long long>(), sn_ld.as<int>(),
                                               sn_m.as<int>(), sn_outbase.as<long long>(), outbase[S],
