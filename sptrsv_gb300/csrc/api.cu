@@ -367,7 +367,7 @@ int Handle::prepare(const sptrsv_opts& o, int rhs, int layout) {
         if ((rc = grow(indeg_work, sizeof(int) * (size_t)n))) return rc;
         if ((rc = grow(left, sizeof(double) * nr))) return rc;
     }
-    if (o.schedule == SPTRSV_SCHED_SUPERNODAL && o.precision == SPTRSV_PREC_FP64 && have_supernodes) {
+    if (o.schedule == SPTRSV_SCHED_SUPERNODAL && o.precision == SPTRSV_PREC_FP64 && have_supernodes && !sn_rows) {
         if ((rc = grow(sn_ppart, sizeof(double) * (size_t)sn_prows * rhs))) return rc;
         if ((rc = grow(sn_pcnt, sizeof(int) * (size_t)sn_npan * p64_groups(rhs)))) return rc;
     }

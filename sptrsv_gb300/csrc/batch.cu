@@ -922,6 +922,7 @@ struct Batch {
     std::vector<int> panel_ok;  // -1 unknown, 0 no, 1 yes
     std::vector<char> have_bf16, have_f64, have_tc;  // have_tc: tensor-core records of the FP64 panels
     bool use_tc = false;  // the FP64 panel items run on the tensor cores (set by build_lists)
+    bool rows64 = false;  // items64 are rows of panels (panel_rows.cu), not column blocks
     long long tot_rows = 0, tot_nnz = 0, tot_x = 0, tot_rp = 0;
     DevBuf rp, col, val, val32, invd, invd32, dsys, dstate, dctl;
     DevBuf r32, d0, d1, bw, xw;
@@ -935,7 +936,8 @@ struct Batch {
     unsigned n_order_all = 0, n_order_plain = 0, n_order_sf32 = 0, n_items = 0;
     DevSeg all_rows, all_el, mixed_rows, mixed_el, jac_rows, pend_el, plain_el;
     std::vector<DevBuf> gbufs;            // per panel system: hi, lo, rect
-    std::vector<std::vector<BChunk>> pchunks;  // per system (host copies, pointers into gbufs)
+    std::vector<std::vector<BChunk>> pchunks, pchunks64;  // per system, BF16 and FP64 panels (pointers into gbufs)
+    std::vector<int> chunk_rows64;  // rows per chunk of every system's FP64 panels (pick_chunk_rows)
     std::vector<int> gidx;                // per system: first of its 3 gbufs, or -1
     bool lists_ready = false;
     // options
@@ -959,6 +961,7 @@ struct Batch {
     ~Batch();
     BArgs args(const double* b, double* x) const;
     int build_lists();
+    void pick_chunk_rows();
     int build_panels(int s, bool f64);
     bool jacobi_elem = false;  // tuning override (SPTRSV_BJAC=elem): the thread-per-element sweep
     void launch_jacobi(const BArgs& A);
@@ -1043,9 +1046,35 @@ static int upload_vec(DevBuf& d, const std::vector<T>& h, cudaStream_t st) {
     return 0;
 }
 
-// Dense panels of system s: uniform 64-row chunks (each one a skyline or exact supernode chunk),
-// G = [T^-1 | -T^-1 Rect] formed in FP64 by the single-system supernodal analysis and kept as
-// its BF16 hi/lo split.
+// Rows per chunk of the FP64 panels: 64, 128 or 256.  The chunks of a system form one chain, so wider ones
+// mean fewer steps (a step costs its warps' way through the products plus ~2 us of publishing, polling
+// and adding up); but a chunk's triangle is dense, w / 2 products a row beside the band's g.  Every system
+// gets the narrowest chunks whose chain ends with the batch: within the FP64 time of all systems (~630
+// G FMA/s) or the longest chain at 256 rows, whichever is longer.  Measured on GB300 (48 systems of up to
+// 30k rows): 64 rows everywhere 4.9 ms, picked here 1.9 ms.
+void Batch::pick_chunk_rows() {
+    chunk_rows64.assign(count, kBPanel);
+    if (panels_mode() != 0) return;  // the other modes' items are 64-row panels
+    auto nnz_of = [&](int s) { return (double)((s + 1 < count ? sys[s + 1].nz0 : tot_nnz) - sys[s].nz0); };
+    auto band = [&](int s) { return nnz_of(s) / sys[s].n; };
+    auto chain_us = [&](int s, int w) {
+        const double steps = std::min<double>(w, band(s)) / 32.0, cols = std::min(sys[s].rhs, kPanelCols);
+        return std::ceil((double)sys[s].n / w) * (2.0 + steps * cols * 0.35);
+    };
+    double fp64_us = 0.0, longest_us = 0.0;
+    for (int s = 0; s < count; ++s) {
+        if (panel_ok[s] == 0 || nnz_of(s) < 8.0 * sys[s].n) continue;
+        fp64_us += sys[s].n * (32.0 + band(s)) * sys[s].rhs / 630e3;
+        longest_us = std::max(longest_us, chain_us(s, 256));
+    }
+    const double goal = std::max(fp64_us, longest_us);
+    for (int s = 0; s < count; ++s)
+        while (chunk_rows64[s] < 256 && chain_us(s, chunk_rows64[s]) > goal) chunk_rows64[s] *= 2;
+}
+
+// Dense panels of system s: uniform chunks (each one a skyline or exact supernode chunk) of 64 rows, or
+// for the FP64 panels of its chunk_rows64, G = [T^-1 | -T^-1 Rect] formed in FP64 by the single-system
+// supernodal analysis and kept as it is or as its BF16 hi/lo split.
 int Batch::build_panels(int s, bool f64) {
     if (panel_ok[s] == 0) return SPTRSV_ERR_SUPERNODES;
     if (panel_ok[s] == 1 && (f64 ? have_f64[s] : have_bf16[s])) return 0;
@@ -1066,7 +1095,7 @@ int Batch::build_panels(int s, bool f64) {
     H.val = val.as<double>() + S.nz0;
     if ((rc = H.analyse())) return rc;
     std::vector<int> sn;
-    for (int a = 0; a < S.n; a += kBPanel) sn.push_back(a);
+    for (int a = 0; a < S.n; a += f64 && panels_mode() == 0 ? chunk_rows64[s] : kBPanel) sn.push_back(a);
     sn.push_back(S.n);
     rc = H.set_supernodes((int)sn.size() - 1, sn.data());
     if (rc == SPTRSV_ERR_SUPERNODES) {
@@ -1098,9 +1127,8 @@ int Batch::build_panels(int s, bool f64) {
     if (roff[C] > 0)
         CUDA_TRY(cudaMemcpyAsync(gbufs[k0 + 3].p, H.sn_rect.p, sizeof(int) * roff[C], cudaMemcpyDeviceToDevice, st));
     CUDA_TRY(cudaStreamSynchronize(st));
-    // keep the other precision's pointers of an earlier build
-    std::vector<BChunk> old = pchunks[s];
-    pchunks[s].clear();
+    std::vector<BChunk>& mine = (f64 ? pchunks64 : pchunks)[s];
+    mine.clear();
     for (int c = 0; c < C; ++c) {
         BChunk ch{};
         ch.sys = s;
@@ -1114,21 +1142,11 @@ int Batch::build_panels(int s, bool f64) {
         if (!f64) {
             ch.ghi = gbufs[k0].as<__nv_bfloat16>() + goff[c];
             ch.glo = gbufs[k0 + 1].as<__nv_bfloat16>() + goff[c];
-            if ((int)old.size() == C) {
-                ch.g64 = old[c].g64;
-                ch.gtc = old[c].gtc;
-                ch.ghl = old[c].ghl;
-                ch.gexp = old[c].gexp;
-            }
         } else {
             ch.g64 = gbufs[k0 + 2].as<double>() + goff[c];
-            if ((int)old.size() == C) {
-                ch.ghi = old[c].ghi;
-                ch.glo = old[c].glo;
-            }
         }
         ch.rect = gbufs[k0 + 3].as<int>() + roff[c];
-        pchunks[s].push_back(ch);
+        mine.push_back(ch);
     }
     have_tc[s] = 0;
     if (f64 && panels_mode() == 1) {
@@ -1136,16 +1154,16 @@ int Batch::build_panels(int s, bool f64) {
         std::vector<size_t> toff(C + 1, 0);
         std::vector<int2> recs;
         for (int c = 0; c < C; ++c) {
-            const BChunk& b = pchunks[s][c];
+            const BChunk& b = mine[c];
             toff[c + 1] = toff[c] + ((tc_panel_bytes(b.w, b.w + b.m) + 127) & ~(size_t)127);
             for (int q = 0; q < b.nblk; ++q) recs.push_back(make_int2(c, q));
         }
         if ((rc = gbufs[k0 + 4].ensure(std::max<size_t>(toff[C], 128)))) return rc;
-        for (int c = 0; c < C; ++c) pchunks[s][c].gtc = gbufs[k0 + 4].as<unsigned char>() + toff[c];
+        for (int c = 0; c < C; ++c) mine[c].gtc = gbufs[k0 + 4].as<unsigned char>() + toff[c];
         DevBuf tch, trec;
         if ((rc = tch.ensure(sizeof(BChunk) * C)) || (rc = trec.ensure(sizeof(int2) * std::max<size_t>(1, recs.size()))))
             return rc;
-        CUDA_TRY(cudaMemcpyAsync(tch.p, pchunks[s].data(), sizeof(BChunk) * C, cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(tch.p, mine.data(), sizeof(BChunk) * C, cudaMemcpyHostToDevice, st));
         CUDA_TRY(cudaMemcpyAsync(trec.p, recs.data(), sizeof(int2) * recs.size(), cudaMemcpyHostToDevice, st));
         int64_t lsplit = 0;
         rc = launch_tc_split(tch.as<BChunk>(), trec.as<int2>(), (int)recs.size(), sm_count, st, &lsplit);
@@ -1162,12 +1180,12 @@ int Batch::build_panels(int s, bool f64) {
             (rc = gbufs[k0 + 6].ensure(sizeof(int) * (size_t)std::max(1, S.n))))
             return rc;
         for (int c = 0; c < C; ++c) {
-            pchunks[s][c].ghl = gbufs[k0 + 5].as<float2>() + goff[c];
-            pchunks[s][c].gexp = gbufs[k0 + 6].as<int>() + ss[c];
+            mine[c].ghl = gbufs[k0 + 5].as<float2>() + goff[c];
+            mine[c].gexp = gbufs[k0 + 6].as<int>() + ss[c];
         }
         DevBuf tch;
         if ((rc = tch.ensure(sizeof(BChunk) * C))) return rc;
-        CUDA_TRY(cudaMemcpyAsync(tch.p, pchunks[s].data(), sizeof(BChunk) * C, cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(tch.p, mine.data(), sizeof(BChunk) * C, cudaMemcpyHostToDevice, st));
         int64_t lconv = 0;
         rc = launch_g_df(tch.as<BChunk>(), C, st, &lconv);
         if (!rc) CUDA_TRY(cudaStreamSynchronize(st));
@@ -1260,25 +1278,37 @@ int Batch::build_lists() {
     use_tc = panels_mode() == 1;
     for (int s = 0; s < count; ++s)
         if (sched[s] == BS_PANEL64 && !have_tc[s]) use_tc = false;
+    // rows of panels, unless every panel system has what the tensor cores or the double-FP32 products need
+    bool df = panels_mode() == 2;
+    for (int s = 0; s < count && df; ++s)
+        if (sched[s] == BS_PANEL64 && !pchunks64[s].empty() && !pchunks64[s][0].ghl) df = false;
+    rows64 = !use_tc && !df;
     long long poff = 0;
     int cbase = 0;
     g_entries64 = g_fma64 = 0;
     for (int s = 0; s < count; ++s) {
         if (sched[s] != BS_PANEL64) continue;
-        const int base = (int)ch64.size(), ng = use_tc ? tc_groups_host(sys[s].rhs) : p64_groups(sys[s].rhs);
-        if (ng > 0x7FFF) return SPTRSV_ERR_TOO_LARGE;  // items carry the group in 15 bits
-        for (const BChunk& b : pchunks[s])
+        const int base = (int)ch64.size();
+        const int ng = rows64 ? panel_groups(sys[s].rhs) : use_tc ? tc_groups_host(sys[s].rhs) : p64_groups(sys[s].rhs);
+        if (ng > (rows64 ? 0x7FFFFF : 0x7FFF)) return SPTRSV_ERR_TOO_LARGE;  // items carry the group in 23 or 15 bits
+        for (const BChunk& b : pchunks64[s])
             if (b.nblk > 0xFFFF) return SPTRSV_ERR_TOO_LARGE;  // and the block in 16
         std::vector<std::vector<int2>> steps;
-        for (int c = (int)pchunks[s].size() - 1; c >= 0; --c) {
-            const BChunk& b = pchunks[s][c];
+        for (int c = (int)pchunks64[s].size() - 1; c >= 0; --c) {
+            const BChunk& b = pchunks64[s][c];
             std::vector<int2> its;
+            if (rows64) {
+                for (int q = 0; q * kPanelRows < b.w; ++q)
+                    for (int g = 0; g < ng; ++g) its.push_back(make_int2(base + c, q | g << 8));
+                steps.push_back(std::move(its));
+                continue;
+            }
             for (int q = 0; q < b.nblk; ++q)
                 for (int g = 0; g < ng; ++g) its.push_back(make_int2(base + c, (q == 0 ? 0 : b.nblk - q) | g << 16));
             steps.push_back(std::move(its));
         }
-        for (BChunk b : pchunks[s]) {
-            if (panels_mode() != 2) b.ghl = nullptr;  // double-FP32 products only in that mode
+        for (BChunk b : pchunks64[s]) {
+            if (!df) b.ghl = nullptr;  // double-FP32 products only in that mode
             b.poff = poff;
             b.cbase = cbase;
             cbase += ng;
@@ -1302,7 +1332,7 @@ int Batch::build_lists() {
     n_chunks64 = (int)ch64.size();
     n_cnt64 = cbase;
     if ((rc = upload_vec(chunks64, ch64, st)) || (rc = upload_vec(items64, it64, st))) return rc;
-    if (n_chunks64 && ((rc = part64.ensure(sizeof(double) * (size_t)std::max(1LL, poff))) ||
+    if (n_chunks64 && !rows64 && ((rc = part64.ensure(sizeof(double) * (size_t)std::max(1LL, poff))) ||
                        (rc = cnt64.ensure(sizeof(int) * (size_t)n_cnt64))))
         return rc;
     lists_ready = true;
@@ -1400,7 +1430,9 @@ int Batch::build_graph(int mode, const double* b, double* x, cudaGraphExec_t* ou
             cudaEventRecord(ev_fork, st);
             cudaStreamWaitEvent(st2, ev_fork, 0);
             int64_t l64 = 0;
-            if (use_tc
+            if (rows64 ? launch_panel_rows(A.sys, 0, A.b, A.x, &A.bc->c, &A.bc->ticket_p64, A.budget, items64.as<int2>(),
+                                           n_items64, chunks64.as<BChunk>(), p64_ctas_per_sm, sm_count, st2, &l64)
+                : use_tc
                     ? launch_panels_tc(A.sys, 0, A.b, A.x, &A.bc->c, &A.bc->ticket_p64, A.budget, items64.as<int2>(),
                                        n_items64, chunks64.as<BChunk>(), part64.as<double>(), cnt64.as<int>(),
                                        n_cnt64, sm_count, st2, &l64)
@@ -1561,7 +1593,10 @@ int Batch::profile(int mode, const double* b, double* x, float* kind_ms, int* ki
         if (n_items64) {
             int64_t l64 = 0;
             if ((rc = timed(13, [&] {
-                     if (use_tc)
+                     if (rows64)
+                         launch_panel_rows(A.sys, 0, A.b, A.x, &A.bc->c, &A.bc->ticket_p64, A.budget,
+                                           items64.as<int2>(), n_items64, chunks64.as<BChunk>(), 64, sm_count, st, &l64);
+                     else if (use_tc)
                          launch_panels_tc(A.sys, 0, A.b, A.x, &A.bc->c, &A.bc->ticket_p64, A.budget, items64.as<int2>(),
                                           n_items64, chunks64.as<BChunk>(), part64.as<double>(), cnt64.as<int>(),
                                           n_cnt64, sm_count, st, &l64);
@@ -1710,6 +1745,7 @@ int sptrsv_batch_create(sptrsv_batch* out, int device, int count, const int* n, 
     B->have_tc.assign(count, 0);
     B->gidx.assign(count, -1);
     B->pchunks.resize(count);
+    B->pchunks64.resize(count);
     int rc = 0;
     auto fail = [&](int code) {
         delete B;
@@ -1783,6 +1819,7 @@ int sptrsv_batch_create(sptrsv_batch* out, int device, int count, const int* n, 
         B->sched[s] = default_schedule(sys[s], nnz[s], r, hs[s].gapped);
         if (hs[s].gapped) B->panel_ok[s] = 0;
     }
+    B->pick_chunk_rows();
     *out = reinterpret_cast<sptrsv_batch>(B);
     return 0;
 }

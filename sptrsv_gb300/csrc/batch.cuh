@@ -80,6 +80,17 @@ int launch_panels64(const BSys* sys, int rhs, const double* b, double* x, Ctl* c
                     const int2* items, unsigned nitems, const BChunk* panels, double* part, int* cnt, int ncnt,
                     int ctas_per_sm, int sm_count, cudaStream_t st, int64_t* launches);
 
+// Exact FP64 panel products, a warp per kPanelRows rows and up to kPanelCols right-hand sides
+// (panel_rows.cu): items {panel, index of its rows}, in an order in which every item waits on earlier
+// ones only.  Batched (sys != nullptr): items carry their group (rows | group << 8).  One system
+// (sys == nullptr, rhs columns, row-major n x rhs): every item runs for each of panel_groups(rhs).
+constexpr int kPanelRows = 4;
+constexpr int kPanelCols = 2;
+__host__ __device__ __forceinline__ int panel_groups(int rhs) { return (rhs + kPanelCols - 1) / kPanelCols; }
+int launch_panel_rows(const BSys* sys, int rhs, const double* b, double* x, Ctl* ctl, unsigned* ticket, int64_t budget,
+                      const int2* items, unsigned nitems, const BChunk* panels, int ctas_per_sm, int sm_count,
+                      cudaStream_t st, int64_t* launches);
+
 // FP64-accurate panel products on the tensor cores (panels_tc.cu): the same items, partial sums
 // and counters as launch_panels64, with tc_groups_host(rhs) groups per item for one system.  The
 // panels' gtc records come from launch_tc_split over every (panel, block) pair in recs.

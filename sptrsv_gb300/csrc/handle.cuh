@@ -120,6 +120,7 @@ struct Handle {
     int sn_npan = 0;
     unsigned sn_npitems = 0;
     long long sn_prows = 0;
+    bool sn_rows = false;     // sn_pitems are rows of panels (panel_rows.cu), not column blocks
     bool have_supernodes = false;
     bool have_offdiag = false;
     bool have_val32 = false;  // val32 holds the FP32 values (built when a mixed solve reads them)

@@ -1,5 +1,6 @@
-// panels64.cu -- exact FP64 products over dense panels, each panel's product split into column
-// blocks taken by different CTAs (used by the batched path and the single-system supernodal path).
+// panels64.cu -- double-FP32 products over dense panels (panel mode 2), each panel's product split into
+// column blocks taken by different CTAs (used by the batched path and the single-system supernodal
+// path).  FP64 products take a warp per four rows instead (panel_rows.cu).
 #include <algorithm>
 #include "common.cuh"
 #include "batch.cuh"
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(128, 8) k_panels64(const BSys* __restrict__ sy
     __shared__ double Vs[kP64][kP64Nc + 1];
     __shared__ unsigned s_t;
     __shared__ int s_ok, s_last;
-    __shared__ int s_vexp[kP64Nc];  // double-FP32 panels: the item's column exponent bounds
+    __shared__ int s_vexp[kP64Nc];  // the item's column exponent bounds
     for (;;) {
         if (threadIdx.x == 0) s_t = aborted(ctl) ? 0xFFFFFFFFu : atomicAdd(ticket, 1u);
         __syncthreads();
@@ -110,7 +111,6 @@ __global__ void __launch_bounds__(128, 8) k_panels64(const BSys* __restrict__ sy
         const int m = sys ? sys[C.sys].rhs : rhs;
         const long long xb0 = sys ? sys[C.sys].xb0 : 0, poff = sys ? C.poff : C.poff * m;
         const int cidx = sys ? C.cbase + cg : C.cbase * ncg + cg;
-        const bool df = C.ghl != nullptr;  // double-FP32 products for this panel
         const int gw = p64_group_width(m), c0 = cg * gw, nc = min(gw, m - c0);
         const int a = C.a, w = C.w, K = C.w + C.m, L = C.ld, blk = it.y, r0 = C.r0, pw = C.pw;
         int k0, kc;
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(128, 8) k_panels64(const BSys* __restrict__ sy
         for (int e = threadIdx.x; e < pw * kc; e += blockDim.x) {
             const int r = e / kc, kk = e - r * kc;
             const size_t g = (size_t)(r0 + r) * L + k0 + kk;
-            cp_async8(&Gs[r][kk], df ? (const void*)(C.ghl + g) : (const void*)(C.g64 + g));
+            cp_async8(&Gs[r][kk], C.ghl + g);
         }
         if (threadIdx.x == 0) s_ok = 1;
         if (threadIdx.x < kP64Nc) s_vexp[threadIdx.x] = -2000;
@@ -154,14 +154,14 @@ __global__ void __launch_bounds__(128, 8) k_panels64(const BSys* __restrict__ sy
                         val = 0.0;
                     }
                     Vs[kk][j] = val;
-                    if (df) atomicMax(&s_vexp[j], df_exp_bound(val));
+                    atomicMax(&s_vexp[j], df_exp_bound(val));
                 }
             }
         }
         cp_async_wait_all();
         __syncthreads();
         const bool ok = s_ok;
-        if (ok && df) {
+        if (ok) {
             // the right-hand side scaled by its columns' bounds and split, in place (8 bytes each)
             float2* V2 = reinterpret_cast<float2*>(&Vs[0][0]);
             for (int e = threadIdx.x; e < kc * nc; e += blockDim.x) {
@@ -180,18 +180,6 @@ __global__ void __launch_bounds__(128, 8) k_panels64(const BSys* __restrict__ sy
                 else if (nc <= 4) df_row<2>(G2, V2, r, jb, kc, nc, er, s_vexp, pb, m, c0);
                 else if (nc <= 8) df_row<4>(G2, V2, r, jb, kc, nc, er, s_vexp, pb, m, c0);
                 else df_row<kP64Nc / 2>(G2, V2, r, jb, kc, nc, er, s_vexp, pb, m, c0);
-            }
-        } else if (ok) {
-            for (int o = threadIdx.x; o < pw * nc; o += blockDim.x) {
-                const int r = o / nc, j = o - r * nc;
-                double s0 = 0.0, s1 = 0.0;
-                int kk = 0;
-                for (; kk + 1 < kc; kk += 2) {
-                    s0 = fma(Gs[r][kk], Vs[kk][j], s0);
-                    s1 = fma(Gs[r][kk + 1], Vs[kk + 1][j], s1);
-                }
-                if (kk < kc) s0 = fma(Gs[r][kk], Vs[kk][j], s0);
-                pb[(size_t)r * m + c0 + j] = s0 + s1;
             }
         }
         __threadfence();  // this thread's partial sums visible before the count moves

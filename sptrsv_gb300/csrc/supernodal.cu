@@ -439,11 +439,34 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
     CUDA_TRY(cudaMemsetAsync(sn_G.p, 0, sizeof(double) * (size_t)gtot, st));
     k_sn_rectcols<<<std::min(S, sm_count * 8), 128, 0, st>>>(S, sn_start.as<int>(), rp, col, sn_roff.as<int>(),
                                                             sn_m.as<int>() + S, sn_rect.as<int>());
+    ++launches;
+    // (the rectangles are fetched here, before the long kernels, so that the lists are built beside them)
+    // A chunk's step: one more than the latest step of the chunks its rectangle reads.  Rows of panels
+    // are queued step by step, so that the warps in flight always work on a whole step's chunks and not
+    // down one branch of the elimination tree after another.
+    std::vector<int> by_step(S);
+    if (panels_mode() == 0) {
+        std::vector<int> rect(roffh[S]), chunk_of(n), step(S);
+        if (roffh[S] > 0)
+            CUDA_TRY(cudaMemcpyAsync(rect.data(), sn_rect.p, sizeof(int) * roffh[S], cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        for (int s = 0; s < S; ++s) std::fill(chunk_of.begin() + ss[s], chunk_of.begin() + ss[s + 1], s);
+        std::vector<int> count(1, 0);
+        for (int s = S - 1; s >= 0; --s) {
+            for (int q = roffh[s]; q < roffh[s + 1]; ++q) step[s] = std::max(step[s], 1 + step[chunk_of[rect[q]]]);
+            if ((int)count.size() < step[s] + 2) count.resize(step[s] + 2, 0);
+            ++count[step[s] + 1];
+        }
+        for (size_t q = 1; q < count.size(); ++q) count[q] += count[q - 1];
+        for (int s = S - 1; s >= 0; --s) by_step[count[step[s]]++] = s;
+    } else {
+        for (int s = 0; s < S; ++s) by_step[s] = S - 1 - s;
+    }
     k_sn_dinv<<<dim3(S, (wmax + 4 * kInvB - 1) / (4 * kInvB)), 128, 0, st>>>(
         sn_start.as<int>(), rp, val, sn_goff.as<long long>(), sn_ld.as<int>(), sn_G.as<double>());
     k_sn_tinv<<<(unsigned)inv.size(), kInvB * kInvCols, 0, st>>>(
         sn_tasks.as<int2>(), sn_start.as<int>(), rp, val, sn_goff.as<long long>(), sn_ld.as<int>(), sn_G.as<double>());
-    launches += 3;
+    launches += 2;
     if (outbase[S] > 0) {
         k_sn_w<<<sm_count * 16, 256, 0, st>>>(S, sn_start.as<int>(), rp, val, sn_goff.as<long long>(), sn_ld.as<int>(),
                                               sn_m.as<int>(), sn_outbase.as<long long>(), outbase[S],
@@ -456,11 +479,12 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
     CUDA_TRY(cudaGetLastError());
     // FP64 panel records: every 64-row panel of every chunk, its G split into column blocks
     // (panels64.cu).  Items run chunk by chunk from the last; within a chunk, every panel's own
-    // right-hand-side blocks first (no waits), then the solved-row blocks farthest first.
+    // right-hand-side blocks first (no waits), then the solved-row blocks farthest first.  Or its rows
+    // (panel_rows.cu).
     std::vector<BChunk> pan;
     std::vector<int2> pit;
     long long prows = 0;
-    for (int s = S - 1; s >= 0; --s) {
+    for (const int s : by_step) {
         const int w = ss[s + 1] - ss[s], K = w + m[s], nb = p64_nblk(w, K), no = p64_nown(w);
         const int first = (int)pan.size();
         for (int r0 = 0; r0 < w; r0 += kP64) {
@@ -481,6 +505,11 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
             pan.push_back(c);
         }
         const int np = (int)pan.size() - first;
+        if (panels_mode() == 0) {
+            for (int p = first; p < first + np; ++p)
+                for (int q = 0; q * kPanelRows < pan[p].pw; ++q) pit.push_back(make_int2(p, q));
+            continue;
+        }
         for (int q = 0; q < no; ++q)
             for (int p = 0; p < np; ++p) pit.push_back(make_int2(first + p, q));
         for (int q = nb - 1; q >= no; --q)
@@ -527,6 +556,7 @@ int Handle::set_supernodes(int sn, const int* snodes_host) {
     sn_npan = (int)pan.size();
     sn_npitems = (unsigned)pit.size();
     sn_prows = prows;
+    sn_rows = panels_mode() == 0;
     sn_count = S;
     sn_nitems = (int)item_s.size();
     have_supernodes = true;
@@ -550,6 +580,10 @@ SnArgs Handle::sn_args() const {
 
 int launch_sn_solve(const Handle& h, bool mixed, const void* b, void* x, int rhs, int64_t budget, int64_t* launches) {
     if (!mixed) {
+        if (h.sn_rows)
+            return launch_panel_rows(nullptr, rhs, (const double*)b, (double*)x, h.ctl, &h.ctl->ticket, budget,
+                                     h.sn_pitems.as<int2>(), h.sn_npitems, h.sn_pan.as<BChunk>(), 64, h.sm_count, h.st,
+                                     launches);
         // the partial sums (sn_prows x rhs doubles) and the counters (one per panel and RHS group)
         // are sized by Handle::prepare
         const int ncnt = h.sn_npan * p64_groups(rhs);
