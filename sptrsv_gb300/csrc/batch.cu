@@ -675,7 +675,8 @@ __global__ void __launch_bounds__(256) k_b_jacobi_rows(BArgs A, const int4* __re
         if (St.done || St.inner_done) continue;
         const int m = A.sys[s].rhs;
         float mx = 0.f, ch = 0.f;
-        if (m == 1) b_jacobi_rows<1>(A, T, k, 0, src, dst, mx, ch);
+        if (T.w) b_jacobi_rows<4>(A, T, k, T.w & 0xFFFFFF, src, dst, mx, ch);  // four of the columns
+        else if (m == 1) b_jacobi_rows<1>(A, T, k, 0, src, dst, mx, ch);
         else if (m == 2) b_jacobi_rows<2>(A, T, k, 0, src, dst, mx, ch);
         else if (m <= 4) b_jacobi_rows<4>(A, T, k, 0, src, dst, mx, ch);
         else if (m <= 8) b_jacobi_rows<8>(A, T, k, 0, src, dst, mx, ch);
@@ -1221,6 +1222,22 @@ int Batch::build_lists() {
         if (sched[s] == BS_SF32) sf32.push_back(s);
     }
     // row tasks of the mixed systems and of the Jacobi ones
+    // Row tasks, a warp each: as much work as amortises a task's start, less where the batch would otherwise
+    // leave warps of the GPU without one (48 systems, 115k rows: a sweep 56 -> 34 us and a residual 542 -> 58 us
+    // with tasks for every warp).
+    const double warps = (double)sm_count * 64;
+    double work = 0.0, elems = 0.0;
+    for (int s = 0; s < count; ++s) {
+        if (sched[s] == BS_PLAIN || sched[s] == BS_PANEL64) continue;
+        const double nnz_s = (double)((s + 1 < count ? sys[s + 1].nz0 : tot_nnz) - sys[s].nz0);
+        work += nnz_s * std::min(sys[s].rhs, 32);
+        if (sched[s] == BS_JACOBI) elems += (double)sys[s].n * sys[s].rhs;
+    }
+    const double task_work = std::min<double>(kTaskWork, work / warps), task_elems = std::min(1024.0, elems / warps);
+    // A row's columns all in one thread read its entries once, four at a time read four entries' columns at
+    // once: the latter while a warp has little more than one such task, and its chain of loads is the sweep
+    // (34 -> 25 us).
+    const bool narrow = elems < warps * 256.0;
     std::vector<int4> tm, tj;
     for (int s = 0; s < count; ++s) {
         if (sched[s] == BS_PLAIN || sched[s] == BS_PANEL64) continue;
@@ -1228,14 +1245,17 @@ int Batch::build_lists() {
         const int nc = std::min(sys[s].rhs, 32);
         const int rpw = std::max(1, 32 / (nc * sys[s].groups));
         const double per_row = std::max(1.0, (double)nnz_s / sys[s].n) * nc;
-        int rows = (int)std::min<double>(kTaskRowsMax, std::max<double>(rpw, kTaskWork / per_row));
+        int rows = (int)std::min<double>(kTaskRowsMax, std::max<double>(rpw, task_work / per_row));
         rows = std::max(rpw, rows / rpw * rpw);
         for (int r0 = 0; r0 < sys[s].n; r0 += rows) tm.push_back(make_int4(s, r0, std::min(rows, sys[s].n - r0), 0));
         if (sched[s] == BS_JACOBI) {
-            // about 1,024 (row, column) elements per task, whole warps of rows
-            const int jrows = std::max(32, (1024 / sys[s].rhs + 31) / 32 * 32);
+            // (row, column) elements, whole warps of rows
+            const int width = narrow && !jacobi_elem ? std::min(4, sys[s].rhs) : sys[s].rhs;
+            const int jrows = std::max(32, ((int)task_elems / width + 31) / 32 * 32);
             for (int r0 = 0; r0 < sys[s].n; r0 += jrows)
-                tj.push_back(make_int4(s, r0, std::min(jrows, sys[s].n - r0), 0));
+                for (int c0 = 0; c0 < sys[s].rhs; c0 += width)
+                    tj.push_back(make_int4(s, r0, std::min(jrows, sys[s].n - r0),
+                                           width < sys[s].rhs ? c0 | width << 24 : 0));
         }
     }
     n_tasks_mixed = (int)tm.size();
