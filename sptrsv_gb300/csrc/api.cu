@@ -245,13 +245,13 @@ static bool auto_window(double mean_len) {
 
 // Whether FP64 AUTO tries the sweeps (settle.cu) before the exact kernel: when the sweeps of a
 // contracting matrix take less than 0.7 of the exact kernel's time (a matrix that does not contract
-// costs nine of them on top).  Measured on GB300, 8.8 entries a row: 24-31 sweeps of 11 us + 4 us per
-// million entries and columns; the exact kernels take 0.19 us a level with one right-hand side
-// (10k rows 332 us, sweeps 334; 50k rows 1.7 ms, sweeps 0.42) and 2 us with several (200k rows x 8
-// 70 ms, sweeps 1.95).  Tiles of long rows do not fit shared memory.
+// costs nine of them on top).  Measured on GB300, 8.8 entries a row: the time of 22 sweeps of 9 us + 4.5 us
+// per million entries and columns (10k rows 207 us, 2M rows 1.8 ms, 200k rows x 8 1.35 ms); the exact
+// kernels take 0.19 us a level with one right-hand side (10k rows 370 us, 50k rows 1.7 ms) and 2 us with
+// several (200k rows x 8 70 ms).  Tiles of long rows do not fit shared memory.
 bool Handle::settle_pays(int rhs) const {
     const double depth = levels_ready ? (double)max_level : depth_est;
-    const double sweeps_us = 28.0 * (11.0 + 4.0e-6 * (double)nnz * rhs);
+    const double sweeps_us = 22.0 * (9.0 + 4.5e-6 * (double)nnz * rhs);
     return mean_len <= kSettleMaxLen && sweeps_us < 0.7 * (rhs == 1 ? 0.19 : 2.0) * depth;
 }
 

@@ -9,14 +9,15 @@
 // settle_hopeless) and solved by the exact kernel launched behind this one, which returns at once
 // when this one has finished (ctl->done).
 //
-// When it stands still: every row's new value differs from the one it replaces by less than 2^-50 of
+// When it stands still: every row's new value differs from the one it replaces by less than 2^-48 of
 // the largest of |x_i|, |b_i / U_ii| and the terms |U_ij x_j / U_ii| it is formed from.  That is the
-// size of the rounding error substitution itself may make in forming x_i (k + 1 half-ulps of the sum
-// of k terms; eight terms a row), so the result is substitution's with local errors of the same size,
-// and what is left after the last sweep has contracted once more.  Measured against 64-bit references
+// size of the rounding error substitution itself may make in forming x_i (k + 1 half-ulps of the sum of
+// k terms' sizes: 2^-48 of the largest for eight terms), so the result is substitution's with local errors
+// of the same size, and what is left after the last sweep has contracted once more.  By then a few hundred
+// rows of millions still move by more than an ulp.  Measured against 64-bit references
 // at 10k to 2M rows: 1.1e-16 in norm (the exact kernels: 1.1e-16 to 1.6e-16) and at most 1e-15 of the
-// root mean square, with bounds of 2^-52 to 2^-49 alike.  (Waiting for equal bits takes the sweeps of the
-// slowest rounding flip: twice as many.)
+// root mean square, with bounds of 2^-52 to 2^-48 alike.  (A sweep gains about four bits; after the 13 or so
+// that bring most rows there, the slowest rounding flips take as many again to die out.)
 //
 // Sweep order.  Each warp owns a contiguous run of rows and walks it upwards from its bottom, 32 rows
 // a tile (lane per row; 32 / NC rows for NC right-hand sides), writing x in place: a row sees this
@@ -25,11 +26,13 @@
 // and cost the most sweeps, so with one right-hand side a tile's changes are folded in once more
 // before they are written (k_settle, "second look"): half the sweeps for a third more arithmetic.
 //
-// Bound by the FP64 pipe (57 % active by ncu at 500k rows; 2 FMAs a clock and SM, and a tile takes its
-// longest row's count: 1.9 times the mean of 7.6 off-diagonals) and, below ~200k rows, by the chain of
-// loads and FMAs through a tile.  Measured on GB300, 8.8 entries a row: 2M rows 68 -> 3.1 ms (24
-// sweeps), 200k rows 6.9 -> 0.60 ms (31), 50k rows 1.7 -> 0.42 ms (28); 200k rows x 8 columns 70 ->
-// 1.95 ms (33).
+// Bound by the FP64 pipe (57 % active by ncu at 500k rows; an operation holds its SM quarter's pipe for 64
+// cycles, and a tile takes its longest row's count, 1.9 times the mean of 7.6 off-diagonals) and, below
+// ~200k rows, by the chain of loads and FMAs through a tile.  Measured on GB300, 8.8 entries a row: 2M rows
+// 68 -> 1.8 ms (16 sweeps), 200k rows 6.9 -> 0.44 ms (18), 50k rows 1.7 -> 0.28 ms (19); 200k rows x 8 columns
+// 70 -> 1.35 ms (22).  Tried and not kept: two FP32 corrections first (their sweeps are bound by instructions
+// and L1, 90 us against 120 at 2M rows: 3.4 ms in all against 3.1 then), rows kept in shared memory for all
+// sweeps (200k rows 0.40, but 200k x 8 1.69), 16-byte copies for the staging (no change).
 //
 // One cooperative launch runs all sweeps, with a grid barrier after each; x of other warps' rows may
 // be read old or new within a sweep, and is new after the barrier.
@@ -42,12 +45,8 @@ namespace sptrsv {
 
 constexpr int kSetWarps = 8;
 constexpr size_t kSetSmem = 220 * 1024;
-// Tiles of the shortest run: longer runs take fewer sweeps (fewer rows see a neighbour's old values),
-// shorter ones spread further: 10k rows 325 / 392 / 514 us at 1 / 2 / 4 tiles, 60k rows x 16 columns
-// 1776 / 1538 / 1586 us.
-constexpr int kSetMinTiles = 2;
 constexpr int kSetPending = 5000;  // offset of a sweep's record: 0 = nothing changed
-constexpr int kSetStill = kSetPending - 51;  // changes below 2^-50 (the exponents are floors)
+constexpr int kSetStill = kSetPending - 49;  // changes below 2^-48 (the exponents are floors)
 
 struct SettleArgs {
     int n, rhs;
@@ -66,15 +65,30 @@ struct SettleArgs {
 
 template <int NC> struct SetShape {
     static constexpr int kRows = 32 / NC;  // rows of a tile
+    // One right-hand side: a tile's buffer at a time and three CTAs an SM (2M rows 1.81 ms; two buffers and
+    // two CTAs 2.11, one and two 2.11, one and four 2.14).  Several: two buffers, two CTAs (200k rows x 8
+    // 1.35 ms; one and three 1.42).
+    static constexpr int kBufs = NC == 1 ? 1 : 2;
+    static constexpr int kCtas = NC == 1 ? 3 : 2;
 };
 
-// Bytes of a warp's buffers: two tiles of `cap` staged entries (columns and values), one tile's x at
+// Bytes of a warp's buffers: one or two tiles of `cap` staged entries (columns and values), one tile's x at
 // every entry (cap * NC), the tile's changes.
-__host__ __device__ __forceinline__ size_t set_warp_bytes(int cap, int nc) {
-    return (size_t)cap * (2 * 12 + 8 * nc) + 32 * 8;
+__host__ __device__ __forceinline__ size_t set_warp_bytes(int cap, int nc, int bufs) {
+    return (size_t)cap * (bufs * 12 + 8 * nc) + 32 * 8;
 }
 
 __device__ __forceinline__ int d_exp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+
+// Exponent of |a - b|, a != b, within one, from their bits (an FP64 subtraction would hold the pipe for 64
+// cycles): bit patterns of one sign are ordered like the values and a unit in the last place apart; with
+// the signs or the exponents further apart the larger value's exponent.
+__device__ __forceinline__ int d_gap(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    const int ea = d_exp(a), eb = d_exp(b), hi = max(ea, eb), lo = min(ea, eb);
+    if ((x ^ y) < 0 || hi - lo > 1) return hi;
+    return lo - 52 + 63 - __clzll(x > y ? x - y : y - x);
+}
 
 // After sweep p (from 0): whether to leave the matrix to the exact kernel.  From the ninth sweep on the
 // largest change has to lose at least a bit a sweep over the last four, until it is within 2^-40 of
@@ -104,18 +118,18 @@ __device__ __forceinline__ double set_ld(const double* p, bool own) {
 }
 
 template <int NC>
-__global__ void __launch_bounds__(kSetWarps * 32, 2) k_settle(SettleArgs A) {
-    constexpr int R = SetShape<NC>::kRows;
+__global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(SettleArgs A) {
+    constexpr int R = SetShape<NC>::kRows, B = SetShape<NC>::kBufs;
     extern __shared__ __align__(16) char set_smem[];
     __shared__ int s_worst;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = lane / NC, j0 = lane % NC;
     const int n = A.n, m = A.rhs, cap = A.cap;
-    char* base = set_smem + warp * set_warp_bytes(cap, NC);
-    double* sv = (double*)base;            // [2][cap] values
-    double* sx = sv + 2 * cap;             // [cap][NC] x at the tile's entries
+    char* base = set_smem + warp * set_warp_bytes(cap, NC, B);
+    double* sv = (double*)base;            // [B][cap] values
+    double* sx = sv + B * cap;             // [cap][NC] x at the tile's entries
     double* dl = sx + cap * NC;            // [32] the tile's changes
-    int* sc = (int*)(dl + 32);             // [2][cap] columns
+    int* sc = (int*)(dl + 32);             // [B][cap] columns
     const int ntiles = (n + R - 1) / R;
     const int t0 = min((int)(blockIdx.x * kSetWarps + warp) * A.tiles, ntiles), t1 = min(t0 + A.tiles, ntiles);
     const int run_top = n - R * t0;
@@ -157,12 +171,13 @@ __global__ void __launch_bounds__(kSetWarps * 32, 2) k_settle(SettleArgs A) {
         __syncthreads();
         int worst = 0;
         Rows cur = rows_of(t0);
-        stage(cur, 0);
+        if (B == 2) stage(cur, 0);
         Rows nxt = rows_of(t0 + 1);
         for (int t = t0; t < t1; ++t) {
-            const int buf = (t - t0) & 1;
+            const int buf = (t - t0) & (B - 1);
             const int top = n - R * t, lo = max(0, top - R), i = lo + r;
-            stage(nxt, buf ^ 1);
+            if (B == 2) stage(nxt, buf ^ 1);
+            else stage(cur, 0);
             const Rows after = rows_of(t + 2);
             const bool staged = cur.e1 - cur.e0 <= cap;
             const double* pv = sv + buf * cap - cur.e0;
@@ -180,7 +195,8 @@ __global__ void __launch_bounds__(kSetWarps * 32, 2) k_settle(SettleArgs A) {
                 }
                 const int eb = d_exp(bi);
                 if (jb == 0) {
-                    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+                    if (B == 2) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+                    else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
                     __syncwarp();
                 }
                 if (staged) {
@@ -225,20 +241,21 @@ __global__ void __launch_bounds__(kSetWarps * 32, 2) k_settle(SettleArgs A) {
                     dl[lane] = mine && __double_as_longlong(y) != __double_as_longlong(old) ? y - old : 0.0;
                     __syncwarp();
                     if (mine) {
+                        double more = 0.0;
                         for (int k = cur.s; inside > 0; ++k) {
                             const int c = staged ? pc[k] : __ldg(A.col + k);
                             if (c < top) {
-                                acc = fma(staged ? pv[k] : __ldg(A.val + k), dl[c - lo], acc);
+                                more = fma(staged ? pv[k] : __ldg(A.val + k), dl[c - lo], more);
                                 --inside;
                             }
                         }
-                        y = (bi - acc) * di;
+                        y = fma(-more, di, y);
                     }
                 }
                 if (mine && __double_as_longlong(y) != __double_as_longlong(old)) {
                     const int ei = d_exp(di) - 1023;
                     const int size = max(d_exp(y), max(eb, (int)(em >> 20) - 1023) + ei);
-                    const int gap = d_exp(y - old) - size;
+                    const int gap = d_gap(y, old) - size;
                     worst = max(worst, gap + kSetPending);
                     A.x[at] = y;
                 }
@@ -281,16 +298,20 @@ static int settle_t(const SolveArgs& a, int* worst) {
     constexpr int R = SetShape<NC>::kRows;
     // staged entries: the mean tile and four deviations of a Poisson count, if shared memory holds it
     const double mean = R * (double)a.nnz / a.n;
-    const int fit = (int)((kSetSmem / kSetWarps - 256) / (24 + 8 * NC));
+    const int fit = (int)((kSetSmem / kSetWarps - 256) / (12 * SetShape<NC>::kBufs + 8 * NC));
     const int cap = std::min(fit, (int)(mean + 4.0 * std::sqrt(mean)) + 15) / 8 * 8;
-    const size_t bytes = kSetWarps * set_warp_bytes(cap, NC);
+    const size_t bytes = kSetWarps * set_warp_bytes(cap, NC, SetShape<NC>::kBufs);
     const void* fn = (const void*)k_settle<NC>;
     CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSetWarps * 32, bytes));
     if (per_sm < 1) return SPTRSV_ERR_UNSUPPORTED;
     const int ntiles = (a.n + R - 1) / R;
-    const int warps = std::max(1, std::min(per_sm * a.sm_count * kSetWarps, ntiles / kSetMinTiles));
+    // Tiles of the shortest run: longer runs take fewer sweeps (fewer rows see a neighbour's old values),
+    // shorter ones spread further.  One right-hand side: 10k rows 207 / 278 / 291 us at 1 / 2 / 3 tiles, 50k
+    // rows 290 / 282 / 283, 200k rows 489 / 496 / 435.  Several: 10k rows x 8 310 / 384 us at 2 / 4.
+    const int shortest = NC > 1 ? 2 : ntiles <= a.sm_count * kSetWarps ? 1 : 3;
+    const int warps = std::max(1, std::min(per_sm * a.sm_count * kSetWarps, ntiles / shortest));
     SettleArgs s{a.n, a.rhs, a.rp, a.col, (const double*)a.val, (const double*)a.invd, (const double*)a.b, (double*)a.x,
                  a.ctl, worst, a.budget, (ntiles + warps - 1) / warps, cap};
     const int grid = ((ntiles + s.tiles - 1) / s.tiles + kSetWarps - 1) / kSetWarps;
