@@ -130,8 +130,14 @@ static int solve_host_timed(Handle* h, const sptrsv_opts& o, const double* b, do
     // warm the graph cache / allocations outside the timed region
     sptrsv_opts r = h->resolve(&o, rhs);
     if ((rc = h->prepare(r, rhs, layout))) return rc;
+    // One solve per matrix: its kernels are launched directly.  Capturing and instantiating a graph to run
+    // it once costs ~40 us; only the device-looped refinement needs one.
     CUDA_TRY(cudaEventRecord(h->ev0, h->st));
-    if ((rc = h->solve(&o, h->db.as<double>(), h->dx.as<double>(), rhs, layout))) return rc;
+    const bool graphs = h->use_graphs;
+    if (!h->cond_eligible(r, rhs)) h->use_graphs = false;
+    rc = h->solve(&o, h->db.as<double>(), h->dx.as<double>(), rhs, layout);
+    h->use_graphs = graphs;
+    if (rc) return rc;
     CUDA_TRY(cudaEventRecord(h->ev1, h->st));
     CUDA_TRY(cudaMemcpyAsync(x, h->dx.p, bytes, cudaMemcpyDeviceToHost, h->st));
     rc = h->sync();
@@ -143,19 +149,20 @@ static int solve_host_timed(Handle* h, const sptrsv_opts& o, const double* b, do
 }
 
 // Whether FP64 accuracy through refinement (FP32 Jacobi sweeps, FP64 residuals) should beat the
-// exact sync-free solve by a wide margin: the exact solve waits one dependent global-memory hop
-// (~1 us on GB300) per level of the DAG (the analysis's depth estimate when the levels have not
-// been computed); the refinement makes about 40 bandwidth-bound sweeps and 4 FP64 residual
-// passes, and needs sweeps that contract (every row strictly dominant).
+// exact sync-free solve by a wide margin, where FP64 AUTO does not sweep itself (Handle::settle_pays):
+// the exact solve takes ~0.19 us per level of the DAG with one right-hand side and ~1 us with several
+// (the analysis's depth estimate when the levels have not been computed); the refinement makes about 40
+// sweeps (bandwidth, and ~12 us each with its test in the graph's loop: 5,000 rows 400 us against 170 for
+// the exact solve) and 4 FP64 residual passes, and needs sweeps that contract (every row strictly dominant).
 static bool refinement_pays(const Handle* h, int rhs) {
     // dense skyline rows go to the exact FP64 panels instead
     if (!(h->max_ratio < 1.0) || rhs > 1024 || h->dense_skyline()) return false;
     const double depth = h->levels_ready ? (double)h->max_level : h->depth_est;
     const double n = h->n, nnz = h->nnz;
-    const double sweep_s = (8.0 * (nnz - n) + 16.0 * n * rhs) / 4.0e12 + 4.0e-6;
+    const double sweep_s = (8.0 * (nnz - n) + 16.0 * n * rhs) / 4.0e12 + 12.0e-6;
     const double resid_s = (12.0 * nnz + 24.0 * n * rhs) / 3.5e12 + 4.0e-6;
     const double refined_s = 40.0 * sweep_s + 4.0 * resid_s;
-    const double exact_s = 1.0e-6 * depth;
+    const double exact_s = (rhs == 1 ? 0.19e-6 : 1.0e-6) * depth;
     return refined_s < 0.25 * exact_s;
 }
 
@@ -167,13 +174,13 @@ static sptrsv_opts fp64(int schedule) {
 }
 
 // The FP64 solve of the serial-substitution entry points (any schedule whose result meets the
-// serial solve's accuracy): for deep DAGs with dominant rows, FP64 accuracy through refinement
-// with the exact AUTO solve if it stalls; otherwise the exact AUTO solve.  *secs: device time of
+// serial solve's accuracy): the AUTO solve, or, for deep DAGs with dominant long rows, FP64 accuracy
+// through refinement with the AUTO solve if it stalls.  *secs: device time of
 // the solves made.
 static int solve_fp64_host(Handle* h, const double* b, double* x, int rhs, double* secs) {
     *secs = 0.0;
     int rc;
-    if (refinement_pays(h, rhs)) {
+    if (!h->settle_pays(rhs) && refinement_pays(h, rhs)) {
         sptrsv_opts o = fp64(SPTRSV_SCHED_JACOBI);
         o.max_refine = 6;
         rc = solve_host_timed(h, o, b, x, rhs, SPTRSV_COL_MAJOR, secs);
