@@ -69,6 +69,7 @@ int Handle::read_ctl(Ctl* out) {
 }
 
 int Handle::reset_ctl() {
+    ctl_copied = false;
     CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     return 0;
 }
@@ -552,6 +553,12 @@ int Handle::enqueue(const sptrsv_opts& o, const double* b, double* x, int rhs, i
         if ((rc = launch_transpose(false, xrm, x, n, rhs, st, &launches))) return rc;
         if ((rc = mark(SPTRSV_K_TRANSPOSE))) return rc;
     }
+    return copy_ctl();
+}
+
+// The control block to the host as the solve's last step, so that sync() waits once and reads it there.
+int Handle::copy_ctl() {
+    CUDA_TRY(cudaMemcpyAsync(h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
     return 0;
 }
 
@@ -753,6 +760,7 @@ int Handle::build_cond_graph(const sptrsv_opts& o, const double* b, double* x, d
         if (!rc) rc = launch_refine_init(ra, true);
         if (!rc && add_while(g, ho, &obody) != cudaSuccess) rc = SPTRSV_ERR_CUDA;
         if (!rc && conv) rc = launch_transpose(false, xrm, x, n, rhs, st, &scratch_launches);
+        if (!rc) rc = copy_ctl();
         cudaGraph_t g2 = nullptr;
         cudaError_t e2 = cudaStreamEndCapture(st, &g2);
         if (!rc && e2 != cudaSuccess) rc = set_cuda_error(e2, "capture top");
@@ -800,6 +808,13 @@ int Handle::build_cond_graph(const sptrsv_opts& o, const double* b, double* x, d
 }
 
 int Handle::solve(const sptrsv_opts* o_in, const double* b, double* x, int rhs, int layout) {
+    ctl_copied = false;
+    const int rc = run_solve(o_in, b, x, rhs, layout);
+    ctl_copied = rc == 0;
+    return rc;
+}
+
+int Handle::run_solve(const sptrsv_opts* o_in, const double* b, double* x, int rhs, int layout) {
     if (!analysed) return SPTRSV_ERR_NO_ANALYSIS;
     if (rhs < 1 || !b || !x || (layout != SPTRSV_COL_MAJOR && layout != SPTRSV_ROW_MAJOR)) return SPTRSV_ERR_INVALID_ARG;
     if ((size_t)n * rhs > (size_t)0x7fffffff) return SPTRSV_ERR_TOO_LARGE;
@@ -890,8 +905,8 @@ int Handle::solve(const sptrsv_opts* o_in, const double* b, double* x, int rhs, 
 int Handle::sync() {
     CUDA_TRY(cudaStreamSynchronize(st));
     Ctl c{};
-    int rc = read_ctl(&c);
-    if (rc) return rc;
+    if (ctl_copied) c = *h_ctl;
+    else if (int rc = read_ctl(&c)) return rc;
     if (c.status) return c.status;
     if (last_mixed) {
         last_steps = c.steps;
@@ -947,6 +962,7 @@ Handle::~Handle() {
                       &sn_G, &sn_Ghi, &sn_Glo, &sn_pan, &sn_pitems, &sn_pcnt, &sn_ppart, &sn_gtc, &sn_tcrec, &sn_ghl, &sn_gexp, &tune_b, &tune_x};
     for (DevBuf* b : bufs) b->release();
     if (ctl) cudaFree(ctl);
+    if (h_ctl) cudaFreeHost(h_ctl);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (st) cudaStreamDestroy(st);
@@ -1019,6 +1035,7 @@ int sptrsv_create(sptrsv_handle* out, int device) {
         if ((er = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking)) != cudaSuccess) { rc = sptrsv::set_cuda_error(er, "stream"); break; }
         if ((er = cudaEventCreate(&h->ev0)) != cudaSuccess) { rc = sptrsv::set_cuda_error(er, "event"); break; }
         if ((er = cudaEventCreate(&h->ev1)) != cudaSuccess) { rc = sptrsv::set_cuda_error(er, "event"); break; }
+        if ((er = cudaMallocHost(&h->h_ctl, sizeof(sptrsv::Ctl))) != cudaSuccess) { rc = sptrsv::set_cuda_error(er, "ctl"); break; }
         if ((er = cudaMalloc(&h->ctl, sizeof(sptrsv::Ctl))) != cudaSuccess) { rc = sptrsv::set_cuda_error(er, "ctl"); break; }
         // a new control block reports no status until a solve or analysis writes one
         if ((er = cudaMemsetAsync(h->ctl, 0, sizeof(sptrsv::Ctl), h->st)) != cudaSuccess ||

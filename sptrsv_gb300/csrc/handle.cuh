@@ -67,6 +67,8 @@ struct Handle {
     int sm_count = 0;
     int64_t launches = 0;
     Ctl* ctl = nullptr;
+    Ctl* h_ctl = nullptr;       // pinned: the control block as the last solve left it
+    bool ctl_copied = false;    // a solve that ends with that copy is the last thing on the stream
     bool use_graphs = true;
     int sweep_kernel = 0;   // 0 bulk-copy pipelined sweeps, 1 warp tiles with plain loads
     int warps_override = 0;
@@ -181,7 +183,9 @@ struct Handle {
     cudaStream_t cancel_st = nullptr;
     int* cancel_flag = nullptr;  // pinned host 1
     int features(float* f, int rhs);
+    int copy_ctl();
     int solve(const sptrsv_opts* o, const double* b, double* x, int rhs, int layout);
+    int run_solve(const sptrsv_opts* o, const double* b, double* x, int rhs, int layout);
     int sync();
 };
 
