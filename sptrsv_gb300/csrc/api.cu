@@ -134,6 +134,12 @@ static int levels_kernel() {
     return k;
 }
 
+// Width of a row's level, averaged over the rows, up to which the buckets are ranked instead of sorted.
+// GB300, rows of one dependency `w` columns on: w = 32, 4,000 / 500,000 rows 168 / 350 us of analysis
+// sorted, 149 / 289 us ranked; w = 512, 171 / 2,644 against 152 / 2,655; w = 2,048, 500,000 rows 2,657
+// against 2,918.
+constexpr double kRankWidth = 256.0;
+
 // Levels (core.cpp:244-270) and level buckets (core.cpp:282-288), computed on first need.
 int Handle::ensure_levels() {
     if (levels_ready) return 0;
@@ -169,27 +175,25 @@ int Handle::ensure_levels() {
         found = c.max_level;
     }
     max_level = found;
-    // level buckets: counts -> level_ptr; stable radix sort of level keys -> level_rows
+    // level buckets: counts -> level_ptr; the rows by rank within their levels, or a stable radix sort of
+    // the level keys -> level_rows
     if ((rc = level_ptr.ensure(sizeof(int) * (size_t)(max_level + 2)))) return rc;
     if ((rc = level_rows.ensure(sizeof(int) * (size_t)n))) return rc;
-    const size_t need = sort_scratch(n) + (size_t)(max_level + 2 + scan_partials_needed(max_level + 1)) * sizeof(int) + 4096;
+    const size_t need = sort_scratch(n) + ((size_t)n + max_level + 2 + scan_partials_needed(max_level + 1)) * sizeof(int) + 4096;
     if ((rc = scratch.ensure(need))) return rc;
     Scratch scr{(char*)scratch.p, scratch.cap, 0};
+    unsigned long long* passes = scr.take<unsigned long long>(3);
     int* cnt = scr.take<int>(max_level + 2);
     int* part = scr.take<int>(scan_partials_needed(max_level + 1));
+    int* slot = scr.take<int>(n);
     CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)(max_level + 2), st));
-    k_level_hist<<<sgrid, 256, 0, st>>>(n, levels.as<int>(), cnt);
+    k_level_hist<<<sgrid, 256, 0, st>>>(n, levels.as<int>(), cnt, slot);
     ++launches;
     if ((rc = scan_exclusive(cnt, level_ptr.as<int>(), max_level + 1, part, st, &launches))) return rc;
-    int bits = 0;
-    while ((1ll << bits) <= (long long)max_level) ++bits;
-    if ((rc = stable_sort_perm((const unsigned*)levels.p, n, bits, level_rows.as<int>(), scr, st, &launches)))
-        return rc;
     // level-set grid: one CTA when its cost model wins.  Measured on GB300: a level costs ~0.3 us of
     // CTA barrier plus ~0.5 us per pass of 32 rows with one CTA; a grid barrier through L2 costs
     // ~1.5 us (one GPU-scope acq_rel atomic per CTA, acquire polls) plus ~0.5 us per pass.
-    unsigned long long* passes = scr.take<unsigned long long>(2);
-    unsigned long long hp[2] = {0, 0};
+    unsigned long long hp[3] = {0, 0, 0};
     CUDA_TRY(cudaMemsetAsync(passes, 0, sizeof(hp), st));
     if (max_level > 0) {
         k_level_passes<<<(max_level + 255) / 256, 256, 0, st>>>(max_level, level_ptr.as<int>(), sm_count, passes);
@@ -198,6 +202,20 @@ int Handle::ensure_levels() {
     CUDA_TRY(cudaMemcpyAsync(hp, passes, sizeof(hp), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     levelset_one_cta = 0.3 * max_level + 0.5 * (double)hp[0] < 1.5 * max_level + 0.5 * (double)hp[1];
+    if ((double)hp[2] <= kRankWidth * n) {
+        int* placed = scr.take<int>(n);
+        if (!slot || !placed) return SPTRSV_ERR_CUDA;
+        k_level_place<<<sm_count * 8, 256, 0, st>>>(n, levels.as<int>(), level_ptr.as<int>(), slot, placed);
+        k_level_rank<<<sm_count * 8, 256, 0, st>>>(n, levels.as<int>(), level_ptr.as<int>(), placed, level_rows.as<int>());
+        launches += 2;
+        CUDA_TRY(cudaGetLastError());
+    } else {
+        int bits = 0;
+        while ((1ll << bits) <= (long long)max_level) ++bits;
+        if ((rc = stable_sort_perm((const unsigned*)levels.p, n, bits, level_rows.as<int>(), scr, st, &launches)))
+            return rc;
+    }
+    CUDA_TRY(cudaStreamSynchronize(st));
     levels_ready = true;
     return 0;
 }

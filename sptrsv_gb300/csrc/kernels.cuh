@@ -31,7 +31,9 @@ int launch_check_rows(int n, int nnz, const int* rp, const int* col, const doubl
                       int64_t* launches);
 __global__ void k_to_f32(size_t count, const double* a, float* b);
 __global__ void k_levels(int n, const int* rp, const int* col, int* level, Ctl* ctl, int64_t budget);
-__global__ void k_level_hist(int n, const int* level, int* cnt);
+__global__ void k_level_hist(int n, const int* level, int* cnt, int* slot);
+__global__ void k_level_place(int n, const int* level, const int* lptr, const int* slot, int* placed);
+__global__ void k_level_rank(int n, const int* level, const int* lptr, const int* placed, int* lrows);
 __global__ void k_level_tasks(int max_level, const int* lptr, const int* lrows, const int* rp, int T, int* tasks);
 __global__ void k_level_passes(int max_level, const int* lptr, int ctas, unsigned long long* out);
 __global__ void k_entry_rows(int n, const int* rp, int* erow);
