@@ -730,7 +730,7 @@ bool Handle::cond_eligible(const sptrsv_opts& o, int rhs) const {
 }
 
 int Handle::build_cond_graph(const sptrsv_opts& o, const double* b, double* x, double* x_out, int rhs, int layout,
-                             cudaGraphExec_t* out, int64_t* fixed_kernels) {
+                             bool loop, cudaGraphExec_t* out, int64_t* fixed_kernels) {
     *out = nullptr;
     const bool conv = rhs > 1 && layout == SPTRSV_COL_MAJOR;
     const double* brm = conv ? bw.as<double>() : b;
@@ -745,7 +745,7 @@ int Handle::build_cond_graph(const sptrsv_opts& o, const double* b, double* x, d
     CUDA_TRY(cudaGraphCreate(&g, 0));
     cudaGraphConditionalHandle ho = 0, hi = 0;
     cudaError_t e = cudaGraphConditionalHandleCreate(&ho, g, 1, cudaGraphCondAssignDefault);
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&hi, g, 0, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess && !loop) e = cudaGraphConditionalHandleCreate(&hi, g, 0, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) { cudaGraphDestroy(g); return set_cuda_error(e, "conditional handle"); }
     cudaGraph_t obody = nullptr, ibody = nullptr;
     const float eps = powf(10.f, -(float)o.inner_tol_exp);
@@ -786,14 +786,18 @@ int Handle::build_cond_graph(const sptrsv_opts& o, const double* b, double* x, d
         rc = set_cuda_error(e, "begin capture top");
     }
     const int64_t fixed = scratch_launches;
-    // outer body: residual (seeds d0), test, WHILE(inner), x += d
+    // outer body: residual (seeds d0), test, then the inner solve and x += d as one kernel or WHILE(inner), x += d
     if (!rc) {
         e = cudaStreamBeginCaptureToGraph(st, obody, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
         if (e == cudaSuccess) {
             rc = launch_residual(ra, true, 0);
             if (!rc) rc = launch_check_outer(ra, o.max_refine, ho, hi);
-            if (!rc && add_while(obody, hi, &ibody) != cudaSuccess) rc = SPTRSV_ERR_CUDA;
-            if (!rc) rc = launch_axpy_pending(ra, 0);
+            if (loop) {
+                if (!rc) rc = launch_jacobi_loop(ra, eps, max_sweeps);
+            } else {
+                if (!rc && add_while(obody, hi, &ibody) != cudaSuccess) rc = SPTRSV_ERR_CUDA;
+                if (!rc) rc = launch_axpy_pending(ra, 0);
+            }
             cudaGraph_t g2 = nullptr;
             cudaError_t e2 = cudaStreamEndCapture(st, &g2);
             if (!rc && e2 != cudaSuccess) rc = set_cuda_error(e2, "capture outer");
@@ -802,7 +806,7 @@ int Handle::build_cond_graph(const sptrsv_opts& o, const double* b, double* x, d
         }
     }
     // inner body: two sweeps (d0 -> d1 -> d0), the second measuring its change, then the test
-    if (!rc) {
+    if (!rc && !loop) {
         e = cudaStreamBeginCaptureToGraph(st, ibody, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
         if (e == cudaSuccess) {
             rc = launch_jacobi_sweep(ra, 0, false, false);
@@ -861,6 +865,7 @@ int Handle::run_solve(const sptrsv_opts* o_in, const double* b, double* x, int r
             CUDA_TRY(cudaGraphLaunch(g.exec, st));
             launches += g.kernels;
             last_cond = cond;
+            last_loop = g.loop;
             last_mirrored = key.xo != nullptr;
             cond_fixed_kernels = g.kernels;
             return 0;
@@ -869,10 +874,18 @@ int Handle::run_solve(const sptrsv_opts* o_in, const double* b, double* x, int r
     if (cond) {
         cudaGraphExec_t exec = nullptr;
         int64_t fixed = 0;
-        rc = build_cond_graph(o, b, x, key.xo, rhs, layout, &exec, &fixed);
+        RefineArgs ra{};
+        if ((rc = refine_args(o, b, x, rhs, &ra))) return rc;
+        bool loop = refine_loops(ra);
+        rc = build_cond_graph(o, b, x, key.xo, rhs, layout, loop, &exec, &fixed);
+        if (loop && (rc || !exec)) {  // a body that takes no cooperative kernel (under MPS)
+            loop = false;
+            rc = build_cond_graph(o, b, x, key.xo, rhs, layout, loop, &exec, &fixed);
+        }
         if (!rc && exec) {
             GraphEntry ge;
             ge.key = key;
+            ge.loop = loop;
             ge.exec = exec;
             ge.kernels = fixed;
             if (graphs.size() >= 16) {
@@ -883,6 +896,7 @@ int Handle::run_solve(const sptrsv_opts* o_in, const double* b, double* x, int r
             CUDA_TRY(cudaGraphLaunch(exec, st));
             launches += fixed;
             last_cond = true;
+            last_loop = loop;
             last_mirrored = key.xo != nullptr;
             cond_fixed_kernels = fixed;
             return 0;
@@ -931,8 +945,9 @@ int Handle::sync() {
         last_sweeps = c.inner_total;
         last_res = c.rel_res;
         if (last_cond) {
-            // per outer iteration: residual, test, axpy; per inner pair: two sweeps + test
-            launches += 3ll * (c.steps + 1) + c.inner_total + c.inner_total / 2;
+            // per outer iteration: residual, test, inner solve or axpy; per inner pair of a WHILE node: two
+            // sweeps + test
+            launches += 3ll * (c.steps + 1) + (last_loop ? 0 : c.inner_total + c.inner_total / 2);
             last_cond = false;
         }
         if (!c.done) return SPTRSV_ERR_NOT_CONVERGED;
@@ -1063,8 +1078,8 @@ int sptrsv_create(sptrsv_handle* out, int device) {
     if (rc) { delete h; return rc; }
     const char* g = getenv("SPTRSV_NO_GRAPH");
     h->use_graphs = !(g && g[0] == '1');
-    // tuning override of the Jacobi sweep kernel (default: lane per row over entry pairs): jds,
-    // batch8, batch4, direct, tile, tile8, direct2, tma, sell
+    // tuning override of the Jacobi sweep kernel (default: lane per row over entry pairs, copied ahead): jds,
+    // batch8, batch4, direct, tile, tile8, direct2, sell
     const char* sk = getenv("SPTRSV_SWEEP_KERNEL");
     h->sweep_kernel = 0;
     if (sk && strcmp(sk, "sell") == 0) h->sweep_kernel = 6;
@@ -1075,7 +1090,6 @@ int sptrsv_create(sptrsv_handle* out, int device) {
     if (sk && strcmp(sk, "direct") == 0) h->sweep_kernel = 2;
     if (sk && strcmp(sk, "tile8") == 0) h->sweep_kernel = 3;
     if (sk && strcmp(sk, "direct2") == 0) h->sweep_kernel = 4;
-    if (sk && strcmp(sk, "tma") == 0) h->sweep_kernel = 5;
     *out = reinterpret_cast<sptrsv_handle>(h);
     return 0;
 }

@@ -41,7 +41,8 @@ struct Ctl {
     int inner_count;       // MIXED + JACOBI: sweeps of the current inner solve
     int inner_total;       // MIXED + JACOBI: sweeps over the whole solve
     int x_zero;            // MIXED: x is still the zero start vector (the residual is b)
-    float inner_eps;       // MIXED + JACOBI: change test of the next inner solve, from the last residual
+    float inner_eps;       // MIXED + JACOBI: change test of the next inner solve, from the last residual (< 0: none)
+    unsigned int dmax2_bits, dchg2_bits;  // MIXED + JACOBI: as dmax_bits and dchg_bits, every other pair of sweeps
 };
 
 template <typename T> struct Pend;

@@ -58,6 +58,7 @@ struct GraphEntry {
     GraphKey key;
     cudaGraphExec_t exec = nullptr;
     int64_t kernels = 0;
+    bool loop = false;  // conditional graph whose inner solves are one launch each
 };
 
 struct Handle {
@@ -70,7 +71,7 @@ struct Handle {
     Ctl* h_ctl = nullptr;       // pinned: the control block as the last solve left it
     bool ctl_copied = false;    // a solve that ends with that copy is the last thing on the stream
     bool use_graphs = true;
-    int sweep_kernel = 0;   // 0 bulk-copy pipelined sweeps, 1 warp tiles with plain loads
+    int sweep_kernel = 0;   // RefineArgs::sweep_kernel
     int warps_override = 0;
 
     // matrix (device; either owned copies or caller-owned pointers)
@@ -132,6 +133,7 @@ struct Handle {
     unsigned flush_byte = 1;
     bool last_mixed = false;
     bool last_cond = false;       // the last solve ran the conditional (device-looped) graph
+    bool last_loop = false;       // ... with one launch per inner solve
     double* x_mirror = nullptr;   // set by sptrsv_solve_host around solve(): pinned host x for the residuals
     bool last_mirrored = false;   // the last solve's residual kernels wrote x_mirror
     int64_t cond_fixed_kernels = 0;
@@ -167,7 +169,7 @@ struct Handle {
     bool cond_eligible(const sptrsv_opts& o, int rhs) const;
     int refine_args(const sptrsv_opts& o, const double* b, double* x, int rhs, RefineArgs* ra);
     int build_cond_graph(const sptrsv_opts& o, const double* b, double* x, double* x_out, int rhs, int layout,
-                         cudaGraphExec_t* out, int64_t* fixed_kernels);
+                         bool loop, cudaGraphExec_t* out, int64_t* fixed_kernels);
     int resident_warps(const sptrsv_opts& o) const;
     int levelset_warps(const sptrsv_opts& o) const;
     int set_supernodes(int sn, const int* snodes_host);

@@ -123,8 +123,8 @@ struct RefineArgs {
     int pairs;         // off/roff in the paired layout: every row's slots padded to an even count
     const int* jmeta;  // group-jagged layout (off holds its entries): per group lane (row << 27) | count
     const int* jbase;  // group-jagged layout: first entry of every 32-row group
-    int sweep_kernel;  // 0 lane per row over entry pairs (default), 1 warp tiles, 2 lane per row,
-                       // 3 tiles at 8 blocks/SM, 4 two rows per lane, 5 bulk-copy pipeline,
+    int sweep_kernel;  // 0 lane per row over entry pairs, copied ahead (default), 1 warp tiles, 2 lane per
+                       // row, 3 tiles at 8 blocks/SM, 4 two rows per lane,
                        // 6 SELL slices, 7/8 lane per row with 4/8-entry batches, 9 warp per
                        // 32-row group over the group-jagged layout
     int nslices;       // SELL: slices of 32 rows
@@ -177,6 +177,9 @@ int launch_check_outer(const RefineArgs& a, int max_refine, cudaGraphConditional
                        cudaGraphConditionalHandle hi);
 int launch_check_inner(const RefineArgs& a, float eps, int max_sweeps, cudaGraphConditionalHandle hi);
 int launch_jacobi_sweep(const RefineArgs& a, int src, bool last, bool stats);
+// A whole inner solve and x += d in one cooperative launch; refine_loops: whether it applies.
+bool refine_loops(const RefineArgs& a);
+int launch_jacobi_loop(const RefineArgs& a, float eps, int max_sweeps);
 int launch_axpy_pending(const RefineArgs& a, int src);
 int launch_exact_inner(const RefineArgs& a, int schedule, int rows_per_warp, int dst, int max_level,
                        const int* lptr, const int* lrows, int warps);

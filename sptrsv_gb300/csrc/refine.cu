@@ -22,8 +22,8 @@
 // Short rows: the FP64 residual uses warp tiles of 32 consecutive rows (the warp copies the
 // tile's entries into shared memory with coalesced loads, then each lane sums its own row in
 // order: deterministic; tiles with more than kTileMax entries read straight from global memory);
-// the default Jacobi sweep gives each lane a row of the paired layout (16-byte loads of two
-// entries).  Long-row matrices use the warp-per-row kernels (LPR lanes per row).
+// the default Jacobi sweep gives each lane a row of the paired layout, whose entries
+// come by bulk copies, and runs a whole inner solve as one launch.  Long-row matrices use the warp-per-row kernels (LPR lanes per row).
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -349,17 +349,18 @@ __global__ void k_check_outer(int rhs, double* rn2, const double* bn2, Ctl* ctl,
     ctl->x_zero = 0;
     if (rel <= tol) ctl->done = 1;
     ctl->inner_count = 0;
-    ctl->dmax_bits = 0u;
-    ctl->dchg_bits = 0u;
+    ctl->dmax_bits = ctl->dmax2_bits = 0u;
+    ctl->dchg_bits = ctl->dchg2_bits = 0u;
     if (stop) {
+        ctl->inner_eps = -1.f;
         cudaGraphSetConditional(h_outer, 0);
-        cudaGraphSetConditional(h_inner, 0);
+        if (h_inner) cudaGraphSetConditional(h_inner, 0);
     } else {
         ctl->steps = step + 1;
         // inexact correction: x + d has residual ~ rel * (relative error of d), so the next inner
         // solve only needs kInnerTarget * tol / rel (never tighter than its own floor, below)
         ctl->inner_eps = (float)fmin(1.0, kInnerTarget * tol / rel);
-        cudaGraphSetConditional(h_inner, 1);
+        if (h_inner) cudaGraphSetConditional(h_inner, 1);
     }
 }
 
@@ -522,64 +523,6 @@ __global__ void __launch_bounds__(256, MINB) k_jacobi_batched(int n, const int* 
             for (int j = 0; j < B; ++j) g[j] = (k0 + j < e) ? __ldg(src + p[j].x) : 0.f;
 #pragma unroll
             for (int j = 0; j < B; ++j) sum = fmaf(__int_as_float(p[j].y), g[j], sum);
-        }
-        const float d = (ri - sum) * di;
-        if (stats) {
-            dmax = fmaxf(dmax, fabsf(d));
-            dchg = fmaxf(dchg, fabsf(d - src[i]));
-        }
-        if (last) x[i] += (double)d;
-        else dst[i] = d;
-        i = inext;
-        s = sn;
-        e = en;
-    }
-    if (stats) reduce_stats(dmax, dchg, ctl, s_max);
-}
-
-// The lane-per-row sweep over the paired layout: every row's slots start on a 16-byte boundary and
-// come in pairs, so one 16-byte load brings two entries (half the load instructions, and the L1
-// wavefronts, of 8-byte entry loads).  B entries (B/2 pair loads, then B gathers, then B FMAs in
-// entry order) per batch; the next row's offsets are fetched while the current row is summed.  The
-// pad entry of an odd row adds 0 * d_i.
-template <int B, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_jacobi_pairs(int n, const int* __restrict__ roff,
-                                                           const int4* __restrict__ off2,
-                                                           const float* __restrict__ invd,
-                                                           const float* __restrict__ r,
-                                                           const float* __restrict__ src, float* __restrict__ dst,
-                                                           double* __restrict__ x, int last, int stats, Ctl* ctl) {
-    static_assert(B % 2 == 0, "entries come in pairs");
-    __shared__ unsigned s_max[2];
-    if (is_done(ctl)) return;
-    if (threadIdx.x < 2) s_max[threadIdx.x] = 0u;
-    __syncthreads();
-    float dmax = 0.f, dchg = 0.f;
-    const int stride = gridDim.x * blockDim.x;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int s = 0, e = 0;
-    if (i < n) { s = __ldg(roff + i); e = __ldg(roff + i + 1); }
-    while (i < n) {
-        const int inext = i + stride;
-        int sn = 0, en = 0;
-        if (inext < n) { sn = __ldg(roff + inext); en = __ldg(roff + inext + 1); }
-        const float ri = r[i], di = invd[i];
-        float sum = 0.f;
-        for (int k0 = s; k0 < e; k0 += B) {
-            int4 p[B / 2];
-            float g[B];
-#pragma unroll
-            for (int j = 0; j < B / 2; ++j) p[j] = (k0 + 2 * j < e) ? __ldg(off2 + (k0 >> 1) + j) : make_int4(i, 0, i, 0);
-#pragma unroll
-            for (int j = 0; j < B / 2; ++j) {
-                g[2 * j] = (k0 + 2 * j < e) ? __ldg(src + p[j].x) : 0.f;
-                g[2 * j + 1] = (k0 + 2 * j < e) ? __ldg(src + p[j].z) : 0.f;
-            }
-#pragma unroll
-            for (int j = 0; j < B / 2; ++j) {
-                sum = fmaf(__int_as_float(p[j].y), g[2 * j], sum);
-                sum = fmaf(__int_as_float(p[j].w), g[2 * j + 1], sum);
-            }
         }
         const float d = (ri - sum) * di;
         if (stats) {
@@ -836,24 +779,30 @@ int sell_fill(int n, const int* rp, const int* col, const double* val, const int
 int sell_slices(int n) { return ((n + kSellWin - 1) / kSellWin) * (kSellWin / 32); }
 
 // ---------------------------------------------------------------------------------------
-// Bulk-copy pipelined sweep.  Each warp walks its tiles (32 rows each) with a kStages-deep
-// pipeline: lane 0 issues cp.async.bulk copies of the next tiles' row offsets and interleaved
-// off-diagonals into the warp's shared-memory stages (completion counted in bytes on an
-// mbarrier), while the lanes compute on the current tile.  No registers hold in-flight data,
-// so every SM keeps tens of KB of matrix traffic in flight.  Copies start on 16-byte
-// boundaries (even int2 index, 32-row aligned offset rows) and move multiples of 16 bytes;
-// `off` and `roff` carry padding so the rounded-up ranges stay inside their allocations.
-// Tiles larger than a stage are read straight from global memory.  Every mbarrier wait is
-// bounded by the spin budget.
-constexpr int kStages = 4;
-constexpr int kTmaWarps = 4;
-constexpr int kStageEntries = 384;  // int2 entries per stage (3 KiB)
-
-struct __align__(128) TmaStage {
-    int2 off[kStageEntries];
-    int roff[36];  // 36 ints = 144 bytes: the tile's 33 row offsets, rounded up to 16 bytes
-};
-
+// The default sweep of short rows with one right-hand side, over the paired layout: every row's slots
+// start on a 16-byte boundary and come in pairs, so one 16-byte load brings two entries; the pad entry of
+// an odd row adds 0 * d_i.  A block takes tiles of R rows.  One more warp brings each tile's entries to
+// shared memory by a bulk copy, S tiles deep, while a lane per row sums the tile before: B entries (B / 2
+// pair loads, B gathers, B FMAs in entry order) at a time.  What is left to wait for is the gathers; with
+// the entries loaded by the lanes as well (L1 76 % busy) a sweep took 38 us
+// at 2M rows and 17.2M entries, 62 % of the measured copy bandwidth.
+//
+// kLoop: the whole inner solve in one cooperative launch.  A grid barrier follows each sweep and every
+// block makes the test of k_check_inner after each second one; then x += d.  Launching the sweeps and the
+// test from a WHILE node cost 4 us a sweep (9 us where the sweep itself is short).  The next sweep's
+// first tiles are copied ahead of the barrier, and a block with no more than S tiles keeps them all in
+// shared memory: up to 311k rows the entries are read once.  Three residuals and 28 sweeps: 2M rows
+// 1.31 -> 1.06 ms, 1M 0.75 -> 0.63, 400k 0.46 -> 0.36, 100k 0.33 -> 0.20, 20k 0.28 -> 0.15, 2k 0.26 -> 0.14.
+// R = 256, four blocks an SM: 128 x 8 spend the gain on a barrier of 1,216 blocks (1.53 ms at 2M rows),
+// 512 x 2, 320 x 3 and three stages are within 4 %.  One sweep a launch: R = 128, eight blocks (1.16 ms,
+// 256 x 4 1.22).
+//
+// Sweeps read 8 bytes an entry and 16 a row.  What does not fit L2 with the four vectors is read
+// evict-first, so that the vectors and the first tiles stay from sweep to sweep: 60 MB in all, half of L2
+// (lines of the other die are held twice).  2M rows: no policy 1.15 ms, everything evict-first 1.07,
+// 28 MB kept 1.05.
+//
+// Every wait is bounded, and copies in flight land before a block ends.
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -889,119 +838,230 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, Ctl* c
     }
 }
 
-__global__ void __launch_bounds__(kTmaWarps * 32) k_jacobi_tma(int n, const int* __restrict__ roff,
-                                                              const int2* __restrict__ off,
-                                                              const float* __restrict__ invd,
-                                                              const float* __restrict__ r,
-                                                              const float* __restrict__ src, float* __restrict__ dst,
-                                                              double* __restrict__ x, int last, int stats, Ctl* ctl,
-                                                              int64_t budget) {
-    extern __shared__ __align__(128) unsigned char tma_smem[];
-    TmaStage(*stages)[kStages] = reinterpret_cast<TmaStage(*)[kStages]>(tma_smem);
-    __shared__ __align__(8) uint64_t bars[kTmaWarps][kStages];
+// L2 policy of entries that no later sweep finds in L2 anyway: first to go, so that the vectors stay.
+__device__ __forceinline__ uint64_t evict_first_policy() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src, unsigned bytes, uint64_t* bar, uint64_t policy) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+                     smem_addr(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_addr(bar)), "l"(policy)
+                 : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// The same without the abort flag: what is in flight lands whatever else went wrong.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, unsigned parity, int64_t budget) {
+    const uint64_t t0 = gtimer();
+    while (!mbar_try_wait(bar, parity) && (int64_t)(gtimer() - t0) <= budget) {}
+}
+
+struct BulkArgs {
+    int n, cap, keep;  // cap: pairs a stage holds; tiles before `keep` are read with no L2 policy
+    const int* roff;
+    const int4* off2;
+    const float *invd, *r;
+    float *d0, *d1;  // the first sweep reads d0
+    double* x;
+    int last, stats;  // one sweep: x += its result; measure its change
+    float eps_floor;  // loop: as k_check_inner
+    int max_sweeps;
+    Ctl* ctl;
+    int64_t budget;
+};
+
+template <int R, int S, int MINB, bool kLoop>
+__global__ void __launch_bounds__(R + 32, MINB) k_jacobi_bulk(const BulkArgs A) {
+    constexpr int B = 8;
+    extern __shared__ __align__(128) int4 stage[];  // S x cap pairs
+    __shared__ __align__(8) uint64_t full[S], empty[S];
+    __shared__ int base[S];  // first pair of the stage's tile, -1: too large for a stage
     __shared__ unsigned s_max[2];
+    Ctl* const ctl = A.ctl;
     if (is_done(ctl)) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (threadIdx.x < 2) s_max[threadIdx.x] = 0u;
-    if (lane == 0)
-        for (int q = 0; q < kStages; ++q) mbar_init(&bars[w][q], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    __syncthreads();
-    const int ntiles = (n + 31) >> 5;
-    const int nw = gridDim.x * kTmaWarps;
-    const int first = blockIdx.x * kTmaWarps + w;
-    TmaStage* st = stages[w];
-    uint64_t* bar = bars[w];
-    // issue tile j (the j-th tile of this warp) into stage j % kStages; returns its mode:
-    // 1 staged, 2 direct (too large for a stage), 0 none (past the end)
-    // lane 0 keeps the row-offset bounds of the next tile to issue in registers, loaded one
-    // iteration before they are needed, so the issue never waits on a global load
-    int nx_e0 = 0, nx_e1 = 0;
-    auto fetch = [&](int j) {
-        const int t = first + j * nw;
-        if (t < ntiles) { nx_e0 = __ldg(roff + 32 * t); nx_e1 = __ldg(roff + 32 * t + 32); }
-    };
-    auto issue = [&](int j) -> int {
-        const int t = first + j * nw;
-        if (t >= ntiles) return 0;
-        const int e0 = nx_e0, e1 = nx_e1;
-        fetch(j + 1);
-        const int a0 = e0 & ~1, a1 = (e1 + 1) & ~1;
-        TmaStage& S = st[j % kStages];
-        uint64_t* b = &bar[j % kStages];
-        if (a1 - a0 > kStageEntries) return 2;
+    const int tid = threadIdx.x, n = A.n, cap = A.cap, grid = gridDim.x;
+    const int tiles = (n + R - 1) / R, mine = (tiles - 1 - (int)blockIdx.x) / grid + 1;  // grid <= tiles
+    const int* const roff = A.roff;
+    const int4* const off2 = A.off2;
+    const float eps = kLoop ? ctl->inner_eps : 0.f;
+    const bool producer = tid >= R;
+    if (tid == 0) {
+        for (int q = 0; q < S; ++q) {
+            mbar_init(&full[q], 1);
+            mbar_init(&empty[q], R / 32);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const unsigned bytes = (unsigned)(a1 - a0) * 8u;
-        mbar_expect_tx(b, bytes + 144u);
-        bulk_g2s(S.roff, roff + 32 * t, 144u, b);
-        if (bytes) bulk_g2s(S.off, off + a0, bytes, b);
-        return 1;
-    };
-    // per-stage mode (2 bits each: 0 none, 1 staged, 2 direct) and mbarrier phase bits
-    unsigned modes = 0u, phases = 0u, pending = 0u;
-    auto set_mode = [&](int q, int md) {
-        modes = (modes & ~(3u << (2 * q))) | ((unsigned)md << (2 * q));
-        if (md == 1) pending |= 1u << q;
-    };
-    // prologue: fill the pipeline (lane 0 issues, the mode is broadcast)
-    if (lane == 0) fetch(0);
-    for (int j = 0; j < kStages - 1; ++j) {
-        int md = 0;
-        if (lane == 0) md = issue(j);
-        set_mode(j % kStages, __shfl_sync(0xffffffffu, md, 0));
     }
-    float dmax = 0.f, dchg = 0.f;
+    if (tid < 2) s_max[tid] = 0u;
+    __syncthreads();
+    // A loop whose tiles all have a stage of their own copies them once.
+    const bool resident = kLoop && mine <= S;
+    unsigned phase = 0u;      // bit q: parity of stage q's next wait (consumers: full, producer: empty)
+    int q = 0, issued = 0;    // producer: stages in use while < S, and tiles copied ahead for the next sweep
+    int ahead = 0, copies = 0, b0 = 0, b1 = 0;
+    uint64_t policy = 0;
     bool ok = true;
-    for (int j = 0;; ++j) {
-        const int t = first + j * nw;
-        if (t >= ntiles) break;
-        {   // keep kStages - 1 tiles in flight ahead of the one being computed
-            int md = 0;
-            if (lane == 0) md = issue(j + kStages - 1);
-            set_mode((j + kStages - 1) % kStages, __shfl_sync(0xffffffffu, md, 0));
+    auto in = [&](int row) { return (unsigned)row < (unsigned)n; };
+    auto bounds = [&](int j) {
+        const long long t = blockIdx.x + (long long)(j < mine ? j : 0) * grid;
+        b0 = __ldg(roff + t * R) >> 1;
+        b1 = __ldg(roff + min((long long)n, (t + 1) * R)) >> 1;
+    };
+    auto issue = [&](int j) {  // tile j of this block; j + 1's bounds are loaded here
+        const int e0 = b0, cnt = b1 - b0;
+        bounds(j + 1);
+        if (issued == S) {
+            if (!(ok = mbar_wait(&empty[q], (phase >> q) & 1u, ctl, A.budget))) return;
+            phase ^= 1u << q;
+        } else {
+            ++issued;
         }
-        const int q = j % kStages;
-        const int r0 = t * 32, i = r0 + lane;
-        float sum = 0.f;
-        const int mq = (modes >> (2 * q)) & 3u;
-        if (mq == 1) {
-            ok = mbar_wait(&bar[q], (phases >> q) & 1u, ctl, budget);
-            phases ^= 1u << q;
-            pending &= ~(1u << q);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            const TmaStage& S = st[q];
-            const int a0 = S.roff[0] & ~1;
-            if (i < n) {
-                const int s = S.roff[lane] - a0, e = S.roff[lane + 1] - a0;
-#pragma unroll 4
-                for (int k = s; k < e; ++k) {
-                    const int2 p = S.off[k];
-                    sum = fmaf(__int_as_float(p.y), __ldg(src + p.x), sum);
+        const bool fits = cnt <= cap;
+        base[q] = fits ? e0 : -1;
+        const unsigned bytes = fits ? (unsigned)cnt * 16u : 0u;
+        mbar_expect_tx(&full[q], bytes);
+        if (bytes) {
+            if ((int)blockIdx.x + j * grid < A.keep) bulk_g2s(stage + (size_t)q * cap, off2 + e0, bytes, &full[q]);
+            else bulk_g2s_hint(stage + (size_t)q * cap, off2 + e0, bytes, &full[q], policy);
+        }
+        ++copies;
+        q = q + 1 == S ? 0 : q + 1;
+    };
+    if (tid == R) {
+        policy = evict_first_policy();
+        bounds(0);
+    }
+    int i = blockIdx.x * R + tid, s = 0, e = 0;
+    float ri = 0.f, di = 0.f;
+    if (!producer && in(i)) {
+        s = __ldg(roff + i);
+        e = __ldg(roff + i + 1);
+        ri = A.r[i];
+        di = A.invd[i];
+    }
+    int sweeps = 0;
+    const bool any = !kLoop || eps >= 0.f;  // below: the last correction is d0 itself
+    while (any) {
+        const float* const src = sweeps & 1 ? A.d1 : A.d0;
+        float* const dst = sweeps & 1 ? A.d0 : A.d1;
+        const bool stats = kLoop ? (sweeps & 1) : A.stats;
+        const bool last = !kLoop && A.last;
+        float dmax = 0.f, dchg = 0.f;
+        if (producer) {
+            if (tid == R && !(resident && sweeps)) {
+                for (int j = ahead; ok && j < mine; ++j) issue(j);
+                ahead = 0;
+                if (kLoop && !resident)
+                    for (; ok && ahead < S; ++ahead) issue(ahead);  // the next sweep's, before the barrier
+            }
+            __syncwarp();
+        } else {
+            if (resident) q = 0;
+            for (int j = 0; j < mine; ++j) {
+                // the next tile's rows; after the last, the first tile's for the next sweep
+                const int inext = j + 1 < mine ? i + grid * R : blockIdx.x * R + tid;
+                int sn = 0, en = 0;
+                float rn = 0.f, dn = 0.f;
+                if (in(inext) && (kLoop || j + 1 < mine)) {
+                    sn = __ldg(roff + inext);
+                    en = __ldg(roff + inext + 1);
+                    rn = A.r[inext];
+                    dn = A.invd[inext];
                 }
-            }
-        } else if (i < n) {
-            const int s = roff[i], e = roff[i + 1];
-            for (int k = s; k < e; ++k) {
-                const int2 p = __ldg(off + k);
-                sum = fmaf(__int_as_float(p.y), __ldg(src + p.x), sum);
+                ok = __all_sync(0xffffffffu, mbar_wait(&full[q], (phase >> q) & 1u, ctl, A.budget));
+                if (!ok) break;
+                if (!resident) phase ^= 1u << q;
+                float sum = 0.f;
+                if (in(i)) {
+                    const int e0 = base[q];
+                    auto walk = [&](auto entry) {
+                        for (int k0 = s; k0 < e; k0 += B) {
+                            int4 p[B / 2];
+                            float g[B];
+#pragma unroll
+                            for (int u = 0; u < B / 2; ++u)
+                                p[u] = (k0 + 2 * u < e) ? entry((k0 >> 1) + u) : make_int4(i, 0, i, 0);
+#pragma unroll
+                            for (int u = 0; u < B / 2; ++u) {
+                                g[2 * u] = (k0 + 2 * u < e) ? src[p[u].x] : 0.f;
+                                g[2 * u + 1] = (k0 + 2 * u < e) ? src[p[u].z] : 0.f;
+                            }
+#pragma unroll
+                            for (int u = 0; u < B / 2; ++u) {
+                                sum = fmaf(__int_as_float(p[u].y), g[2 * u], sum);
+                                sum = fmaf(__int_as_float(p[u].w), g[2 * u + 1], sum);
+                            }
+                        }
+                    };
+                    if (e0 >= 0) walk([&](int k) { return stage[q * cap + (k - e0)]; });
+                    else walk([&](int k) { return __ldg(off2 + k); });
+                }
+                if (!resident) {
+                    __syncwarp();
+                    if ((tid & 31) == 0) mbar_arrive(&empty[q]);
+                }
+                if (in(i)) {
+                    const float d = (ri - sum) * di;
+                    if (stats) {
+                        dmax = fmaxf(dmax, fabsf(d));
+                        dchg = fmaxf(dchg, fabsf(d - src[i]));
+                    }
+                    if (last) A.x[i] += (double)d;
+                    else dst[i] = d;
+                }
+                q = q + 1 == S ? 0 : q + 1;
+                i = inext;
+                s = sn;
+                e = en;
+                ri = rn;
+                di = dn;
             }
         }
-        __syncwarp();  // every lane is done with stage q before it is refilled
-        if (i < n) {
-            const float d = (r[i] - sum) * invd[i];
-            if (stats) {
-                dmax = fmaxf(dmax, fabsf(d));
-                dchg = fmaxf(dchg, fabsf(d - src[i]));
+        ++sweeps;
+        unsigned* const top = !kLoop || (sweeps >> 1) & 1 ? &ctl->dmax_bits : &ctl->dmax2_bits;  // and its neighbour
+        if (stats) {
+            for (int o = 16; o > 0; o >>= 1) {
+                dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+                dchg = fmaxf(dchg, __shfl_xor_sync(0xffffffffu, dchg, o));
             }
-            if (last) x[i] += (double)d;
-            else dst[i] = d;
+            if ((tid & 31) == 0) {
+                atomicMax(&s_max[0], __float_as_uint(dmax));
+                atomicMax(&s_max[1], __float_as_uint(dchg));
+            }
+            __syncthreads();
+            if (tid < 2) {
+                atomicMax(top + tid, s_max[tid]);
+                s_max[tid] = 0u;
+                // the other pair's maxima: every block has read them (before the first sweep's barrier)
+                if (kLoop && blockIdx.x == 0)
+                    st_relaxed((int*)(top == &ctl->dmax_bits ? &ctl->dmax2_bits : &ctl->dmax_bits) + tid, 0);
+            }
+        }
+        if (!kLoop) break;
+        if (!grid_barrier(ctl, grid, A.budget) || __syncthreads_or(!ok)) break;
+        if (stats) {
+            const float m = __int_as_float(ld_relaxed((const int*)top)), c = __int_as_float(ld_relaxed((const int*)top + 1));
+            if (!(c > fmaxf(A.eps_floor, eps) * m) || sweeps >= A.max_sweeps) break;
         }
     }
-    // drain: copies issued but not consumed (only after an aborted wait) complete before the
-    // block exits, each wait again bounded by the budget
-    for (int q = 0; q < kStages; ++q)
-        if (pending & (1u << q)) (void)mbar_wait(&bar[q], (phases >> q) & 1u, ctl, budget);
-    if (stats) reduce_stats(dmax, dchg, ctl, s_max);
+    // copies that no sweep took (ahead of one that did not come, after a wait that was given up) land
+    // before the block's memory is let go
+    if (tid == R)
+        for (int z = 0; z < S && z < copies; ++z)
+            mbar_drain(&full[z], (unsigned)((copies - z + S - 1) / S - 1) & 1u, A.budget);
+    if (!kLoop) return;
+    for (int j = 0, row = blockIdx.x * R + tid; !producer && j < mine; ++j, row += grid * R)
+        if (in(row)) A.x[row] += (double)A.d0[row];
+    if (blockIdx.x == 0 && tid == 0) {
+        ctl->inner_count = sweeps;
+        ctl->inner_total += sweeps;
+    }
 }
 
 // Same sweep, LPR lanes per row over the CSR FP32 values (long rows).
@@ -1105,8 +1165,6 @@ static int resident_grid(const void* fn, int block, int sm_count) {
     return per_sm * sm_count;
 }
 
-static size_t tma_smem_bytes() { return sizeof(TmaStage) * kStages * kTmaWarps; }
-
 int launch_pair_offsets(int n, const int* rp, int* len2, int* roff, int roff_pad, int* part, int sm_count,
                         cudaStream_t st, int64_t* launches) {
     k_pair_len<<<sm_count * 4, 256, 0, st>>>(n, rp, len2);
@@ -1153,7 +1211,6 @@ int launch_build_offdiag(int n, const int* rp, const int* col, const double* val
     *launches += 2;
     CUDA_TRY(cudaGetLastError());
     // opt in to the sweep kernel's dynamic shared memory here, outside any stream capture
-    CUDA_TRY(cudaFuncSetAttribute(k_jacobi_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem_bytes()));
     return 0;
 }
 
@@ -1224,6 +1281,65 @@ int launch_check_inner(const RefineArgs& a, float eps, int max_sweeps, cudaGraph
     return 0;
 }
 
+// The launch shape of k_jacobi_bulk.
+template <int R, int S>
+struct BulkShape {
+    int cap, tiles, keep;
+    size_t smem;
+    explicit BulkShape(const RefineArgs& a) {
+        // a stage holds the mean tile (half a row's entries and pads) and a tenth more; larger tiles are
+        // read from global memory.  At most 61 KB (14 entries a row).
+        cap = (int)(R * 0.55 * ((double)a.nnz / a.n - 0.45)) + 16;
+        smem = (size_t)cap * 16 * S;
+        tiles = (int)(((long long)a.n + R - 1) / R);
+        const double bytes = 8.0 * ((double)a.nnz - 0.5 * a.n), room = 60e6 - 16.0 * a.n;
+        keep = room >= bytes ? tiles : room <= 0.0 ? 0 : (int)(tiles * (room / bytes));
+    }
+    BulkArgs args(const RefineArgs& a) const {
+        BulkArgs A{};
+        A.n = a.n;
+        A.cap = cap;
+        A.keep = keep;
+        A.roff = a.roff;
+        A.off2 = reinterpret_cast<const int4*>(a.off);
+        A.invd = a.invd32;
+        A.r = a.r32;
+        A.x = a.x;
+        A.ctl = a.ctl;
+        A.budget = std::max<int64_t>(a.budget, kDefaultBudgetNs);  // a caller's budget is for waits on rows
+        return A;
+    }
+    int grid(const void* fn, const RefineArgs& a, int* blocks) const {
+        int per_sm = 0;
+        CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, R + 32, smem));
+        if (per_sm < 1) return SPTRSV_ERR_UNSUPPORTED;
+        *blocks = std::min(tiles, per_sm * a.sm_count);
+        return 0;
+    }
+};
+
+// Whether the inner solve runs as one launch (launch_jacobi_loop).
+bool refine_loops(const RefineArgs& a) { return use_tiles(a) && !a.jmeta && a.roff && a.pairs; }
+
+int launch_jacobi_loop(const RefineArgs& a, float eps, int max_sweeps) {
+    constexpr int R = 256, S = 2;
+    const BulkShape<R, S> shape(a);
+    BulkArgs A = shape.args(a);
+    A.d0 = a.d32[0];
+    A.d1 = a.d32[1];
+    A.eps_floor = eps;
+    A.max_sweeps = max_sweeps;
+    const void* fn = (const void*)k_jacobi_bulk<R, S, 4, true>;
+    int blocks;
+    int rc = shape.grid(fn, a, &blocks);
+    if (rc) return rc;
+    void* args[] = {(void*)&A};
+    CUDA_TRY(cudaLaunchCooperativeKernel(fn, blocks, R + 32, args, shape.smem, a.st));
+    ++*a.launches;
+    return 0;
+}
+
 int launch_jacobi_sweep(const RefineArgs& a, int src, bool last, bool stats) {
     const int grid = stream_grid(a.sm_count);
     const float* s = a.d32[src];
@@ -1235,10 +1351,17 @@ int launch_jacobi_sweep(const RefineArgs& a, int src, bool last, bool stats) {
         k_jacobi_jds<6, 6><<<grid_j6, 256, 0, a.st>>>(a.n, (a.n + 31) / 32, a.jmeta, a.jbase, a.off, a.invd32, a.r32, s,
                                                      d, a.x, last, st_flag, a.ctl);
     } else if (use_tiles(a) && a.roff && a.pairs) {
-        static int grid_p8 = 0;
-        if (!grid_p8) grid_p8 = resident_grid((const void*)k_jacobi_pairs<8, 6>, 256, a.sm_count);
-        k_jacobi_pairs<8, 6><<<grid_p8, 256, 0, a.st>>>(a.n, a.roff, reinterpret_cast<const int4*>(a.off), a.invd32,
-                                                       a.r32, s, d, a.x, last, st_flag, a.ctl);
+        constexpr int R = 128, S = 2;
+        const BulkShape<R, S> shape(a);
+        BulkArgs A = shape.args(a);
+        A.d0 = a.d32[src];
+        A.d1 = d;
+        A.last = last;
+        A.stats = st_flag;
+        int blocks;
+        int rc = shape.grid((const void*)k_jacobi_bulk<R, S, 8, false>, a, &blocks);
+        if (rc) return rc;
+        k_jacobi_bulk<R, S, 8, false><<<blocks, R + 32, shape.smem, a.st>>>(A);
     } else if (use_tiles(a) && a.roff && (a.sweep_kernel == 7)) {
         static int grid_b4 = 0;
         if (!grid_b4) grid_b4 = resident_grid((const void*)k_jacobi_batched<4, 8>, 256, a.sm_count);
@@ -1268,17 +1391,6 @@ int launch_jacobi_sweep(const RefineArgs& a, int src, bool last, bool stats) {
         if (!grid_t8) grid_t8 = resident_grid((const void*)k_jacobi_tile<384, 8>, kJacWarps * 32, a.sm_count);
         k_jacobi_tile<384, 8><<<grid_t8, kJacWarps * 32, 0, a.st>>>(a.n, a.rp, a.off, a.invd32, a.r32, s, d, a.x,
                                                                    last, st_flag, a.ctl);
-    } else if (use_tiles(a) && a.roff && a.sweep_kernel == 5) {
-        static int grid_tma = 0;
-        if (!grid_tma) {
-            int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_jacobi_tma, kTmaWarps * 32,
-                                                              tma_smem_bytes()) != cudaSuccess || per_sm < 1)
-                per_sm = 1;
-            grid_tma = per_sm * a.sm_count;
-        }
-        k_jacobi_tma<<<grid_tma, kTmaWarps * 32, tma_smem_bytes(), a.st>>>(a.n, a.roff, a.off, a.invd32, a.r32, s, d,
-                                                                         a.x, last, st_flag, a.ctl, a.budget);
     } else if (use_tiles(a)) {
         static int grid_jt = 0;
         if (!grid_jt) grid_jt = resident_grid((const void*)k_jacobi_tile<kTileMax, 1>, kJacWarps * 32, a.sm_count);
