@@ -363,10 +363,11 @@ int Handle::prepare(const sptrsv_opts& o, int rhs, int layout) {
         if ((rc = grow(xw, sizeof(double) * nr))) return rc;
     }
     if (o.precision == SPTRSV_PREC_MIXED) {
-        if (o.inner == SPTRSV_SCHED_JACOBI && rhs == 1)
+        const bool few = rhs == 1 || (sweep_kernel == 0 && rhs <= kBulkCols);
+        if (o.inner == SPTRSV_SCHED_JACOBI && (rhs == 1 || (few && mean_len <= kShortRowLen)))
             if ((rc = ensure_offdiag())) return rc;
-        if (!have_val32 && !(o.inner == SPTRSV_SCHED_JACOBI && rhs == 1 && mean_len <= kShortRowLen)) {
-            // the FP32 values, where the inner solve reads them (the Jacobi sweeps of one right-hand side
+        if (!have_val32 && !(o.inner == SPTRSV_SCHED_JACOBI && few && mean_len <= kShortRowLen)) {
+            // the FP32 values, where the inner solve reads them (the Jacobi sweeps of few right-hand sides
             // on short rows have their own layout)
             if ((rc = val32.ensure(sizeof(float) * (size_t)nnz))) return rc;
             k_to_f32<<<sm_count * 4, 256, 0, st>>>((size_t)nnz, val, val32.as<float>());
@@ -695,8 +696,9 @@ int Handle::refine_args(const sptrsv_opts& o, const double* b, double* x, int rh
     r.invd = invd.as<double>();
     r.invd32 = invd32.as<float>();
     const bool sl = have_offdiag && rhs == 1 && sweep_kernel == 6;
-    r.off = (have_offdiag && rhs == 1 && !sl) ? offdiag.as<int2>() : nullptr;
-    r.roff = (have_offdiag && rhs == 1 && !sl) ? roff.as<int>() : nullptr;
+    const bool laid = have_offdiag && !sl && (rhs == 1 || (sweep_kernel == 0 && off_pairs && rhs <= kBulkCols));
+    r.off = laid ? offdiag.as<int2>() : nullptr;
+    r.roff = laid ? roff.as<int>() : nullptr;
     r.pairs = off_pairs ? 1 : 0;
     r.jmeta = (have_offdiag && rhs == 1 && off_jds) ? jmeta.as<int>() : nullptr;
     r.jbase = (have_offdiag && rhs == 1 && off_jds) ? jbase.as<int>() : nullptr;

@@ -108,8 +108,12 @@ struct SnArgs {
 };
 
 // refine.cu
-// Mean entries per row up to which the sweeps of one right-hand side use the off-diagonals' own layouts.
+// Mean entries per row up to which the sweeps of few right-hand sides use the off-diagonals' own layouts.
 constexpr double kShortRowLen = 14.0;
+// Right-hand sides up to which they do: a lane sums a row's columns four at a time (mixed solve, 28 sweeps:
+// 600k rows x 3 5.58 -> 1.09 ms, 250k x 8 2.59 -> 1.09, 100k x 16 1.26 -> 1.17); with more, the kernels
+// whose lanes take the columns coalesce (60k x 32 0.95 ms, 2.01 with a lane a row).
+constexpr int kBulkCols = 12;
 struct RefineArgs {
     int n, nnz, rhs;
     const int* rp;
@@ -118,7 +122,7 @@ struct RefineArgs {
     const float* val32;
     const double* invd;
     const float* invd32;
-    const int2* off;   // interleaved (column, FP32 value) off-diagonals, or nullptr
+    const int2* off;   // interleaved (column, FP32 value) off-diagonals (few right-hand sides), or nullptr
     const int* roff;   // first off-diagonal slot of every row (rp[i] - i), padded, or nullptr
     int pairs;         // off/roff in the paired layout: every row's slots padded to an even count
     const int* jmeta;  // group-jagged layout (off holds its entries): per group lane (row << 27) | count

@@ -239,6 +239,78 @@ __global__ void __launch_bounds__(kResWarps * 32) k_residual_tile(int n, const i
     if (threadIdx.x == 0) atomicAdd(rn2, s_acc);
 }
 
+// r = b - U x for several right-hand sides, short rows: as k_residual_tile, four columns of a row at a time.
+__global__ void __launch_bounds__(kResWarps * 32) k_residual_tile_m(int n, int rhs, const int* __restrict__ rp,
+                                                                    const int* __restrict__ col,
+                                                                    const double* __restrict__ val,
+                                                                    const float* __restrict__ invd,
+                                                                    const double* __restrict__ b,
+                                                                    const double* __restrict__ x,
+                                                                    float* __restrict__ r32, float* __restrict__ d0,
+                                                                    int seed, double* __restrict__ rn2, const Ctl* ctl) {
+    constexpr int NC = 4;
+    __shared__ int s_col[kResWarps][kTileMax];
+    __shared__ double s_val[kResWarps][kTileMax];
+    extern __shared__ double s_accm[];
+    if (is_done(ctl)) return;
+    const bool zero = *(volatile const int*)&ctl->x_zero;  // r = b, the matrix is not read
+    for (int c = threadIdx.x; c < rhs; c += blockDim.x) s_accm[c] = 0.0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (long long t = blockIdx.x * kResWarps + w; t * 32 < n; t += gridDim.x * kResWarps) {
+        const int r0 = (int)(t * 32), rows = min(32, n - r0), i = r0 + min(lane, rows - 1);
+        const int s = rp[i], e = rp[i + 1];
+        const int E0 = __shfl_sync(0xffffffffu, s, 0), E1 = __shfl_sync(0xffffffffu, e, rows - 1);
+        const bool staged = !zero && E1 - E0 <= kTileMax;
+        if (staged)
+            for (int q = lane; q < E1 - E0; q += 32) {
+                s_col[w][q] = __ldg(col + E0 + q);
+                s_val[w][q] = __ldg(val + E0 + q);
+            }
+        __syncwarp();
+        const float di = invd[i];
+        for (int c0 = 0; c0 < rhs; c0 += NC) {
+            double sum[NC], sq[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) sum[c] = sq[c] = 0.0;
+            auto walk = [&](auto entry) {
+#pragma unroll 4
+                for (int k = s - E0; k < e - E0; ++k) {
+                    double v;
+                    const double* xj = x + (size_t)entry(k, v) * rhs + c0;
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        if (c0 + c < rhs) sum[c] = fma(v, xj[c], sum[c]);
+                }
+            };
+            if (lane < rows) {
+                if (zero) {
+                } else if (staged) walk([&](int k, double& v) { v = s_val[w][k]; return s_col[w][k]; });
+                else walk([&](int k, double& v) { v = __ldg(val + E0 + k); return __ldg(col + E0 + k); });
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (c0 + c < rhs) {
+                        const size_t p = (size_t)i * rhs + c0 + c;
+                        const double r = b[p] - sum[c];
+                        const float rf = (float)r;
+                        r32[p] = rf;
+                        seed_out(seed, d0, p, rf, di);
+                        sq[c] = r * r;
+                    }
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                if (c0 + c >= rhs) break;
+                const double v = warp_sum(sq[c]);
+                if (lane == 0) atomicAdd(&s_accm[c0 + c], v);
+            }
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < rhs; c += blockDim.x) atomicAdd(rn2 + c, s_accm[c]);
+}
+
 // r = b - U x (rhs == 1), LPR lanes per row (long rows).
 template <int LPR>
 __global__ void __launch_bounds__(256) k_residual_v(int n, const int* __restrict__ rp, const int* __restrict__ col,
@@ -779,7 +851,7 @@ int sell_fill(int n, const int* rp, const int* col, const double* val, const int
 int sell_slices(int n) { return ((n + kSellWin - 1) / kSellWin) * (kSellWin / 32); }
 
 // ---------------------------------------------------------------------------------------
-// The default sweep of short rows with one right-hand side, over the paired layout: every row's slots
+// The default sweep of short rows with few right-hand sides, over the paired layout: every row's slots
 // start on a 16-byte boundary and come in pairs, so one 16-byte load brings two entries; the pad entry of
 // an odd row adds 0 * d_i.  A block takes tiles of R rows.  One more warp brings each tile's entries to
 // shared memory by a bulk copy, S tiles deep, while a lane per row sums the tile before: B entries (B / 2
@@ -801,6 +873,9 @@ int sell_slices(int n) { return ((n + kSellWin - 1) / kSellWin) * (kSellWin / 32
 // evict-first, so that the vectors and the first tiles stay from sweep to sweep: 60 MB in all, half of L2
 // (lines of the other die are held twice).  2M rows: no policy 1.15 ms, everything evict-first 1.07,
 // 28 MB kept 1.05.
+//
+// NC = 4: several right-hand sides, a lane on four columns of its row at a time, over the same copy of
+// the entries (kBulkCols has the times).
 //
 // Every wait is bounded, and copies in flight land before a block ends.
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
@@ -862,7 +937,7 @@ __device__ __forceinline__ void mbar_drain(uint64_t* bar, unsigned parity, int64
 }
 
 struct BulkArgs {
-    int n, cap, keep;  // cap: pairs a stage holds; tiles before `keep` are read with no L2 policy
+    int n, rhs, cap, keep;  // cap: pairs a stage holds; tiles before `keep` are read with no L2 policy
     const int* roff;
     const int4* off2;
     const float *invd, *r;
@@ -875,9 +950,10 @@ struct BulkArgs {
     int64_t budget;
 };
 
-template <int R, int S, int MINB, bool kLoop>
+template <int R, int S, int MINB, bool kLoop, int NC>
 __global__ void __launch_bounds__(R + 32, MINB) k_jacobi_bulk(const BulkArgs A) {
-    constexpr int B = 8;
+    constexpr int B = NC == 1 ? 8 : 4;
+    const int rhs = NC == 1 ? 1 : A.rhs;
     extern __shared__ __align__(128) int4 stage[];  // S x cap pairs
     __shared__ __align__(8) uint64_t full[S], empty[S];
     __shared__ int base[S];  // first pair of the stage's tile, -1: too large for a stage
@@ -942,7 +1018,7 @@ __global__ void __launch_bounds__(R + 32, MINB) k_jacobi_bulk(const BulkArgs A) 
     if (!producer && in(i)) {
         s = __ldg(roff + i);
         e = __ldg(roff + i + 1);
-        ri = A.r[i];
+        if (NC == 1) ri = A.r[i];
         di = A.invd[i];
     }
     int sweeps = 0;
@@ -971,49 +1047,119 @@ __global__ void __launch_bounds__(R + 32, MINB) k_jacobi_bulk(const BulkArgs A) 
                 if (in(inext) && (kLoop || j + 1 < mine)) {
                     sn = __ldg(roff + inext);
                     en = __ldg(roff + inext + 1);
-                    rn = A.r[inext];
+                    if (NC == 1) rn = A.r[inext];
                     dn = A.invd[inext];
                 }
                 ok = __all_sync(0xffffffffu, mbar_wait(&full[q], (phase >> q) & 1u, ctl, A.budget));
                 if (!ok) break;
                 if (!resident) phase ^= 1u << q;
-                float sum = 0.f;
-                if (in(i)) {
-                    const int e0 = base[q];
-                    auto walk = [&](auto entry) {
-                        for (int k0 = s; k0 < e; k0 += B) {
-                            int4 p[B / 2];
-                            float g[B];
+                if constexpr (NC == 1) {
+                    float sum = 0.f;
+                    if (in(i)) {
+                        const int e0 = base[q];
+                        auto walk = [&](auto entry) {
+                            for (int k0 = s; k0 < e; k0 += B) {
+                                int4 p[B / 2];
+                                float g[B];
 #pragma unroll
-                            for (int u = 0; u < B / 2; ++u)
-                                p[u] = (k0 + 2 * u < e) ? entry((k0 >> 1) + u) : make_int4(i, 0, i, 0);
+                                for (int u = 0; u < B / 2; ++u)
+                                    p[u] = (k0 + 2 * u < e) ? entry((k0 >> 1) + u) : make_int4(i, 0, i, 0);
 #pragma unroll
-                            for (int u = 0; u < B / 2; ++u) {
-                                g[2 * u] = (k0 + 2 * u < e) ? src[p[u].x] : 0.f;
-                                g[2 * u + 1] = (k0 + 2 * u < e) ? src[p[u].z] : 0.f;
+                                for (int u = 0; u < B / 2; ++u) {
+                                    g[2 * u] = (k0 + 2 * u < e) ? src[p[u].x] : 0.f;
+                                    g[2 * u + 1] = (k0 + 2 * u < e) ? src[p[u].z] : 0.f;
+                                }
+#pragma unroll
+                                for (int u = 0; u < B / 2; ++u) {
+                                    sum = fmaf(__int_as_float(p[u].y), g[2 * u], sum);
+                                    sum = fmaf(__int_as_float(p[u].w), g[2 * u + 1], sum);
+                                }
                             }
-#pragma unroll
-                            for (int u = 0; u < B / 2; ++u) {
-                                sum = fmaf(__int_as_float(p[u].y), g[2 * u], sum);
-                                sum = fmaf(__int_as_float(p[u].w), g[2 * u + 1], sum);
-                            }
-                        }
-                    };
-                    if (e0 >= 0) walk([&](int k) { return stage[q * cap + (k - e0)]; });
-                    else walk([&](int k) { return __ldg(off2 + k); });
-                }
-                if (!resident) {
-                    __syncwarp();
-                    if ((tid & 31) == 0) mbar_arrive(&empty[q]);
-                }
-                if (in(i)) {
-                    const float d = (ri - sum) * di;
-                    if (stats) {
-                        dmax = fmaxf(dmax, fabsf(d));
-                        dchg = fmaxf(dchg, fabsf(d - src[i]));
+                        };
+                        if (e0 >= 0) walk([&](int k) { return stage[q * cap + (k - e0)]; });
+                        else walk([&](int k) { return __ldg(off2 + k); });
                     }
-                    if (last) A.x[i] += (double)d;
-                    else dst[i] = d;
+                    if (!resident) {
+                        __syncwarp();
+                        if ((tid & 31) == 0) mbar_arrive(&empty[q]);
+                    }
+                    if (in(i)) {
+                        const float d = (ri - sum) * di;
+                        if (stats) {
+                            dmax = fmaxf(dmax, fabsf(d));
+                            dchg = fmaxf(dchg, fabsf(d - src[i]));
+                        }
+                        if (last) A.x[i] += (double)d;
+                        else dst[i] = d;
+                    }
+                } else {
+                    const int e0 = base[q];
+                    for (int c0 = 0; c0 < rhs; c0 += NC) {
+                        const size_t row = (size_t)i * rhs + c0;
+                        float rc[NC], sum[NC];
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            rc[c] = in(i) && c0 + c < rhs ? A.r[row + c] : 0.f;
+                            sum[c] = 0.f;
+                        }
+                        auto walk = [&](auto entry, auto gather) {
+                            for (int k0 = s; k0 < e; k0 += B) {
+                                int4 p[B / 2];
+                                float g[B][NC];
+#pragma unroll
+                                for (int u = 0; u < B / 2; ++u)
+                                    p[u] = (k0 + 2 * u < e) ? entry((k0 >> 1) + u) : make_int4(i, 0, i, 0);
+#pragma unroll
+                                for (int u = 0; u < B / 2; ++u) {
+                                    const bool here = k0 + 2 * u < e;
+                                    gather(here, src + (size_t)p[u].x * rhs + c0, g[2 * u]);
+                                    gather(here, src + (size_t)p[u].z * rhs + c0, g[2 * u + 1]);
+                                }
+#pragma unroll
+                                for (int u = 0; u < B / 2; ++u)
+#pragma unroll
+                                    for (int c = 0; c < NC; ++c) {
+                                        sum[c] = fmaf(__int_as_float(p[u].y), g[2 * u][c], sum[c]);
+                                        sum[c] = fmaf(__int_as_float(p[u].w), g[2 * u + 1][c], sum[c]);
+                                    }
+                            }
+                        };
+                        auto staged = [&](int k) { return stage[q * cap + (k - e0)]; };
+                        auto direct = [&](int k) { return __ldg(off2 + k); };
+                        auto each = [&](bool here, const float* v, float* g) {
+#pragma unroll
+                            for (int c = 0; c < NC; ++c) g[c] = here && c0 + c < rhs ? v[c] : 0.f;
+                        };
+                        auto four = [&](bool here, const float* v, float* g) {
+                            const float4 w = here ? *reinterpret_cast<const float4*>(v) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            g[0] = w.x;
+                            g[1] = w.y;
+                            g[2] = w.z;
+                            g[3] = w.w;
+                        };
+                        if (rhs % 4 == 0) {
+                            if (e0 >= 0) walk(staged, four);
+                            else walk(direct, four);
+                        } else {
+                            if (e0 >= 0) walk(staged, each);
+                            else walk(direct, each);
+                        }
+                        if (!resident && c0 + NC >= rhs) {  // the stage is free
+                            __syncwarp();
+                            if ((tid & 31) == 0) mbar_arrive(&empty[q]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < NC; ++c)
+                            if (in(i) && c0 + c < rhs) {
+                                const float d = (rc[c] - sum[c]) * di;
+                                if (stats) {
+                                    dmax = fmaxf(dmax, fabsf(d));
+                                    dchg = fmaxf(dchg, fabsf(d - src[row + c]));
+                                }
+                                if (last) A.x[row + c] += (double)d;
+                                else dst[row + c] = d;
+                            }
+                    }
                 }
                 q = q + 1 == S ? 0 : q + 1;
                 i = inext;
@@ -1056,8 +1202,23 @@ __global__ void __launch_bounds__(R + 32, MINB) k_jacobi_bulk(const BulkArgs A) 
         for (int z = 0; z < S && z < copies; ++z)
             mbar_drain(&full[z], (unsigned)((copies - z + S - 1) / S - 1) & 1u, A.budget);
     if (!kLoop) return;
-    for (int j = 0, row = blockIdx.x * R + tid; !producer && j < mine; ++j, row += grid * R)
-        if (in(row)) A.x[row] += (double)A.d0[row];
+    if (!producer) {  // x += d, four loads of each in flight (one: 90 us of the 2M-row solve)
+        constexpr int U = 4;
+        const size_t total = (size_t)n * rhs, step = (size_t)grid * R;
+        for (size_t p = blockIdx.x * (size_t)R + tid; p < total; p += U * step) {
+            double xv[U];
+            float dv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (p + u * step < total) {
+                    xv[u] = A.x[p + u * step];
+                    dv[u] = A.d0[p + u * step];
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (p + u * step < total) A.x[p + u * step] = xv[u] + (double)dv[u];
+        }
+    }
     if (blockIdx.x == 0 && tid == 0) {
         ctl->inner_count = sweeps;
         ctl->inner_total += sweeps;
@@ -1152,7 +1313,7 @@ static int lpr_for(int n, int nnz) {
     return 32;
 }
 // warp tiles pay off while a 32-row tile usually fits the stage
-static bool short_rows(const RefineArgs& a) { return a.rhs == 1 && (double)a.nnz / a.n <= kShortRowLen; }
+static bool short_rows(const RefineArgs& a) { return (double)a.nnz / a.n <= kShortRowLen; }
 static bool use_tiles(const RefineArgs& a) { return short_rows(a) && a.off; }
 
 static int stream_grid(int sm_count) { return sm_count * 8; }
@@ -1238,11 +1399,17 @@ int launch_refine_init(const RefineArgs& a, bool mark_zero) {
 int launch_residual(const RefineArgs& a, bool jacobi_seed, int final_check) {
     const int seed = final_check ? 0 : (jacobi_seed ? 1 : 2);
     const int grid = stream_grid(a.sm_count);
-    if (short_rows(a)) {
+    if (short_rows(a) && a.rhs == 1) {
         static int grid_rt = 0;
         if (!grid_rt) grid_rt = resident_grid((const void*)k_residual_tile, kResWarps * 32, a.sm_count);
         k_residual_tile<<<grid_rt, kResWarps * 32, 0, a.st>>>(a.n, a.rp, a.col, a.val, a.invd32, a.b, a.x,
                                                                       a.x_out, a.r32, a.d32[0], seed, a.rn2, a.ctl);
+    } else if (short_rows(a) && a.off) {
+        const size_t smem = sizeof(double) * a.rhs;
+        int per_sm = 0;
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_residual_tile_m, kResWarps * 32, smem));
+        k_residual_tile_m<<<std::max(1, per_sm) * a.sm_count, kResWarps * 32, smem, a.st>>>(
+            a.n, a.rhs, a.rp, a.col, a.val, a.invd32, a.b, a.x, a.r32, a.d32[0], seed, a.rn2, a.ctl);
     } else if (a.rhs == 1) {
         switch (lpr_for(a.n, a.nnz)) {
             case 4: k_residual_v<4><<<grid, 256, 0, a.st>>>(a.n, a.rp, a.col, a.val, a.invd32, a.b, a.x, a.x_out, a.r32, a.d32[0], seed, a.rn2, a.ctl); break;
@@ -1292,12 +1459,13 @@ struct BulkShape {
         cap = (int)(R * 0.55 * ((double)a.nnz / a.n - 0.45)) + 16;
         smem = (size_t)cap * 16 * S;
         tiles = (int)(((long long)a.n + R - 1) / R);
-        const double bytes = 8.0 * ((double)a.nnz - 0.5 * a.n), room = 60e6 - 16.0 * a.n;
+        const double bytes = 8.0 * ((double)a.nnz - 0.5 * a.n), room = 60e6 - (4.0 + 12.0 * a.rhs) * a.n;
         keep = room >= bytes ? tiles : room <= 0.0 ? 0 : (int)(tiles * (room / bytes));
     }
     BulkArgs args(const RefineArgs& a) const {
         BulkArgs A{};
         A.n = a.n;
+        A.rhs = a.rhs;
         A.cap = cap;
         A.keep = keep;
         A.roff = a.roff;
@@ -1330,7 +1498,7 @@ int launch_jacobi_loop(const RefineArgs& a, float eps, int max_sweeps) {
     A.d1 = a.d32[1];
     A.eps_floor = eps;
     A.max_sweeps = max_sweeps;
-    const void* fn = (const void*)k_jacobi_bulk<R, S, 4, true>;
+    const void* fn = a.rhs == 1 ? (const void*)k_jacobi_bulk<R, S, 4, true, 1> : (const void*)k_jacobi_bulk<R, S, 3, true, 4>;
     int blocks;
     int rc = shape.grid(fn, a, &blocks);
     if (rc) return rc;
@@ -1345,7 +1513,7 @@ int launch_jacobi_sweep(const RefineArgs& a, int src, bool last, bool stats) {
     const float* s = a.d32[src];
     float* d = a.d32[src ^ 1];
     const int st_flag = stats ? 1 : 0;
-    if (use_tiles(a) && a.jmeta) {
+    if (use_tiles(a) && a.jmeta) {  // (the layouts other than the paired one: one right-hand side)
         static int grid_j6 = 0;
         if (!grid_j6) grid_j6 = resident_grid((const void*)k_jacobi_jds<6, 6>, 256, a.sm_count);
         k_jacobi_jds<6, 6><<<grid_j6, 256, 0, a.st>>>(a.n, (a.n + 31) / 32, a.jmeta, a.jbase, a.off, a.invd32, a.r32, s,
@@ -1358,10 +1526,11 @@ int launch_jacobi_sweep(const RefineArgs& a, int src, bool last, bool stats) {
         A.d1 = d;
         A.last = last;
         A.stats = st_flag;
+        void (*fn)(BulkArgs) = a.rhs == 1 ? k_jacobi_bulk<R, S, 8, false, 1> : k_jacobi_bulk<R, S, 6, false, 4>;
         int blocks;
-        int rc = shape.grid((const void*)k_jacobi_bulk<R, S, 8, false>, a, &blocks);
+        int rc = shape.grid((const void*)fn, a, &blocks);
         if (rc) return rc;
-        k_jacobi_bulk<R, S, 8, false><<<blocks, R + 32, shape.smem, a.st>>>(A);
+        fn<<<blocks, R + 32, shape.smem, a.st>>>(A);
     } else if (use_tiles(a) && a.roff && (a.sweep_kernel == 7)) {
         static int grid_b4 = 0;
         if (!grid_b4) grid_b4 = resident_grid((const void*)k_jacobi_batched<4, 8>, 256, a.sm_count);

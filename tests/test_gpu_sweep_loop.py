@@ -36,20 +36,35 @@ MATRICES = (
     + [("clustered", (20_000, 0, 400)), ("clustered", (20_000, 19_600, 400)), ("clustered", (300_000, 1000, 100))])
 
 
-@pytest.mark.parametrize("kind,args", MATRICES, ids=lambda v: v if isinstance(v, str) else "-".join(map(str, v)))
-def test_loop_equals_single_sweeps(orc, monkeypatch, kind, args):
-    rp, col, val = _random(*args) if kind == "random" else _clustered(*args)
+def _equal(orc, monkeypatch, rp, col, val, rhs, layout):
     n = len(rp) - 1
-    b = gen.uniform(n + 3, n)
+    b = gen.uniform(n + 3, n * rhs)
     out = {}
-    for layout in ("", "batch8"):
-        monkeypatch.setenv("SPTRSV_SWEEP_KERNEL", layout)
+    for kernel in ("", "batch8"):
+        monkeypatch.setenv("SPTRSV_SWEEP_KERNEL", kernel)
         with sp.Solver(0) as s:
             s.analyse(rp, col, val)
-            x = [s.solve(b, precision="mixed", schedule="jacobi", max_refine=20) for _ in range(2)]
+            x = [s.solve(b, rhs=rhs, precision="mixed", schedule="jacobi", max_refine=20, layout=layout) for _ in range(2)]
             assert np.array_equal(x[0], x[1])
             assert s.last_refine()[1] <= 1e-13
-            out[layout] = x[0], s.last_sweeps()
+            out[kernel] = x[0], s.last_sweeps()
     assert out[""][1] == out["batch8"][1]
     assert np.array_equal(out[""][0], out["batch8"][0])
-    assert orc.rel_residual(rp.astype(np.uint64), col, val, out[""][0], b, 1) <= 2e-13
+    if layout == sp.COL_MAJOR:
+        assert orc.rel_residual(rp.astype(np.uint64), col, val, out[""][0], b, rhs) <= 2e-13
+
+
+@pytest.mark.parametrize("kind,args", MATRICES, ids=lambda v: v if isinstance(v, str) else "-".join(map(str, v)))
+def test_loop_equals_single_sweeps(orc, monkeypatch, kind, args):
+    _equal(orc, monkeypatch, *(_random(*args) if kind == "random" else _clustered(*args)), 1, sp.COL_MAJOR)
+
+
+@pytest.mark.parametrize("rhs", [2, 3, 4, 5, 8, 12, 13])
+@pytest.mark.parametrize("n", [1, 257, 20_001, 320_000])
+def test_several_right_hand_sides(orc, monkeypatch, n, rhs):
+    """Four columns a lane, up to the count where the kernels with lanes along the columns take over."""
+    _equal(orc, monkeypatch, *_random(n, 8.0, 0.9, 64), rhs, sp.ROW_MAJOR if rhs % 2 else sp.COL_MAJOR)
+
+
+def test_several_right_hand_sides_over_large_tiles(orc, monkeypatch):
+    _equal(orc, monkeypatch, *_clustered(20_000, 700, 400), 6, sp.COL_MAJOR)
