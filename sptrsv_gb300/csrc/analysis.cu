@@ -1,12 +1,13 @@
 // analysis.cu -- matrix checks and the dependency analysis of U, all on the device.
 //
-//  * validate: row pointer monotone and starting at 0, diagonal first in every row, every
+//  * checks: row pointer monotone and starting at 0, diagonal first in every row, every
 //    other column in (i, n), finite non-zero pivot.  Also writes in_degree (row length,
 //    diagonal included -- the value kernel_full.cl:40-52 accumulates over the CSC), the
-//    reciprocal diagonal in FP64 and FP32, and the FP32 copy of the values.
+//    reciprocal diagonal in FP64 and FP32, and the matrix's statistics.
 //  * levels (core.cpp:244-270): level[i] = 1 for a diagonal-only row, else
-//    1 + max(1, max_j level[j]); computed by a sync-free pull over the same dependency DAG
-//    as the solve, with 0 as the "pending" value.  Bit-exact with the reference.
+//    1 + max(1, max_j level[j]); computed by the window kernel over chunks of rows (window.cu) or by
+//    a sync-free pull over the same dependency DAG as the solve, with 0 as the "pending" value.
+//    Bit-exact with the reference.
 //  * level buckets (core.cpp:282-288): rows grouped by level, ascending within a level --
 //    by rank within narrow levels, else a stable LSD radix sort of the level keys.
 //  * level tasks (core.cpp:289-332): the reference's greedy nnz-balanced split of each

@@ -248,7 +248,7 @@ int Handle::build_csc() {
     return 0;
 }
 
-// FP64 AUTO with one RHS: the one-CTA window kernel up to ~90 entries per row, the block kernel on
+// The exact kernel of FP64 AUTO with one RHS: the one-CTA window kernel up to ~90 entries per row, the block kernel on
 // longer rows, whose many entries per lane the window kernel walks one a round.  Measured on GB300
 // (kernel times, same GPU): random factors of 200k rows with 8.6 / 27 / 54 / 80 / 106 entries per
 // row 11.8 / 28.4 / 54.3 / 96.4 / 123.6 ms against 32.0 / 87.5 / 99.2 / 104.3 / 106.8 ms for the

@@ -17,9 +17,8 @@
 //     FP32 sync-free pull), x += d in FP64 and the FP64 residual r = b - U x, until every
 //     system's ||r||_F / ||b||_F <= tol.  Converged systems drop out of the later steps.
 //     Systems scheduled BS_PLAIN are solved exactly in FP64 first, by the same persistent pull;
-//     systems scheduled BS_PANEL64 exactly in FP64 on their dense panels, each panel's product
-//     split into 64-column blocks taken by different CTAs (the FP64 work spreads over the GPU,
-//     only the block of the nearest solved rows lies on the dependency chain).
+//     systems scheduled BS_PANEL64 exactly in FP64 on their dense panels, a warp per four rows of a
+//     panel, queued by dependency step across the systems (panel_rows.cu).
 //
 // Every wait is a bounded pending-sentinel poll (common.cuh); per-system reductions are flushed
 // once per run of rows of one system, so no address sees one atomic per row.
@@ -44,7 +43,7 @@ constexpr int kBKc = 64;        // K rows staged per chunk (a multiple of 16: ch
 constexpr int kBNc = 32;        // right-hand-side columns per pass
 constexpr int kBRowChunk = 32;  // rows per warp task in the row kernels
 constexpr int kBatchKinds = 14;  // kernel kinds of the profiled replay
-constexpr int kP64CtasPerSm = 4; // FP64 panel CTAs per SM beside the refinement (measured: 2: 190, 3: 137, 4: 135, 5: 146 ms)
+constexpr int kP64CtasPerSm = 4; // panel CTAs per SM beside the refinement (column blocks, 512-system mix: 2: 190, 3: 137, 4: 135, 5: 146 ms)
 
 
 

@@ -1,5 +1,5 @@
 // batch.cuh -- records shared by the batched path and the single-system supernodal path: system
-// descriptors, dense panel chunks, and the exact FP64 panel kernel that both use.
+// descriptors, dense panel chunks, and the exact panel kernels that both use.
 #pragma once
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -70,12 +70,11 @@ __host__ __device__ __forceinline__ void p64_block(int w, int K, int blk, int& k
     }
 }
 
-// Exact FP64 panel products over a ticketed queue of (panel, column block, RHS group) items
-// (panels64.cu).  Batched (sys != nullptr): b and x are the arenas the systems' xb0 offsets index,
+// Double-FP32 panel products over a ticketed queue of (panel, column block, RHS group) items, for panels
+// that carry double-FP32 copies of G (panels64.cu).  Batched (sys != nullptr): b and x are the arenas the systems' xb0 offsets index,
 // items carry their group (block | group << 16), poff counts doubles and cbase counters.  One
 // system (sys == nullptr, rhs columns, row-major n x rhs): every item runs for each of the
 // p64_groups(rhs) groups, poff counts per column and cbase per group.  ncnt counters are cleared.
-// Panels that carry double-FP32 copies of G (ghl) are multiplied in double-FP32.
 int launch_panels64(const BSys* sys, int rhs, const double* b, double* x, Ctl* ctl, unsigned* ticket, int64_t budget,
                     const int2* items, unsigned nitems, const BChunk* panels, double* part, int* cnt, int ncnt,
                     int ctas_per_sm, int sm_count, cudaStream_t st, int64_t* launches);

@@ -113,8 +113,9 @@ struct Handle {
     // supernode partition and its dense panels (supernodal.cu)
     DevBuf sn_start, sn_m, sn_roff, sn_rect, sn_goff, sn_ld, sn_tasks, sn_outbase, sn_items, sn_G, sn_Ghi, sn_Glo;
     int sn_count = 0, sn_nitems = 0;
-    // the FP64 solve's 64-row panels split into column blocks (panels64.cu): panel records,
-    // (panel, block) items, per-panel completion counters, partial sums (sn_prows per column)
+    // the FP64 solve's 64-row panels: panel records and items (rows of panels, panel_rows.cu; in the
+    // double-FP32 and tensor-core modes column blocks, with per-panel completion counters and partial sums,
+    // sn_prows per column)
     DevBuf sn_pan, sn_pitems, sn_pcnt, sn_ppart;
     DevBuf sn_gtc, sn_tcrec;  // tensor-core schedule: digit-slice G records of every panel block
     DevBuf sn_ghl, sn_gexp;   // double-FP32 schedule: G as scaled FP32 pairs, row exponents

@@ -8,8 +8,9 @@
 // X_s is an independent dot product.  The solve is a sync-free walk over 64-row panels of the
 // supernodes in reverse order (a panel waits only on rows of higher supernodes, whose panels hold
 // smaller tickets):
-//   * FP64: each panel's product split into column blocks taken by different CTAs, partial sums
-//     added in block order by the CTA that completes the panel (panels64.cu);
+//   * FP64: a warp per four rows of a panel, queued by dependency step (panel_rows.cu); in the
+//     double-FP32 and tensor-core modes each panel's product split into column blocks taken by
+//     different CTAs, partial sums added in block order (panels64.cu, panels_tc.cu);
 //   * MIXED inner solve: one CTA per panel, BF16x3 tensor-core products (G = G_hi + G_lo and
 //     V = V_hi + V_lo in bfloat16; G V ~ G_hi V_hi + G_hi V_lo + G_lo V_hi) accumulated in FP32
 //     with mma.sync.m16n8k16, inside the FP64 refinement of refine.cu.
