@@ -7,23 +7,28 @@
 // no partial sums, counters or fences between SMs lie on that way.  Lanes take the columns 32 at a time
 // -- the chunk's own right-hand side first, from the rows' diagonal on, then the solved columns from the
 // farthest to the nearest, so that only the last few wait -- and hold the sums of four rows by up to four
-// right-hand sides, added across the lanes at the end.  G is read straight into registers, coalesced, one
-// step ahead of the products; solved columns' indices are read two steps ahead.  The order of additions
-// is fixed, so results do not depend on timing.
+// right-hand sides, added across the lanes at the end.  G is read straight into registers, coalesced, for
+// U steps at once, with their right-hand sides; solved columns' indices one such group ahead.  A poll
+// reads again all of the group's values that are pending, and a step is multiplied as soon as its own are
+// there, so that a chunk's columns cost one latency of L2 (or of HBM, for its G) a group, not one each.
+// The order of additions is fixed, so results do not depend on timing.
 //
 // Items are taken from a ticketed queue in an order in which every item waits on smaller tickets only; a
 // warp draws its next ticket before it works on the one in hand, and works on them in order, so the
 // smallest unfinished ticket is always being worked on.
 //
 // An FP64 operation holds its SM quarter's pipe for 64 cycles: a chunk of 256 rows after one of 256 costs
-// a warp 8 steps of 4 products (one right-hand side) or 8 (two), ~1 or ~2 us.  Four right-hand sides to
-// a warp read G half as often, 2 % faster on the 40^3 factor with 32 columns and slower everywhere else
-// (24^3 x 3 99 -> 154 us, 64 x 64 band x 3 79 -> 106 us); one to a warp 40 % slower there.  Five CTAs an SM
-// (92 registers): 3 / 4 / 5 / 6 / 8 take 2.09 / 1.77 / 1.72 / 1.73 / 1.81 ms on 40^3 x 32.
+// a warp 8 steps of 4 products (one right-hand side) or 8 (two), ~1 or ~2 us.  U = 4 and 2 for them, 2 and 1
+// where registers are few.  Bands of 64 / 128 / 181 / 256 with one right-hand side, against one step read
+// ahead: 50 / 201 / 619 / 1994 -> 39 / 139 / 369 / 864 us (U = 2: 1071 at 256; own and solved columns in
+// one group 63 / 213 / 541 / 1231, its first products held up by the wait), the 40^3 factor 183 -> 159 us.
+// Four right-hand sides to a warp read G half as often, 2 % faster on the 40^3 factor with 32 columns and
+// slower everywhere else (24^3 x 3 99 -> 154 us, 64 x 64 band x 3 79 -> 106 us); one to a warp 40 % slower
+// there.  Five CTAs an SM (96 registers): 3 / 4 / 5 / 6 / 8 took 2.09 / 1.77 / 1.72 / 1.73 / 1.81 ms on 40^3 x 32.
 //
 // Measured on GB300 against column blocks of 64-row panels with partial sums in global memory: the 40^3
-// dissection factor with 1 / 8 / 32 right-hand sides 538 / 1375 / 4282 -> 184 / 540 / 1725 us (the last is
-// 75 % of the FP64 rate), the 64 x 64 band factor 97 -> 60 us (a chain of 16 steps of ~2 us).
+// dissection factor with 1 / 32 right-hand sides 538 / 4282 -> 156 / 1680 us (the last is 77 % of the FP64
+// rate), the 64 x 64 band factor 99 -> 39 us (a chain of 16 steps of ~2 us).
 #include <algorithm>
 #include "common.cuh"
 #include "batch.cuh"
@@ -32,36 +37,8 @@ namespace sptrsv {
 
 constexpr int kRowsItem = kPanelRows;  // rows of an item
 
-// Waits until no lane's value at p[0 .. NC) is pending (lanes with want only).  Returns false on timeout or
-// abort.
-template <int NC>
-__device__ __noinline__ bool rows_wait(bool want, const double* p, double (&v)[NC], Ctl* ctl, int64_t budget) {
-    uint64_t t0 = 0;
-    for (unsigned q = 0;; ++q) {
-        bool pend = false;
-        if (want)
-#pragma unroll
-            for (int j = 0; j < NC; ++j)
-                if (Pend<double>::is(v[j])) {
-                    v[j] = ld_relaxed(p + j);
-                    pend |= Pend<double>::is(v[j]);
-                }
-        if (!__any_sync(0xffffffffu, pend)) return true;
-        if (q >= 4) __nanosleep(q < 256 ? 20 : 100);
-        if ((q & 63u) == 63u) {
-            bool ok = !aborted(ctl);
-            if (t0 == 0) t0 = gtimer();
-            else if (ok && (int64_t)(gtimer() - t0) > budget) {
-                record_error(ctl, SPTRSV_ERR_TIMEOUT);
-                ok = false;
-            }
-            if (!__all_sync(0xffffffffu, ok)) return false;
-        }
-    }
-}
-
-// Rows [r, r + nr) of the chunk by right-hand sides [c0, c0 + NC).
-template <int NC>
+// Rows [r, r + nr) of the chunk by right-hand sides [c0, c0 + NC), U steps of 32 columns at a time.
+template <int NC, int U>
 __device__ __forceinline__ bool rows_item(const BChunk& C, int r, int nr, int m, int c0,
                                           const double* __restrict__ b, double* x, Ctl* ctl, int64_t budget) {
     constexpr int R = kRowsItem;
@@ -71,59 +48,84 @@ __device__ __forceinline__ bool rows_item(const BChunk& C, int r, int nr, int m,
 #pragma unroll
     for (int i = 0; i < R; ++i) g[i] = C.g64 + (size_t)(r + min(i, nr - 1)) * C.ld;
     const int n_own = (w - r + 31) >> 5, n_all = n_own + ((M + 31) >> 5);
-    // step s: the lane's column of G (-1: none) and where its right-hand side is
-    auto column = [&](int s) -> int {
-        if (s < n_own) {
-            const int k = r + 32 * s + lane;
-            return k < w ? k : -1;
-        }
-        const int k = 32 * (n_all - 1 - s) + lane;
-        return s < n_all && k < M ? w + k : -1;
-    };
-    auto source = [&](int s, int k) -> const double* {
-        if (k < 0) return nullptr;
-        return s < n_own ? b + (size_t)(C.a + k) * m + c0 : x + (size_t)C.rect[k - w] * m + c0;
-    };
-    auto load = [&](int s, int k, const double* p, double (&gv)[R], double (&v)[NC]) {
-#pragma unroll
-        for (int i = 0; i < R; ++i) gv[i] = k >= 0 ? __ldg(g[i] + k) : 0.0;
-#pragma unroll
-        for (int j = 0; j < NC; ++j) {
-            v[j] = 0.0;
-            if (k >= 0) v[j] = s < n_own ? __ldg(p + j) : ld_relaxed(p + j);
-        }
-    };
     double acc[R * NC];
 #pragma unroll
     for (int q = 0; q < R * NC; ++q) acc[q] = 0.0;
-    int k0 = column(0), k1 = column(1);
-    const double* p0 = source(0, k0);
-    const double* p1 = source(1, k1);
-    double gv[R], v[NC];
-    load(0, k0, p0, gv, v);
-    for (int s = 0; s < n_all; ++s) {
-        const int k2 = column(s + 2);
-        const double* p2 = source(s + 2, k2);
-        double gn[R], vn[NC];
-        load(s + 1, k1, p1, gn, vn);
-        if (s >= n_own) {
-            bool pend = false;
+    double gv[U][R], v[U][NC];
+    int at[U];
+    auto load_g = [&](int u, int k) {
 #pragma unroll
-            for (int j = 0; j < NC; ++j) pend |= k0 >= 0 && Pend<double>::is(v[j]);
-            if (__any_sync(0xffffffffu, pend) && !rows_wait<NC>(pend, p0, v, ctl, budget)) return false;
-        }
+        for (int i = 0; i < R; ++i) gv[u][i] = k >= 0 ? __ldg(g[i] + k) : 0.0;
+    };
+    auto multiply = [&](int u) {
 #pragma unroll
         for (int i = 0; i < R; ++i)
 #pragma unroll
-            for (int j = 0; j < NC; ++j) acc[i * NC + j] = fma(gv[i], v[j], acc[i * NC + j]);
+            for (int j = 0; j < NC; ++j) acc[i * NC + j] = fma(gv[u][i], v[u][j], acc[i * NC + j]);
+    };
+    // solved columns, from the farthest; the lane's column of step s (-1: none) and its row of x
+    auto column = [&](int s) -> int {
+        const int k = 32 * (n_all - 1 - s) + lane;
+        return s < n_all && k < M ? w + k : -1;
+    };
+    auto row = [&](int s) -> int {
+        const int k = column(s);
+        return k < 0 ? -1 : C.rect[k - w];
+    };
 #pragma unroll
-        for (int i = 0; i < R; ++i) gv[i] = gn[i];
+    for (int u = 0; u < U; ++u) at[u] = row(n_own + u);
+    for (int s = 0; s < n_own; s += U) {
 #pragma unroll
-        for (int j = 0; j < NC; ++j) v[j] = vn[j];
-        k0 = k1;
-        p0 = p1;
-        k1 = k2;
-        p1 = p2;
+        for (int u = 0; u < U; ++u) {
+            const int k = r + 32 * (s + u) + lane;
+            load_g(u, k < w ? k : -1);
+#pragma unroll
+            for (int j = 0; j < NC; ++j) v[u][j] = k < w ? __ldg(b + (size_t)(C.a + k) * m + c0 + j) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (s + u < n_own) multiply(u);
+    }
+    for (int s = n_own; s < n_all; s += U) {
+        int next[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            load_g(u, column(s + u));
+#pragma unroll
+            for (int j = 0; j < NC; ++j) v[u][j] = at[u] >= 0 ? ld_relaxed(x + (size_t)at[u] * m + c0 + j) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) next[u] = row(s + U + u);
+        uint64_t t0 = 0;
+        unsigned q = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (s + u >= n_all) break;
+            for (;; ++q) {
+                bool pend = false;
+#pragma unroll
+                for (int j = 0; j < NC; ++j) pend |= at[u] >= 0 && Pend<double>::is(v[u][j]);
+                if (!__any_sync(0xffffffffu, pend)) break;
+                if (q >= 4) __nanosleep(q < 256 ? 20 : 100);
+                if ((q & 63u) == 63u) {
+                    bool ok = !aborted(ctl);
+                    if (t0 == 0) t0 = gtimer();
+                    else if (ok && (int64_t)(gtimer() - t0) > budget) {
+                        record_error(ctl, SPTRSV_ERR_TIMEOUT);
+                        ok = false;
+                    }
+                    if (!__all_sync(0xffffffffu, ok)) return false;
+                }
+#pragma unroll
+                for (int z = u; z < U; ++z)
+#pragma unroll
+                    for (int j = 0; j < NC; ++j)
+                        if (at[z] >= 0 && Pend<double>::is(v[z][j])) v[z][j] = ld_relaxed(x + (size_t)at[z] * m + c0 + j);
+            }
+            multiply(u);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) at[u] = next[u];
     }
     // sums across the lanes: halves exchanged while a lane holds more than one, so R * NC + log2 additions
     // in all; lane l ends with sum (l >> shift)
@@ -184,8 +186,8 @@ __global__ void __launch_bounds__(128, kBeside ? 8 : 5) k_panel_rows(const BSys*
         const double* b = bbase + xb0;
         double* x = xbase + xb0;
         bool ok;
-        if (nc == 1) ok = rows_item<1>(C, r, nr, m, c0, b, x, ctl, budget);
-        else ok = rows_item<kPanelCols>(C, r, nr, m, c0, b, x, ctl, budget);
+        if (nc == 1) ok = rows_item<1, kBeside ? 2 : 4>(C, r, nr, m, c0, b, x, ctl, budget);
+        else ok = rows_item<kPanelCols, kBeside ? 1 : 2>(C, r, nr, m, c0, b, x, ctl, budget);
         if (!ok) break;
     }
 }

@@ -61,3 +61,26 @@ def test_batch_keeps_its_panels_when_the_mode_changes(orc, before, after):
             ref = orc.base_gauss_upper(m.row_ptr.astype(np.uint64), m.col, m.val, bs.T.copy().reshape(-1), r)
             assert _close(xs.T.reshape(-1), ref) <= 1e-8
     B.close()
+
+
+@pytest.mark.parametrize("rhs", [1, 2])
+@pytest.mark.parametrize("band", [1, 31, 32, 33, 64, 65, 96, 97, 128, 129, 160, 255])
+@pytest.mark.parametrize("chunk", [4, 37, 129, 250])
+def test_bands_around_the_groups_of_steps(orc, chunk, band, rhs):
+    """Own and solved columns around one to eight steps of 32, read two and four at a time."""
+    n = 700
+    k = np.minimum(band, n - 1 - np.arange(n))
+    rp = np.zeros(n + 1, np.int64)
+    rp[1:] = np.cumsum(1 + k)
+    off = np.arange(rp[-1]) - np.repeat(rp[:-1], 1 + k)
+    col = (np.repeat(np.arange(n), 1 + k) + off).astype(np.int32)
+    val = np.where(off == 0, 2.0, np.random.default_rng(band).uniform(-1.0, 1.0, len(off)) / band)
+    b = gen.uniform(rhs, n * rhs)
+    rpu = rp.astype(np.uint64)
+    ref = orc.base_gauss_upper(rpu, col, val, b, rhs)
+    with sp.Solver(0) as s:
+        s.analyse(rp, col, val)
+        s.set_supernodes(np.append(np.arange(0, n, chunk), n).astype(np.int32))
+        x = s.solve(b, rhs=rhs, schedule="supernodal")
+    assert _close(x, ref) <= 1e-10
+    assert orc.rel_residual(rpu, col, val, x, b, rhs) <= 1e-12
