@@ -469,7 +469,7 @@ def run_ours(args, dist):
     dom_times = [t for t in per_kind[dom_kind] if t > 0]
     dom_avg_ms = sum(dom_times) / len(dom_times)
     if dom_kind == 9:
-        dom_bytes, dom_name = jacobi_bytes(n, nnz), "k_jacobi_pairs"
+        dom_bytes, dom_name = jacobi_bytes(n, nnz), "k_jacobi_bulk"
     elif dom_kind == 7:
         dom_bytes, dom_name = fp64_bytes(n, nnz) - 8 * n, "k_residual_tile"
     else:
@@ -848,7 +848,7 @@ def batch_record(args, dist, steps, warmup, with_cpu=True, sample_errors=True):
                                      for k, v in sp.BATCH_SCHED.items() if np.any(sched == v)},
         "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": nb, "d2h_bytes_per_step": nb},
         "roofline": ({"bound": "hbm", "kernel": {"residual_f64": "k_b_residual", "jacobi_sweep": "k_b_jacobi",
-                                                 "panels_f64": "k_panels64"}[dom],
+                                                 "panels_f64": "k_panel_rows"}[dom],
                       "achieved": dom_bytes / (dom_first * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                       "frac": dom_bytes / (dom_first * 1e-3) / 1e9 / peak, "peak_source": peak_src, "traffic": None,
                       "algorithmic_bytes_per_launch": dom_bytes, "launch_ms": dom_first,
