@@ -1453,10 +1453,11 @@ template <int R, int S>
 struct BulkShape {
     int cap, tiles, keep;
     size_t smem;
+    // a stage holds the mean tile (half a row's entries and pads) and a tenth more; larger tiles are
+    // read from global memory.  At most 61 KB (kShortRowLen).
+    static int pairs(double mean_len) { return (int)(R * 0.55 * (mean_len - 0.45)) + 16; }
     explicit BulkShape(const RefineArgs& a) {
-        // a stage holds the mean tile (half a row's entries and pads) and a tenth more; larger tiles are
-        // read from global memory.  At most 61 KB (14 entries a row).
-        cap = (int)(R * 0.55 * ((double)a.nnz / a.n - 0.45)) + 16;
+        cap = pairs((double)a.nnz / a.n);
         smem = (size_t)cap * 16 * S;
         tiles = (int)(((long long)a.n + R - 1) / R);
         const double bytes = 8.0 * ((double)a.nnz - 0.5 * a.n), room = 60e6 - (4.0 + 12.0 * a.rhs) * a.n;
@@ -1479,7 +1480,9 @@ struct BulkShape {
     }
     int grid(const void* fn, const RefineArgs& a, int* blocks) const {
         int per_sm = 0;
-        CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // (the limit belongs to the kernel on the device: the largest any matrix asks for, for every thread's
+        // launches)
+        CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pairs(kShortRowLen) * 16 * S));
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, R + 32, smem));
         if (per_sm < 1) return SPTRSV_ERR_UNSUPPORTED;
         *blocks = std::min(tiles, per_sm * a.sm_count);

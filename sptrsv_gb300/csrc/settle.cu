@@ -302,7 +302,9 @@ static int settle_t(const SolveArgs& a, int* worst) {
     const int cap = std::min(fit, (int)(mean + 4.0 * std::sqrt(mean)) + 15) / 8 * 8;
     const size_t bytes = kSetWarps * set_warp_bytes(cap, NC, SetShape<NC>::kBufs);
     const void* fn = (const void*)k_settle<NC>;
-    CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // the limit belongs to the kernel on the device: the largest any matrix asks for, so that no thread's
+    // launch finds it lowered by another's
+    CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSetSmem));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSetWarps * 32, bytes));
     if (per_sm < 1) return SPTRSV_ERR_UNSUPPORTED;
