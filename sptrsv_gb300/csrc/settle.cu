@@ -314,8 +314,10 @@ static int settle_t(const SolveArgs& a, int* worst) {
     // rows 290 / 282 / 283, 200k rows 489 / 496 / 435.  Several: 10k rows x 8 310 / 384 us at 2 / 4.
     const int shortest = NC > 1 ? 2 : ntiles <= a.sm_count * kSetWarps ? 1 : 3;
     const int warps = std::max(1, std::min(per_sm * a.sm_count * kSetWarps, ntiles / shortest));
+    // a caller's budget is for waits on rows: a sweep over millions of rows keeps a barrier waiting longer
+    const int64_t budget = std::max<int64_t>(a.budget, kDefaultBudgetNs);
     SettleArgs s{a.n, a.rhs, a.rp, a.col, (const double*)a.val, (const double*)a.invd, (const double*)a.b, (double*)a.x,
-                 a.ctl, worst, a.budget, (ntiles + warps - 1) / warps, cap};
+                 a.ctl, worst, budget, (ntiles + warps - 1) / warps, cap};
     const int grid = ((ntiles + s.tiles - 1) / s.tiles + kSetWarps - 1) / kSetWarps;
     void* args[] = {(void*)&s};
     CUDA_TRY(cudaLaunchCooperativeKernel(fn, grid, kSetWarps * 32, args, bytes, a.st));
