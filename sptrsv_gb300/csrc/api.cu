@@ -48,6 +48,12 @@ __global__ void k_narrow_rp(int count, const int64_t* __restrict__ in, int* __re
     }
 }
 
+cudaError_t launch_cooperative(const void* fn, int grid, int block, void** args, size_t smem, cudaStream_t st) {
+    const char* e = getenv("SPTRSV_NO_COOPERATIVE");
+    if (e && e[0] == '1') return cudaErrorNotSupported;
+    return cudaLaunchCooperativeKernel(fn, grid, block, args, smem, st);
+}
+
 int Handle::mark(int kind) {
     if (!profiling) return 0;
     if (prof_n >= (int)prof_ev.size()) {
@@ -271,7 +277,7 @@ static bool auto_window(double mean_len) {
 bool Handle::settle_pays(int rhs) const {
     const double depth = levels_ready ? (double)max_level : depth_est;
     const double sweeps_us = 22.0 * (9.0 + 4.5e-6 * (double)nnz * rhs);
-    return mean_len <= kSettleMaxLen && sweeps_us < 0.7 * (rhs == 1 ? 0.19 : 2.0) * depth;
+    return !settle_refused && mean_len <= kSettleMaxLen && sweeps_us < 0.7 * (rhs == 1 ? 0.19 : 2.0) * depth;
 }
 
 // The exact sync-free kernel of FP64 AUTO: for one RHS the window or the block kernel (auto_window),
@@ -845,6 +851,18 @@ int Handle::run_solve(const sptrsv_opts* o_in, const double* b, double* x, int r
     if (o_in && o_in->schedule == kSchedSettle) return SPTRSV_ERR_UNSUPPORTED;
     sptrsv_opts o = resolve(o_in, rhs);
     if (o.precision == SPTRSV_PREC_MIXED && rhs > 1024) return SPTRSV_ERR_UNSUPPORTED;
+    int rc = run_resolved(o, b, x, rhs, layout);
+    if (rc && o.schedule == kSchedSettle) {
+        // the sweeps could not be set up (no cooperative launches, no memory): the exact kernel needs neither
+        (void)cudaGetLastError();
+        settle_refused = true;
+        o.schedule = exact_schedule(rhs);
+        rc = run_resolved(o, b, x, rhs, layout);
+    }
+    return rc;
+}
+
+int Handle::run_resolved(const sptrsv_opts& o, const double* b, double* x, int rhs, int layout) {
     int rc;
     if ((rc = prepare(o, rhs, layout))) return rc;
     last_mixed = o.precision == SPTRSV_PREC_MIXED;

@@ -129,7 +129,7 @@ static int solve_host_timed(Handle* h, const sptrsv_opts& o, const double* b, do
     CUDA_TRY(cudaMemcpyAsync(h->db.p, b, bytes, cudaMemcpyHostToDevice, h->st));
     // warm the graph cache / allocations outside the timed region
     sptrsv_opts r = h->resolve(&o, rhs);
-    if ((rc = h->prepare(r, rhs, layout))) return rc;
+    if ((rc = h->prepare(r, rhs, layout)) && r.schedule != kSchedSettle) return rc;  // (solve() falls back)
     // One solve per matrix: its kernels are launched directly.  Capturing and instantiating a graph to run
     // it once costs ~40 us; only the device-looped refinement needs one.
     CUDA_TRY(cudaEventRecord(h->ev0, h->st));

@@ -162,6 +162,7 @@ struct Handle {
     int ensure_levels();
     int build_csc();
     bool settle_pays(int rhs) const;
+    bool settle_refused = false;  // the sweeps could not be launched: FP64 AUTO takes the exact kernels
     int exact_schedule(int rhs) const;
     sptrsv_opts resolve(const sptrsv_opts* o, int rhs) const;
     int prepare(const sptrsv_opts& o, int rhs, int layout);
@@ -189,6 +190,7 @@ struct Handle {
     int copy_ctl();
     int solve(const sptrsv_opts* o, const double* b, double* x, int rhs, int layout);
     int run_solve(const sptrsv_opts* o, const double* b, double* x, int rhs, int layout);
+    int run_resolved(const sptrsv_opts& o, const double* b, double* x, int rhs, int layout);
     int sync();
 };
 

@@ -23,6 +23,8 @@ struct Scratch {
 };
 
 // api.cu
+// A cooperative launch; SPTRSV_NO_COOPERATIVE=1 has it refused, as some MPS set-ups do.
+cudaError_t launch_cooperative(const void* fn, int grid, int block, void** args, size_t smem, cudaStream_t st);
 __global__ void k_narrow_rp(int count, const int64_t* in, int* out, Ctl* ctl);
 
 // analysis.cu

@@ -1506,7 +1506,7 @@ int launch_jacobi_loop(const RefineArgs& a, float eps, int max_sweeps) {
     int rc = shape.grid(fn, a, &blocks);
     if (rc) return rc;
     void* args[] = {(void*)&A};
-    CUDA_TRY(cudaLaunchCooperativeKernel(fn, blocks, R + 32, args, shape.smem, a.st));
+    CUDA_TRY(launch_cooperative(fn, blocks, R + 32, args, shape.smem, a.st));
     ++*a.launches;
     return 0;
 }

@@ -320,7 +320,7 @@ static int settle_t(const SolveArgs& a, int* worst) {
                  a.ctl, worst, budget, (ntiles + warps - 1) / warps, cap};
     const int grid = ((ntiles + s.tiles - 1) / s.tiles + kSetWarps - 1) / kSetWarps;
     void* args[] = {(void*)&s};
-    CUDA_TRY(cudaLaunchCooperativeKernel(fn, grid, kSetWarps * 32, args, bytes, a.st));
+    CUDA_TRY(launch_cooperative(fn, grid, kSetWarps * 32, args, bytes, a.st));
     ++*a.launches;
     return 0;
 }

@@ -24,3 +24,26 @@ def test_small_spin_budget(solver):
     y = solver.solve(b)
     x = solver.solve(b, spin_budget_ns=20_000)
     assert np.max(np.abs(x - y)) <= 1e-12 * np.max(np.abs(y))
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+@pytest.mark.parametrize("rhs", [1, 3])
+def test_without_cooperative_launches(monkeypatch, graphs, rhs):
+    """Cooperative launches refused: FP64 AUTO and the mixed solve answer all the same, on a handle and on host arrays."""
+    m = gen.random_upper(20_000, 8.0, 0.9, 64, 5)
+    b = gen.uniform(6, m.n * rhs)
+    with sp.Solver(0) as s:
+        y = s.analyse(m.row_ptr, m.col, m.val).solve(b, rhs=rhs, schedule="syncfree_window" if rhs == 1 else "syncfree_warp")
+    monkeypatch.setenv("SPTRSV_NO_COOPERATIVE", "1")
+    if not graphs:
+        monkeypatch.setenv("SPTRSV_NO_GRAPH", "1")
+    with sp.Solver(0) as s:
+        s.analyse(m.row_ptr, m.col, m.val)
+        for _ in range(2):
+            x = s.solve(b, rhs=rhs)  # (the window kernel's last bits follow its timing, the warp kernel's do not)
+            assert np.max(np.abs(x - y)) <= (1e-12 * np.max(np.abs(y)) if rhs == 1 else 0.0)
+        x = s.solve(b, rhs=rhs, precision="mixed")
+        assert np.max(np.abs(x - y)) <= 1e-9 * np.max(np.abs(y))
+    z = np.zeros_like(b)
+    assert sp.base_gauss_upper(m.n, m.val, m.row_ptr.astype(np.uint64), m.col, z, b, rhs) >= 0
+    assert np.max(np.abs(z - y)) <= 1e-9 * np.max(np.abs(y))
