@@ -5,19 +5,20 @@
 // computes what the exact kernels compute, from any start and in any order, once the sweeps stand
 // still; they do after a few dozen when U's off-diagonals are small against its diagonal, instead of
 // after as many dependent hops as the DAG has levels.  A sweep reads U once at bandwidth, a hop costs
-// 0.2 us on one CTA.  A matrix whose sweeps do not contract is given up after a few of them (see
-// settle_hopeless) and solved by the exact kernel launched behind this one, which returns at once
+// 0.2 us on one CTA.  A matrix whose sweeps contract too slowly is given up after a few of them (see
+// settle_verdict) and solved by the exact kernel launched behind this one, which returns at once
 // when this one has finished (ctl->done).
 //
-// When it stands still: every row's new value differs from the one it replaces by less than 2^-48 of
-// the largest of |x_i|, |b_i / U_ii| and the terms |U_ij x_j / U_ii| it is formed from.  That is the
-// size of the rounding error substitution itself may make in forming x_i (k + 1 half-ulps of the sum of
-// k terms' sizes: 2^-48 of the largest for eight terms), so the result is substitution's with local errors
-// of the same size, and what is left after the last sweep has contracted once more.  By then a few hundred
-// rows of millions still move by more than an ulp.  Measured against 64-bit references
-// at 10k to 2M rows: 1.1e-16 in norm (the exact kernels: 1.1e-16 to 1.6e-16) and at most 1e-15 of the
-// root mean square, with bounds of 2^-52 to 2^-48 alike.  (A sweep gains about four bits; after the 13 or so
-// that bring most rows there, the slowest rounding flips take as many again to die out.)
+// When it stands still: a sweep's record is the largest change of any row, relative to the largest of
+// |x_i|, |b_i / U_ii| and the terms |U_ij x_j / U_ii| that row is formed from.  The change is not the
+// error: with a rate rho a sweep, rho / (1 - rho) of it is left, as much as the change itself at one bit a
+// sweep.  So the rate is read from the records where contraction rules them (2^-40; from 2^-48 on,
+// rounding flips keep a few hundred rows of millions moving by a few ulps for as many sweeps again), and
+// the sweeps go on until what is left at that rate is below 2^-54, half the rounding of one term.
+// Emulated on the CPU against 80-bit solutions, 20,000 rows, error in norm as a multiple of
+// substitution's: chains x_i = b_i + w x_i+1 with w = 0.3 / 0.5 / 0.6 / 0.7 1.01 / 1.00 / 1.12 / 1.08
+// (stopped at a record of 2^-48: 1.0 / 1.1 / 1.5 / 6.6), two entries of 0.35 0.92 (12), eight of 0.075
+// 0.66 (3.2), the random recipe 0.72 (0.72: it gains four bits a sweep).
 //
 // Sweep order.  Each warp owns a contiguous run of rows and walks it upwards from its bottom, 32 rows
 // a tile (lane per row; 32 / NC rows for NC right-hand sides), writing x in place: a row sees this
@@ -46,7 +47,9 @@ namespace sptrsv {
 constexpr int kSetWarps = 8;
 constexpr size_t kSetSmem = 220 * 1024;
 constexpr int kSetPending = 5000;  // offset of a sweep's record: 0 = nothing changed
+constexpr int kSetRated = kSetPending - 40;  // the rate is read at the first record at or below
 constexpr int kSetStill = kSetPending - 49;  // changes below 2^-48 (the exponents are floors)
+constexpr float kSetLeft = -54.f;            // what may be left when the sweeps end
 
 struct SettleArgs {
     int n, rhs;
@@ -90,13 +93,26 @@ __device__ __forceinline__ int d_gap(double a, double b) {
     return lo - 52 + 63 - __clzll(x > y ? x - y : y - x);
 }
 
-// After sweep p (from 0): whether to leave the matrix to the exact kernel.  From the ninth sweep on the
-// largest change has to lose at least a bit a sweep over the last four, until it is within 2^-40 of
-// its row's size, where single rows decide it.
-__device__ __forceinline__ bool settle_hopeless(const int* worst, int p) {
-    if (p < 8) return false;
-    const int now = ld_relaxed(worst + p), then = ld_relaxed(worst + p - 4);
-    return now > kSetPending - 40 && now > then - 4;
+// After sweep p (from 0), of at most `most`: 0 go on, 1 the solution stands still, 2 leave the matrix to
+// the exact kernel.  `last`: the sweep after which what is left is small enough, -1 until the rate is read
+// (over the last four and eight sweeps, the slower one).  Until then, from the ninth sweep on, the faster
+// one has to get there within `most`.
+__device__ __forceinline__ int settle_verdict(const int* worst, int p, int most, int& last) {
+    const int now = ld_relaxed(worst + p);
+    if (now <= 0) return 1;  // no row changed
+    const float size = (float)(now - kSetPending);
+    auto rate = [&](int back) { return (float)(ld_relaxed(worst + p - min(back, p)) - now) / (float)min(back, p); };
+    if (last < 0 && now <= kSetRated) {
+        const float g = p == 0 ? 1.f : fmaxf(0.05f, fminf(rate(4), rate(8)));  // bits a sweep
+        last = p + max(0, (int)ceilf((size + 1.f - log2f(exp2f(g) - 1.f) - kSetLeft) / g));
+    }
+    if (last >= 0) {
+        if (p >= last && now <= kSetStill) return 1;
+        return last < most ? 0 : 2;
+    }
+    if (p < 8) return 0;
+    const float g = fmaxf(rate(4), rate(8));
+    return g > 0.f && (float)p + (size - kSetLeft) / g <= (float)most ? 0 : 2;
 }
 
 __device__ __forceinline__ void set_cp4(void* s, const void* g) {
@@ -166,6 +182,7 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 
+    int last = -1;
     for (int p = 0; p < kSettleSweeps; ++p) {
         if (threadIdx.x == 0) s_worst = 0;
         __syncthreads();
@@ -271,14 +288,12 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
         __syncthreads();
         if (threadIdx.x == 0 && s_worst > 0) atomicMax(A.worst + p, s_worst);
         if (!grid_barrier(A.ctl, gridDim.x, A.budget)) return;
-        if (ld_relaxed(A.worst + p) <= kSetStill) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                A.ctl->done = 1;
-                A.ctl->steps = p + 1;
-            }
-            return;
+        const int verdict = settle_verdict(A.worst, p, kSettleSweeps, last);
+        if (verdict == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
+            A.ctl->done = 1;
+            A.ctl->steps = p + 1;
         }
-        if (settle_hopeless(A.worst, p)) return;
+        if (verdict) return;
     }
 }
 
