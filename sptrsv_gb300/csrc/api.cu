@@ -387,7 +387,7 @@ int Handle::prepare(const sptrsv_opts& o, int rhs, int layout) {
         if ((rc = grow(norms, sizeof(double) * 2 * (size_t)rhs))) return rc;
     }
     if (o.schedule == kSchedSettle)
-        if ((rc = grow(settle, sizeof(int) * kSettleSweeps))) return rc;
+        if ((rc = grow(settle, settle_work(n, rhs)))) return rc;
     if (o.schedule == SPTRSV_SCHED_SYNCFREE_CSC && o.precision == SPTRSV_PREC_FP64) {
         if ((rc = build_csc())) return rc;
         if ((rc = grow(indeg_work, sizeof(int) * (size_t)n))) return rc;
@@ -439,7 +439,7 @@ int Handle::enqueue(const sptrsv_opts& o, const double* b, double* x, int rhs, i
     if (o.precision == SPTRSV_PREC_FP64) {
         switch (o.schedule) {
             case kSchedSettle:
-                if ((rc = launch_settle(a, settle.as<int>()))) return rc;
+                if ((rc = launch_settle(a, settle.p))) return rc;
                 if ((rc = mark(SPTRSV_K_SETTLE))) return rc;
                 // the exact kernel, for a matrix whose sweeps did not contract
                 switch (exact_schedule(rhs)) {

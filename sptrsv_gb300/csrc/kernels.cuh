@@ -90,11 +90,12 @@ int launch_transpose(bool to_row_major, const double* src, double* dst, int n, i
                      int64_t* launches);
 
 // settle.cu: FP64 sweeps in place until the solution stands still; sets ctl->done (and prepares the
-// exact kernel launched behind it: x pending and rows to claim only when it is not set).  `worst`:
-// kSettleSweeps ints of device memory.
+// exact kernel launched behind it: x pending and rows to claim only when it is not set).  `work`:
+// settle_work bytes of device memory.
 constexpr int kSettleSweeps = 64;
 constexpr double kSettleMaxLen = 20.0;  // mean entries per row
-int launch_settle(const SolveArgs& a, int* worst);
+size_t settle_work(int n, int rhs);
+int launch_settle(const SolveArgs& a, void* work);
 
 // supernodal.cu -- the panel work list and dense panels of a supernode partition
 struct SnArgs {

@@ -21,11 +21,19 @@
 // 0.66 (3.2), the random recipe 0.72 (0.72: it gains four bits a sweep).
 //
 // Sweep order.  Each warp owns a contiguous run of rows and walks it upwards from its bottom, 32 rows
-// a tile (lane per row; 32 / NC rows for NC right-hand sides), writing x in place: a row sees this
-// sweep's values of everything below it in the run, so only columns inside the tile, across the run's
-// lower edge and far away are one sweep old.  Those inside the tile are a quarter of a 64-column band
+// a tile (lane per row; 32 / NC rows for NC right-hand sides): a row sees this sweep's values of
+// everything below it in the run, so only columns inside the tile, across the run's lower edge and far
+// away are one sweep old.  Those inside the tile are a quarter of a 64-column band
 // and cost the most sweeps, so with one right-hand side a tile's changes are folded in once more
 // before they are written (k_settle, "second look"): half the sweeps for a third more arithmetic.
+//
+// Repeatability.  With several right-hand sides the exact kernel (a warp per row) gives the same bits every
+// time, and so do the sweeps: they go from one vector to another, and a row outside the run is always the
+// last sweep's.  With one, the exact kernel's last bits follow its timing (the window kernel's rows split
+// their sums where they have to wait), and x is swept in place: another run's row may be this sweep's or
+// the last one's, a few sweeps fewer (2M rows 15, 20 with two vectors), and the result differs by roundings
+// from solve to solve.  Two vectors cost, 8.8 entries a row: 2k rows x 8 233 -> 274 us, 10k x 2 307 -> 371,
+// 50k x 8 542 -> 740, 200k x 8 1,288 -> 1,418 (of it about a sweep for the stop above).
 //
 // Bound by the FP64 pipe (57 % active by ncu at 500k rows; an operation holds its SM quarter's pipe for 64
 // cycles, and a tile takes its longest row's count, 1.9 times the mean of 7.6 off-diagonals) and, below
@@ -35,8 +43,7 @@
 // and L1, 90 us against 120 at 2M rows: 3.4 ms in all against 3.1 then), rows kept in shared memory for all
 // sweeps (200k rows 0.40, but 200k x 8 1.69), 16-byte copies for the staging (no change).
 //
-// One cooperative launch runs all sweeps, with a grid barrier after each; x of other warps' rows may
-// be read old or new within a sweep, and is new after the barrier.
+// One cooperative launch runs all sweeps, with a grid barrier after each.
 #include <algorithm>
 #include <cmath>
 #include "common.cuh"
@@ -59,6 +66,7 @@ struct SettleArgs {
     const double* invd;
     const double* b;
     double* x;
+    double* y;   // several right-hand sides: the other vector
     Ctl* ctl;
     int* worst;  // kSettleSweeps records: the largest change of each sweep, as an exponent
     int64_t budget;
@@ -68,6 +76,7 @@ struct SettleArgs {
 
 template <int NC> struct SetShape {
     static constexpr int kRows = 32 / NC;  // rows of a tile
+    static constexpr bool kPair = NC > 1;  // two vectors
     // One right-hand side: a tile's buffer at a time and three CTAs an SM (2M rows 1.81 ms; two buffers and
     // two CTAs 2.11, one and two 2.11, one and four 2.14).  Several: two buffers, two CTAs (200k rows x 8
     // 1.35 ms; one and three 1.42).
@@ -124,11 +133,11 @@ __device__ __forceinline__ void set_cp8(void* s, const void* g) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(g) : "memory");
 }
 
-// x changes within the launch, so never the read-only path: a warp's own run through L1 (its stores
-// update it), other rows from L2, where this sweep's values are.
-__device__ __forceinline__ double set_ld(const double* p, bool own) {
+// x changes within the launch, so never the read-only path: rows that no other warp writes in this sweep
+// through L1 (a warp's own stores update it), other rows from L2, where this sweep's values are.
+__device__ __forceinline__ double set_ld(const double* p, bool still) {
     double v;
-    if (own) asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    if (still) asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     else asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
@@ -136,6 +145,7 @@ __device__ __forceinline__ double set_ld(const double* p, bool own) {
 template <int NC>
 __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(SettleArgs A) {
     constexpr int R = SetShape<NC>::kRows, B = SetShape<NC>::kBufs;
+    constexpr bool kPair = SetShape<NC>::kPair;
     extern __shared__ __align__(16) char set_smem[];
     __shared__ int s_worst;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -187,6 +197,14 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
         if (threadIdx.x == 0) s_worst = 0;
         __syncthreads();
         int worst = 0;
+        const double* const src = kPair && (p & 1) ? A.y : A.x;
+        double* const dst = kPair && !(p & 1) ? A.y : A.x;
+        // x of a column of a tile that ends at row `top`: this sweep's in the rest of the run
+        auto x_of = [&](int c, int top, int j) {
+            const size_t k = (size_t)c * m + j;
+            if constexpr (kPair) return set_ld((c >= top && c < run_top ? dst : src) + k, true);
+            else return set_ld(src + k, c < run_top);
+        };
         Rows cur = rows_of(t0);
         if (B == 2) stage(cur, 0);
         Rows nxt = rows_of(t0 + 1);
@@ -208,7 +226,7 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
                 double acc = 0.0, bi = 0.0, old = 0.0;
                 if (mine) {
                     bi = A.b[at];
-                    old = set_ld(A.x + at, true);
+                    old = set_ld(src + at, true);
                 }
                 const int eb = d_exp(bi);
                 if (jb == 0) {
@@ -226,7 +244,7 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
                             const int q = q0 + lane + 32 * u;
                             if (q < cnt) {
                                 const int c = sc[buf * cap + q / NC];
-                                if (jb + q % NC < m) xv[u] = set_ld(A.x + (size_t)c * m + jb + q % NC, c < run_top);
+                                if (jb + q % NC < m) xv[u] = x_of(c, top, jb + q % NC);
                             }
                         }
 #pragma unroll
@@ -244,7 +262,7 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
                     for (int k = cur.s; k < cur.e; ++k) {
                         const int c = staged ? pc[k] : __ldg(A.col + k);
                         const double v = staged ? pv[k] : __ldg(A.val + k);
-                        const double xv = staged ? px[(size_t)k * NC] : set_ld(A.x + (size_t)c * m + j, c < run_top);
+                        const double xv = staged ? px[(size_t)k * NC] : x_of(c, top, j);
                         acc = fma(v, xv, acc);
                         em = max(em, ((unsigned)__double2hiint(v) & 0x7ff00000u) +
                                          ((unsigned)__double2hiint(xv) & 0x7ff00000u));
@@ -274,8 +292,9 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
                     const int size = max(d_exp(y), max(eb, (int)(em >> 20) - 1023) + ei);
                     const int gap = d_gap(y, old) - size;
                     worst = max(worst, gap + kSetPending);
-                    A.x[at] = y;
+                    if (!kPair) st_relaxed(dst + at, y);
                 }
+                if (kPair && mine) dst[at] = y;
                 __syncwarp();  // sx and dl are read before they are written again
             }
             __syncwarp();  // the staged entries are read, the tile's x written, before the next tile
@@ -293,6 +312,8 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
             A.ctl->done = 1;
             A.ctl->steps = p + 1;
         }
+        if (verdict == 1 && dst != A.x)  // the run's rows of the solution
+            for (size_t k = (size_t)max(0, n - R * t1) * m + lane; k < (size_t)max(0, run_top) * m; k += 32) A.x[k] = dst[k];
         if (verdict) return;
     }
 }
@@ -309,7 +330,7 @@ __global__ void k_settle_gate(double* x, size_t count, Ctl* ctl) {
 }
 
 template <int NC>
-static int settle_t(const SolveArgs& a, int* worst) {
+static int settle_t(const SolveArgs& a, int* worst, double* y) {
     constexpr int R = SetShape<NC>::kRows;
     // staged entries: the mean tile and four deviations of a Poisson count, if shared memory holds it
     const double mean = R * (double)a.nnz / a.n;
@@ -331,7 +352,7 @@ static int settle_t(const SolveArgs& a, int* worst) {
     const int warps = std::max(1, std::min(per_sm * a.sm_count * kSetWarps, ntiles / shortest));
     // a caller's budget is for waits on rows: a sweep over millions of rows keeps a barrier waiting longer
     const int64_t budget = std::max<int64_t>(a.budget, kDefaultBudgetNs);
-    SettleArgs s{a.n, a.rhs, a.rp, a.col, (const double*)a.val, (const double*)a.invd, (const double*)a.b, (double*)a.x,
+    SettleArgs s{a.n, a.rhs, a.rp, a.col, (const double*)a.val, (const double*)a.invd, (const double*)a.b, (double*)a.x, y,
                  a.ctl, worst, budget, (ntiles + warps - 1) / warps, cap};
     const int grid = ((ntiles + s.tiles - 1) / s.tiles + kSetWarps - 1) / kSetWarps;
     void* args[] = {(void*)&s};
@@ -340,16 +361,22 @@ static int settle_t(const SolveArgs& a, int* worst) {
     return 0;
 }
 
-// `worst`: kSettleSweeps ints of device memory.
-int launch_settle(const SolveArgs& a, int* worst) {
+// Bytes of `work`: the sweeps' records and the other vector.
+size_t settle_work(int n, int rhs) {
+    return sizeof(int) * kSettleSweeps + (rhs > 1 ? sizeof(double) * (size_t)n * rhs : 0);
+}
+
+int launch_settle(const SolveArgs& a, void* work) {
+    int* worst = (int*)work;
+    double* y = a.rhs > 1 ? (double*)(worst + kSettleSweeps) : nullptr;
     CUDA_TRY(cudaMemsetAsync(worst, 0, sizeof(int) * kSettleSweeps, a.st));
     int rc;
-    if (a.rhs == 1) rc = settle_t<1>(a, worst);
-    else if (a.rhs == 2) rc = settle_t<2>(a, worst);
-    else if (a.rhs <= 4) rc = settle_t<4>(a, worst);
-    else if (a.rhs <= 8) rc = settle_t<8>(a, worst);
-    else if (a.rhs <= 16) rc = settle_t<16>(a, worst);
-    else rc = settle_t<32>(a, worst);
+    if (a.rhs == 1) rc = settle_t<1>(a, worst, y);
+    else if (a.rhs == 2) rc = settle_t<2>(a, worst, y);
+    else if (a.rhs <= 4) rc = settle_t<4>(a, worst, y);
+    else if (a.rhs <= 8) rc = settle_t<8>(a, worst, y);
+    else if (a.rhs <= 16) rc = settle_t<16>(a, worst, y);
+    else rc = settle_t<32>(a, worst, y);
     if (rc) return rc;
     const size_t count = (size_t)a.n * a.rhs;
     k_settle_gate<<<(int)std::min<size_t>((count + 255) / 256, 2048), 256, 0, a.st>>>((double*)a.x, count, a.ctl);

@@ -47,3 +47,31 @@ def test_without_cooperative_launches(monkeypatch, graphs, rhs):
     z = np.zeros_like(b)
     assert sp.base_gauss_upper(m.n, m.val, m.row_ptr.astype(np.uint64), m.col, z, b, rhs) >= 0
     assert np.max(np.abs(z - y)) <= 1e-9 * np.max(np.abs(y))
+
+
+@pytest.mark.parametrize("n,rhs,layout", [
+    (20_000, 2, sp.ROW_MAJOR), (20_001, 3, sp.COL_MAJOR), (60_002, 4, sp.ROW_MAJOR), (200_003, 8, sp.COL_MAJOR),
+    (20_005, 17, sp.ROW_MAJOR), (20_006, 33, sp.COL_MAJOR)])
+def test_several_right_hand_sides_repeat(n, rhs, layout):
+    """With several right-hand sides FP64 AUTO repeats bit for bit, on one handle and on another."""
+    m = gen.random_upper(n, 8.0, 0.9, 64, 5)
+    b = gen.uniform(6, n * rhs)
+    first = None
+    for _ in range(2):
+        with sp.Solver(0) as s:
+            s.analyse(m.row_ptr, m.col, m.val)
+            for _ in range(4):
+                x = s.solve(b, rhs=rhs, layout=layout)
+                first = x if first is None else first
+                assert np.array_equal(x, first)
+
+
+def test_one_right_hand_side_repeats_to_rounding(solver):
+    """With one, solves differ by roundings (2^-53 of a term, a few terms to a row): the window kernel's do too."""
+    m = gen.random_upper(200_000, 8.0, 0.9, 64, 5)
+    solver.analyse(m.row_ptr, m.col, m.val)
+    b = gen.uniform(6, m.n)
+    for schedule in ("auto", "syncfree_window"):
+        x = [solver.solve(b, schedule=schedule) for _ in range(4)]
+        for y in x[1:]:
+            assert np.max(np.abs(y - x[0])) <= 16 * 2.0**-53 * np.max(np.abs(x[0]))
