@@ -96,6 +96,7 @@ void Handle::drop_matrix() {
     auto_supernodes = false;
     skyline = false;
     for (bool& v : tuned_valid) v = false;
+    settle_failed = false;
     n = nnz = max_level = 0;
     rp = col = nullptr;
     val = nullptr;
@@ -268,16 +269,26 @@ static bool auto_window(double mean_len) {
     return w < 0 ? mean_len <= 90.0 : w == 1;
 }
 
-// Whether FP64 AUTO tries the sweeps (settle.cu) before the exact kernel: when the sweeps of a
-// contracting matrix take less than 0.7 of the exact kernel's time (a matrix that does not contract
-// costs nine of them on top).  Measured on GB300, 8.8 entries a row: the time of 22 sweeps of 9 us + 4.5 us
-// per million entries and columns (10k rows 207 us, 2M rows 1.8 ms, 200k rows x 8 1.35 ms); the exact
-// kernels take 0.19 us a level with one right-hand side (10k rows 370 us, 50k rows 1.7 ms) and 2 us with
-// several (200k rows x 8 70 ms).  Tiles of long rows do not fit shared memory.
+// The exact kernels of FP64 AUTO, in microseconds.  Measured on GB300, 8.8 entries a row: 0.19 us a level with
+// one right-hand side (10k rows 370 us, 50k rows 1.7 ms) and 2 us with several (200k rows x 8 70 ms).
+double Handle::exact_us(int rhs) const { return (rhs == 1 ? 0.19 : 2.0) * (levels_ready ? (double)max_level : depth_est); }
+
+// Whether FP64 AUTO tries the sweeps (settle.cu) before the exact kernel: when the sweeps of a contracting
+// matrix take less than 0.7 of the exact kernel's time.  Rows that are not strictly dominant need not
+// contract, and nine sweeps in vain come on top of the exact kernel: there the sweeps have to take less than
+// 0.15 of its time, so that a failed attempt costs 6 %.  A matrix pays for one: its sweeps are not tried
+// again (settle_failed).  Measured on GB300, 8.8 entries a row: 22 times 9 us + 4.5 us per million entries and
+// columns (10k rows 225 us, 2M rows 1.9 ms, 200k rows x 8 1.5 ms).  Tiles of long rows do not fit shared
+// memory.
 bool Handle::settle_pays(int rhs) const {
-    const double depth = levels_ready ? (double)max_level : depth_est;
-    const double sweeps_us = 22.0 * (9.0 + 4.5e-6 * (double)nnz * rhs);
-    return !settle_refused && mean_len <= kSettleMaxLen && sweeps_us < 0.7 * (rhs == 1 ? 0.19 : 2.0) * depth;
+    return !settle_refused && !settle_failed && mean_len <= kSettleMaxLen &&
+           22.0 * (9.0 + 4.5e-6 * (double)nnz * rhs) < (max_ratio < 1.0 ? 0.7 : 0.15) * exact_us(rhs);
+}
+
+// The most sweeps: as many as take the exact kernel's time.  Small systems make more and shorter sweeps than
+// the rule above counts (10k rows: 34 of 6 us).
+int Handle::settle_most(int rhs) const {
+    return (int)std::min<double>(kSettleSweeps, exact_us(rhs) / (6.0 + 4.5e-6 * (double)nnz * rhs));
 }
 
 // The exact sync-free kernel of FP64 AUTO: for one RHS the window or the block kernel (auto_window),
@@ -439,7 +450,7 @@ int Handle::enqueue(const sptrsv_opts& o, const double* b, double* x, int rhs, i
     if (o.precision == SPTRSV_PREC_FP64) {
         switch (o.schedule) {
             case kSchedSettle:
-                if ((rc = launch_settle(a, settle.p))) return rc;
+                if ((rc = launch_settle(a, settle.p, settle_most(rhs)))) return rc;
                 if ((rc = mark(SPTRSV_K_SETTLE))) return rc;
                 // the exact kernel, for a matrix whose sweeps did not contract
                 switch (exact_schedule(rhs)) {
@@ -866,6 +877,7 @@ int Handle::run_resolved(const sptrsv_opts& o, const double* b, double* x, int r
     int rc;
     if ((rc = prepare(o, rhs, layout))) return rc;
     last_mixed = o.precision == SPTRSV_PREC_MIXED;
+    last_settle = o.schedule == kSchedSettle;
     last_cond = false;
     last_mirrored = false;
     // profiled solves launch directly: their per-step events are timed from the host stream
@@ -960,6 +972,7 @@ int Handle::sync() {
     if (ctl_copied) c = *h_ctl;
     else if (int rc = read_ctl(&c)) return rc;
     if (c.status) return c.status;
+    if (last_settle && !c.done && !c.abort) settle_failed = true;
     if (last_mixed) {
         last_steps = c.steps;
         last_sweeps = c.inner_total;

@@ -161,7 +161,11 @@ struct Handle {
     int analyse();
     int ensure_levels();
     int build_csc();
+    double exact_us(int rhs) const;
+    int settle_most(int rhs) const;
     bool settle_pays(int rhs) const;
+    bool last_settle = false;     // the last solve ran the sweeps
+    bool settle_failed = false;   // this matrix's sweeps did not settle: FP64 AUTO takes the exact kernels
     bool settle_refused = false;  // the sweeps could not be launched: FP64 AUTO takes the exact kernels
     int exact_schedule(int rhs) const;
     sptrsv_opts resolve(const sptrsv_opts* o, int rhs) const;

@@ -91,11 +91,11 @@ int launch_transpose(bool to_row_major, const double* src, double* dst, int n, i
 
 // settle.cu: FP64 sweeps in place until the solution stands still; sets ctl->done (and prepares the
 // exact kernel launched behind it: x pending and rows to claim only when it is not set).  `work`:
-// settle_work bytes of device memory.
-constexpr int kSettleSweeps = 64;
+// settle_work bytes of device memory; at most `most` sweeps.
+constexpr int kSettleSweeps = 128;  // half a bit a sweep
 constexpr double kSettleMaxLen = 20.0;  // mean entries per row
 size_t settle_work(int n, int rhs);
-int launch_settle(const SolveArgs& a, void* work);
+int launch_settle(const SolveArgs& a, void* work, int most);
 
 // supernodal.cu -- the panel work list and dense panels of a supernode partition
 struct SnArgs {

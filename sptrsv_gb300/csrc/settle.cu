@@ -70,6 +70,7 @@ struct SettleArgs {
     Ctl* ctl;
     int* worst;  // kSettleSweeps records: the largest change of each sweep, as an exponent
     int64_t budget;
+    int most;   // sweeps, up to kSettleSweeps
     int tiles;  // tiles per warp
     int cap;    // staged entries of a tile; a tile with more is read from global memory
 };
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
     };
 
     int last = -1;
-    for (int p = 0; p < kSettleSweeps; ++p) {
+    for (int p = 0; p < A.most; ++p) {
         if (threadIdx.x == 0) s_worst = 0;
         __syncthreads();
         int worst = 0;
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(kSetWarps * 32, SetShape<NC>::kCtas) k_settle(
         __syncthreads();
         if (threadIdx.x == 0 && s_worst > 0) atomicMax(A.worst + p, s_worst);
         if (!grid_barrier(A.ctl, gridDim.x, A.budget)) return;
-        const int verdict = settle_verdict(A.worst, p, kSettleSweeps, last);
+        const int verdict = settle_verdict(A.worst, p, A.most, last);
         if (verdict == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
             A.ctl->done = 1;
             A.ctl->steps = p + 1;
@@ -330,7 +331,7 @@ __global__ void k_settle_gate(double* x, size_t count, Ctl* ctl) {
 }
 
 template <int NC>
-static int settle_t(const SolveArgs& a, int* worst, double* y) {
+static int settle_t(const SolveArgs& a, int* worst, double* y, int most) {
     constexpr int R = SetShape<NC>::kRows;
     // staged entries: the mean tile and four deviations of a Poisson count, if shared memory holds it
     const double mean = R * (double)a.nnz / a.n;
@@ -353,7 +354,7 @@ static int settle_t(const SolveArgs& a, int* worst, double* y) {
     // a caller's budget is for waits on rows: a sweep over millions of rows keeps a barrier waiting longer
     const int64_t budget = std::max<int64_t>(a.budget, kDefaultBudgetNs);
     SettleArgs s{a.n, a.rhs, a.rp, a.col, (const double*)a.val, (const double*)a.invd, (const double*)a.b, (double*)a.x, y,
-                 a.ctl, worst, budget, (ntiles + warps - 1) / warps, cap};
+                 a.ctl, worst, budget, most, (ntiles + warps - 1) / warps, cap};
     const int grid = ((ntiles + s.tiles - 1) / s.tiles + kSetWarps - 1) / kSetWarps;
     void* args[] = {(void*)&s};
     CUDA_TRY(launch_cooperative(fn, grid, kSetWarps * 32, args, bytes, a.st));
@@ -366,17 +367,17 @@ size_t settle_work(int n, int rhs) {
     return sizeof(int) * kSettleSweeps + (rhs > 1 ? sizeof(double) * (size_t)n * rhs : 0);
 }
 
-int launch_settle(const SolveArgs& a, void* work) {
+int launch_settle(const SolveArgs& a, void* work, int most) {
     int* worst = (int*)work;
     double* y = a.rhs > 1 ? (double*)(worst + kSettleSweeps) : nullptr;
     CUDA_TRY(cudaMemsetAsync(worst, 0, sizeof(int) * kSettleSweeps, a.st));
     int rc;
-    if (a.rhs == 1) rc = settle_t<1>(a, worst, y);
-    else if (a.rhs == 2) rc = settle_t<2>(a, worst, y);
-    else if (a.rhs <= 4) rc = settle_t<4>(a, worst, y);
-    else if (a.rhs <= 8) rc = settle_t<8>(a, worst, y);
-    else if (a.rhs <= 16) rc = settle_t<16>(a, worst, y);
-    else rc = settle_t<32>(a, worst, y);
+    if (a.rhs == 1) rc = settle_t<1>(a, worst, y, most);
+    else if (a.rhs == 2) rc = settle_t<2>(a, worst, y, most);
+    else if (a.rhs <= 4) rc = settle_t<4>(a, worst, y, most);
+    else if (a.rhs <= 8) rc = settle_t<8>(a, worst, y, most);
+    else if (a.rhs <= 16) rc = settle_t<16>(a, worst, y, most);
+    else rc = settle_t<32>(a, worst, y, most);
     if (rc) return rc;
     const size_t count = (size_t)a.n * a.rhs;
     k_settle_gate<<<(int)std::min<size_t>((count + 255) / 256, 2048), 256, 0, a.st>>>((double*)a.x, count, a.ctl);

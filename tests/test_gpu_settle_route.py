@@ -75,3 +75,48 @@ def test_one_right_hand_side_repeats_to_rounding(solver):
         x = [solver.solve(b, schedule=schedule) for _ in range(4)]
         for y in x[1:]:
             assert np.max(np.abs(y - x[0])) <= 16 * 2.0**-53 * np.max(np.abs(x[0]))
+
+
+def _chain(n, w):
+    """x_i = b_i - w x_i+1."""
+    rp = np.zeros(n + 1, np.int64)
+    rp[1:] = np.cumsum(np.where(np.arange(n) < n - 1, 2, 1))
+    col, val = np.empty(rp[-1], np.int32), np.empty(rp[-1])
+    col[rp[:-1]], val[rp[:-1]] = np.arange(n), 1.0
+    col[rp[:-2] + 1], val[rp[:-2] + 1] = np.arange(1, n), w
+    return rp, col, val
+
+
+def _kernels(s, n, rhs):
+    s.profile(True)
+    x = s.solve(gen.uniform(1, n * rhs), rhs=rhs)
+    kinds = [k for k, _ in s.profile_read()]
+    s.profile(False)
+    return x, kinds
+
+
+SETTLE = 16
+
+
+@pytest.mark.parametrize("rhs", [1, 3])
+@pytest.mark.parametrize("w,tries", [(0.9, 1), (1.0, 1), (1.001, 1), (0.5, 9)])
+def test_sweeps_that_do_not_settle_are_tried_once(w, tries, rhs):
+    """30,000 rows deep, so that an attempt is cheap beside the exact kernel: one attempt a matrix, and the exact
+    kernel's result from the first solve on (several right-hand sides: its bits)."""
+    n = 30_000
+    with sp.Solver(0) as s:
+        s.analyse(*_chain(n, w))
+        runs = [_kernels(s, n, rhs) for _ in range(3)]
+        assert [SETTLE in k for _, k in runs] == [q < tries for q in range(3)]
+        if rhs > 1:
+            assert all(np.array_equal(x, runs[0][0]) for x, _ in runs)
+        s.analyse(*_chain(n, 0.3))  # another matrix on the handle
+        assert SETTLE in _kernels(s, n, rhs)[1]
+
+
+@pytest.mark.parametrize("w,swept", [(0.5, True), (1.0, False)])
+def test_rows_that_are_not_dominant(w, swept):
+    """3,000 rows deep, where an attempt in vain would be a good part of the exact kernel's time."""
+    with sp.Solver(0) as s:
+        s.analyse(*_chain(3_000, w))
+        assert (SETTLE in _kernels(s, 3_000, 1)[1]) == swept
