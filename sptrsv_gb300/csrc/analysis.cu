@@ -30,7 +30,7 @@ __global__ void k_to_f32(size_t count, const double* __restrict__ a, float* __re
 //   over rows of 1 / (distance to the row's nearest dependency), which is about the depth of the DAG
 //   when dependencies chain through their nearest columns (the levels themselves take a DAG traversal),
 //   stats[3] the number of rows that are not one contiguous column range from the diagonal (zero for a
-//   banded factor stored with its explicit zeros: a skyline matrix).
+//   banded factor stored with its explicit zeros: a skyline matrix), stats[4] the longest row.
 // Rows go 32 a tile.  Short ones (kLong = false): a warp per tile copies the tile's entries to shared
 // memory in order and each lane walks its own row there.  Long ones (mean above kRowsLong): a block of
 // eight warps per tile, each walking four rows, 32 entries a step.  Either way one lane finishes each
@@ -72,6 +72,7 @@ k_check_rows(int n, int nnz, const int* __restrict__ rp, const int* __restrict__
     double worst = 0.0, worst_off = 0.0, worst_d = 1.0;  // the lane's row of the largest off / |d|
     float depth = 0.f;
     unsigned long long len2 = 0, gapped = 0;
+    int longest = 0;
     const int first = kLong ? blockIdx.x : blockIdx.x * W + w, step = kLong ? gridDim.x : gridDim.x * W;
     for (int t = first; (long long)t * 32 < n; t += step) {
         const int r0 = t * 32, i = r0 + lane;
@@ -156,6 +157,7 @@ k_check_rows(int n, int nnz, const int* __restrict__ rp, const int* __restrict__
         if (e > s + 1) depth += 1.f / (float)f.near;
         gapped += f.contiguous ? 0ull : 1ull;
         len2 += (unsigned long long)(e - s) * (unsigned long long)(e - s);
+        longest = max(longest, e - s);
     }
     __syncwarp();
     if (!kLong || w == 0) {
@@ -166,11 +168,13 @@ k_check_rows(int n, int nnz, const int* __restrict__ rp, const int* __restrict__
             len2 += __shfl_xor_sync(0xffffffffu, len2, o);
             gapped += __shfl_xor_sync(0xffffffffu, gapped, o);
         }
+        longest = __reduce_max_sync(0xffffffffu, longest);
         if (lane == 0) {
             atomicMax(stats, (unsigned long long)__double_as_longlong(mr));  // mr >= 0: bit order = value order
             atomicAdd(stats + 1, len2);
             atomicAdd(reinterpret_cast<double*>(stats + 2), dep);
             atomicAdd(stats + 3, gapped);
+            atomicMax(stats + 4, (unsigned long long)longest);
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && rp[n] != nnz) record_error(ctl, SPTRSV_ERR_ROW_PTR);
@@ -179,7 +183,7 @@ k_check_rows(int n, int nnz, const int* __restrict__ rp, const int* __restrict__
 int launch_check_rows(int n, int nnz, const int* rp, const int* col, const double* val, int* in_degree, double* invd,
                       float* invd32, unsigned long long* stats, Ctl* ctl, int sm_count, cudaStream_t st,
                       int64_t* launches) {
-    CUDA_TRY(cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), st));
+    CUDA_TRY(cudaMemsetAsync(stats, 0, 5 * sizeof(unsigned long long), st));
     const int tiles = (n + 31) / 32;
     if ((double)nnz > kRowsLong * n)
         k_check_rows<true><<<std::min(tiles, sm_count * 8), kRowsLongWarps * 32, 0, st>>>(n, nnz, rp, col, val, in_degree,

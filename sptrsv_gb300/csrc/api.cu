@@ -111,11 +111,11 @@ int Handle::analyse() {
     if ((rc = invd.ensure(sizeof(double) * (size_t)n))) return rc;
     if ((rc = invd32.ensure(sizeof(float) * (size_t)n))) return rc;
     if ((rc = levels.ensure(sizeof(int) * (size_t)n))) return rc;
-    if ((rc = stats.ensure(4 * sizeof(unsigned long long)))) return rc;
+    if ((rc = stats.ensure(5 * sizeof(unsigned long long)))) return rc;
     if ((rc = launch_check_rows(n, nnz, rp, col, val, in_degree.as<int>(), invd.as<double>(), invd32.as<float>(),
                                 stats.as<unsigned long long>(), ctl, sm_count, st, &launches)))
         return rc;
-    unsigned long long hs[4];
+    unsigned long long hs[5];
     CUDA_TRY(cudaMemcpyAsync(hs, stats.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
     if ((rc = read_ctl(&c))) return rc;
     if (c.status) return c.status;
@@ -124,6 +124,7 @@ int Handle::analyse() {
     max_ratio = mr;
     memcpy(&depth_est, &hs[2], sizeof(double));
     skyline = hs[3] == 0;
+    longest = (int)hs[4];
     mean_len = (double)nnz / n;
     const double ex2 = (double)hs[1] / n;
     std_len = std::sqrt(std::fmax(0.0, ex2 - mean_len * mean_len));
@@ -278,17 +279,17 @@ double Handle::exact_us(int rhs) const { return (rhs == 1 ? 0.19 : 2.0) * (level
 // contract, and nine sweeps in vain come on top of the exact kernel: there the sweeps have to take less than
 // 0.15 of its time, so that a failed attempt costs 6 %.  A matrix pays for one: its sweeps are not tried
 // again (settle_failed).  Measured on GB300, 8.8 entries a row: 22 times 9 us + 4.5 us per million entries and
-// columns (10k rows 225 us, 2M rows 1.9 ms, 200k rows x 8 1.5 ms).  Tiles of long rows do not fit shared
-// memory.
+// columns (10k rows 225 us, 2M rows 1.9 ms, 200k rows x 8 1.5 ms), and the longest row's walk where its tile
+// is not staged (settle_long_us).
 bool Handle::settle_pays(int rhs) const {
     return !settle_refused && !settle_failed && mean_len <= kSettleMaxLen &&
-           22.0 * (9.0 + 4.5e-6 * (double)nnz * rhs) < (max_ratio < 1.0 ? 0.7 : 0.15) * exact_us(rhs);
+           22.0 * (9.0 + 4.5e-6 * (double)nnz * rhs + settle_long_us(n, nnz, rhs, longest)) < (max_ratio < 1.0 ? 0.7 : 0.15) * exact_us(rhs);
 }
 
 // The most sweeps: as many as take the exact kernel's time.  Small systems make more and shorter sweeps than
 // the rule above counts (10k rows: 34 of 6 us).
 int Handle::settle_most(int rhs) const {
-    return (int)std::min<double>(kSettleSweeps, exact_us(rhs) / (6.0 + 4.5e-6 * (double)nnz * rhs));
+    return (int)std::min<double>(kSettleSweeps, exact_us(rhs) / (6.0 + 4.5e-6 * (double)nnz * rhs + settle_long_us(n, nnz, rhs, longest)));
 }
 
 // The exact sync-free kernel of FP64 AUTO: for one RHS the window or the block kernel (auto_window),

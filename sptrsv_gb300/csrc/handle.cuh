@@ -89,6 +89,7 @@ struct Handle {
     int max_level = 0;
     double max_ratio = 0.0, mean_len = 0.0, std_len = 0.0;
     double depth_est = 0.0;  // analysis: sum over rows of 1 / (distance to the nearest dependency)
+    int longest = 0;         // analysis: entries of the longest row
     bool skyline = false;    // analysis: every row is one contiguous column range from its diagonal
     bool auto_supernodes = false;  // the supernode partition was built by prepare(), not the caller
     // FP64 AUTO solves dense skyline matrices (rows of similar length, so the dense panels stay

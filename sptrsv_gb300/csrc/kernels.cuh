@@ -95,6 +95,7 @@ int launch_transpose(bool to_row_major, const double* src, double* dst, int n, i
 constexpr int kSettleSweeps = 128;  // half a bit a sweep
 constexpr double kSettleMaxLen = 20.0;  // mean entries per row
 size_t settle_work(int n, int rhs);
+double settle_long_us(int n, long long nnz, int rhs, int longest);
 int launch_settle(const SolveArgs& a, void* work, int most);
 
 // supernodal.cu -- the panel work list and dense panels of a supernode partition

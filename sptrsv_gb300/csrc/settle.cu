@@ -330,13 +330,37 @@ __global__ void k_settle_gate(double* x, size_t count, Ctl* ctl) {
     for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) x[k] = v;
 }
 
+// Staged entries of a tile: the mean tile and four deviations of a Poisson count, if shared memory holds it.
+template <int NC>
+static int set_cap(int n, long long nnz) {
+    const double mean = SetShape<NC>::kRows * (double)nnz / n;
+    const int fit = (int)((kSetSmem / kSetWarps - 256) / (12 * SetShape<NC>::kBufs + 8 * NC));
+    return std::min(fit, (int)(mean + 4.0 * std::sqrt(mean)) + 15) / 8 * 8;
+}
+
+template <int NC>
+static double long_us_t(int n, long long nnz, int rhs, int longest) {
+    if ((SetShape<NC>::kRows - 1) * (double)nnz / n + longest <= set_cap<NC>(n, nnz)) return 0.0;
+    return (NC == 1 ? 0.2 : 0.46) * longest * ((rhs + NC - 1) / NC);
+}
+
+// What the longest row adds to a sweep, in microseconds: where its tile does not fit the staging buffer, a
+// lane walks it through global memory, an entry after the other, while the other warps wait.  Measured on
+// GB300, 40,000 rows with one row of 400 / 3,000 / 12,000 entries, 22 sweeps: 2.0 / 12.6 / 47.9 ms with one
+// right-hand side (the exact kernel 1.4 / 2.0 / 4.2), 4.5 / 31.7 / 118.8 ms with eight (11.0 / 11.3 / 12.4).
+double settle_long_us(int n, long long nnz, int rhs, int longest) {
+    if (rhs == 1) return long_us_t<1>(n, nnz, rhs, longest);
+    if (rhs == 2) return long_us_t<2>(n, nnz, rhs, longest);
+    if (rhs <= 4) return long_us_t<4>(n, nnz, rhs, longest);
+    if (rhs <= 8) return long_us_t<8>(n, nnz, rhs, longest);
+    if (rhs <= 16) return long_us_t<16>(n, nnz, rhs, longest);
+    return long_us_t<32>(n, nnz, rhs, longest);
+}
+
 template <int NC>
 static int settle_t(const SolveArgs& a, int* worst, double* y, int most) {
     constexpr int R = SetShape<NC>::kRows;
-    // staged entries: the mean tile and four deviations of a Poisson count, if shared memory holds it
-    const double mean = R * (double)a.nnz / a.n;
-    const int fit = (int)((kSetSmem / kSetWarps - 256) / (12 * SetShape<NC>::kBufs + 8 * NC));
-    const int cap = std::min(fit, (int)(mean + 4.0 * std::sqrt(mean)) + 15) / 8 * 8;
+    const int cap = set_cap<NC>(a.n, a.nnz);
     const size_t bytes = kSetWarps * set_warp_bytes(cap, NC, SetShape<NC>::kBufs);
     const void* fn = (const void*)k_settle<NC>;
     // the limit belongs to the kernel on the device: the largest any matrix asks for, so that no thread's

@@ -120,3 +120,24 @@ def test_rows_that_are_not_dominant(w, swept):
     with sp.Solver(0) as s:
         s.analyse(*_chain(3_000, w))
         assert (SETTLE in _kernels(s, 3_000, 1)[1]) == swept
+
+
+@pytest.mark.parametrize("rhs", [1, 3])
+@pytest.mark.parametrize("entries,swept", [(30, True), (3_000, False), (19_000, False)])
+def test_one_long_row(orc, entries, swept, rhs):
+    """A row that one lane would walk through global memory in every sweep goes to the exact kernel."""
+    n, at = 40_000, 20_000
+    m = gen.random_upper(n, 7.0, 0.9, 64, 5)
+    rng = np.random.default_rng(3)
+    c = np.concatenate([[at], np.sort(rng.choice(np.arange(at + 1, n), entries, replace=False))]).astype(np.int32)
+    v = np.concatenate([[entries + 1.0], rng.uniform(-1, 1, entries)])
+    a, e = m.row_ptr[at], m.row_ptr[at + 1]
+    rp = m.row_ptr.copy()
+    rp[at + 1:] += len(c) - (e - a)
+    col, val = np.concatenate([m.col[:a], c, m.col[e:]]), np.concatenate([m.val[:a], v, m.val[e:]])
+    with sp.Solver(0) as s:
+        s.analyse(rp, col, val)
+        x, kinds = _kernels(s, n, rhs)
+    assert (SETTLE in kinds) == swept
+    ref = orc.base_gauss_upper(rp.astype(np.uint64), col, val, gen.uniform(1, n * rhs), rhs)
+    assert np.max(np.abs(x - ref)) <= 1e-10 * np.max(np.abs(ref))
