@@ -143,7 +143,8 @@ SPTRSV_API int sptrsv_set_supernodes(sptrsv_handle h, int sn, const int* superno
  * columns (device buffers, CUDA events), each run capped at cap_ms after its first run and
  * repeated `reps` times otherwise; writes every candidate's best time in ms (INFINITY when not
  * applicable or failed) to cand_ms[SPTRSV_TUNE_CANDIDATES], the winner's index and options, and
- * caches the winner for the RHS class (1, 2-8, 9-32, >32), where SPTRSV_SCHED_AUTO uses it. */
+ * caches the winner for the RHS class (1, 2-8, 9-32, >32), where SPTRSV_SCHED_AUTO uses it.  FP64
+ * AUTO's own choice is timed beside them; where it is faster (by 5 %) AUTO stays with it. */
 #define SPTRSV_TUNE_CANDIDATES 16
 #define SPTRSV_FEATURES 24
 SPTRSV_API int sptrsv_autotune(sptrsv_handle h, int rhs, float cap_ms, int reps, float* cand_ms, int* best_id,

@@ -220,7 +220,8 @@ class Solver:
     def autotune(self, rhs=1, cap_ms=50.0, reps=2, abort_ms=0.0, with_censored=False):
         """Exhaustive tuning over the candidate table; returns (best id, times in ms per candidate)
         and, with_censored, the flags of candidates cancelled after abort_ms (their times are lower
-        bounds).  The winner is cached for this RHS class and used by schedule="auto"."""
+        bounds).  The winner is cached for this RHS class and used by schedule="auto", unless untuned
+        FP64 "auto" was faster."""
         ms = np.zeros(N_CANDIDATES, dtype=np.float32)
         cens = np.zeros(N_CANDIDATES, dtype=np.int32)
         best = ctypes.c_int(-1)

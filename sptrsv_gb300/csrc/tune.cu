@@ -3,7 +3,8 @@
 // The autotuner times every applicable schedule of a fixed candidate table on the resident
 // matrix (device buffers, a seeded random right-hand side, CUDA events on the handle's stream),
 // keeps the fastest that reaches the accuracy contract (FP64 paths exact; mixed paths at the
-// refinement tolerance) and caches it per RHS class, where AUTO picks it up.  A candidate whose
+// refinement tolerance) and caches it per RHS class, where AUTO picks it up, unless FP64 AUTO's own choice
+// (the sweeps of settle.cu or the window kernel, which are not in the table) was faster still.  A candidate whose
 // first run exceeds the per-candidate cap is measured once; failures (for instance a refinement
 // that does not converge) are recorded as infinite.  The timing table is returned so that it can
 // train and judge the learned selector.
@@ -140,8 +141,27 @@ int Handle::autotune(int rhs, float cap_ms, int reps, float abort_ms, float* ms_
     int K = 0;
     const sptrsv_opts* cand = tune_candidates(&K);
     static const int order[SPTRSV_TUNE_CANDIDATES] = {7, 14, 11, 12, 0, 8, 13, 2, 3, 4, 9, 10, 6, 5, 1, 15};
-    float best = INFINITY;
+    const int cls = rhs_class(rhs);
+    const bool had = tuned_valid[cls];
+    float best = INFINITY, own = INFINITY;
     int bid = -1;
+    // one time of o, the best of 1 + reps; infinite when it failed
+    auto time_of = [&](const sptrsv_opts& o, float lim, float* t, bool* cens) -> int {
+        *t = INFINITY;
+        float first = INFINITY;
+        int r = timed_candidate(o, rhs, lim, &first, cens);
+        if (r == SPTRSV_ERR_CUDA || r == SPTRSV_ERR_NO_DEVICE) return r;
+        if (r) return 0;
+        *t = first;
+        for (int k = 0; k < reps && first <= cap_ms && !*cens; ++k) {
+            float e = INFINITY;
+            bool c2 = false;
+            if ((r = timed_candidate(o, rhs, lim, &e, &c2)) || c2) break;
+            *t = std::min(*t, e);
+        }
+        if (r) *t = INFINITY;
+        return 0;
+    };
     for (int q = 0; q < K; ++q) {
         const int k = order[q];
         float t = INFINITY;
@@ -150,32 +170,25 @@ int Handle::autotune(int rhs, float cap_ms, int reps, float abort_ms, float* ms_
             const sptrsv_opts o = cand[k];
             // nothing is cancelled before one candidate has finished, so a pick always exists
             const float lim = abort_ms > 0.f && std::isfinite(best) ? std::max(abort_ms, 20.f * best) : 0.f;
-            float first = INFINITY;
-            rc = timed_candidate(o, rhs, lim, &first, &cens);
-            if (rc == 0 && !cens) {
-                t = first;
-                for (int r = 0; r < reps && first <= cap_ms; ++r) {
-                    float e = INFINITY;
-                    bool c2 = false;
-                    if ((rc = timed_candidate(o, rhs, lim, &e, &c2)) || c2) break;
-                    t = std::min(t, e);
-                }
-                if (rc) t = INFINITY;
-            } else if (rc == 0 && cens) {
-                t = first;
-            } else if (rc == SPTRSV_ERR_CUDA || rc == SPTRSV_ERR_NO_DEVICE) {
-                return rc;
-            }
-            rc = 0;
+            if ((rc = time_of(o, lim, &t, &cens))) return rc;
         }
         if (ms_out) ms_out[k] = t;
         if (censored_out) censored_out[k] = cens ? 1 : 0;
         if (!cens && t < best) { best = t; bid = k; }
     }
     if (bid < 0) return SPTRSV_ERR_UNSUPPORTED;
-    const int cls = rhs_class(rhs);
-    tuned[cls] = cand[bid];
-    tuned_valid[cls] = true;
+    sptrsv_opts untuned;
+    sptrsv_default_opts(&untuned);
+    tuned_valid[cls] = false;  // AUTO's own choice
+    bool cens = false;
+    if ((rc = time_of(untuned, abort_ms > 0.f ? std::max(abort_ms, 20.f * best) : 0.f, &own, &cens))) {
+        tuned_valid[cls] = had;
+        return rc;
+    }
+    if (cens || best <= 1.05f * own) {  // (within the noise: the pick)
+        tuned[cls] = cand[bid];
+        tuned_valid[cls] = true;
+    }
     if (best_id) *best_id = bid;
     return 0;
 }
