@@ -860,7 +860,10 @@ int Handle::run_solve(const sptrsv_opts* o_in, const double* b, double* x, int r
     if (!analysed) return SPTRSV_ERR_NO_ANALYSIS;
     if (rhs < 1 || !b || !x || (layout != SPTRSV_COL_MAJOR && layout != SPTRSV_ROW_MAJOR)) return SPTRSV_ERR_INVALID_ARG;
     if ((size_t)n * rhs > (size_t)0x7fffffff) return SPTRSV_ERR_TOO_LARGE;
-    if (o_in && o_in->schedule == kSchedSettle) return SPTRSV_ERR_UNSUPPORTED;
+    // the sweeps are AUTO's own choice: no caller names them, nor through sptrsv_set_tuned
+    const int named = o_in ? o_in->schedule : (int)SPTRSV_SCHED_AUTO, cls = rhs_class(rhs);
+    if (named == kSchedSettle || (named == SPTRSV_SCHED_AUTO && tuned_valid[cls] && tuned[cls].schedule == kSchedSettle))
+        return SPTRSV_ERR_UNSUPPORTED;
     sptrsv_opts o = resolve(o_in, rhs);
     if (o.precision == SPTRSV_PREC_MIXED && rhs > 1024) return SPTRSV_ERR_UNSUPPORTED;
     int rc = run_resolved(o, b, x, rhs, layout);

@@ -1,10 +1,12 @@
 """What FP64 AUTO's sweeps (settle.cu) take on and leave to the exact kernels: calls that the exact kernels
 answer are answered, and as well."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import sptrsv_gb300 as sp
-from sptrsv_gb300 import gen
+from sptrsv_gb300 import _lib, gen
 
 pytestmark = pytest.mark.gpu
 
@@ -141,3 +143,14 @@ def test_one_long_row(orc, entries, swept, rhs):
     assert (SETTLE in kinds) == swept
     ref = orc.base_gauss_upper(rp.astype(np.uint64), col, val, gen.uniform(1, n * rhs), rhs)
     assert np.max(np.abs(x - ref)) <= 1e-10 * np.max(np.abs(ref))
+
+
+def test_tuned_options_that_name_the_sweeps_are_refused(solver):
+    m = gen.random_upper(100, 4.0, 0.9, 8, 2)
+    solver.analyse(m.row_ptr, m.col, m.val)
+    assert _lib.lib().sptrsv_set_tuned(solver.handle, 1, ctypes.byref(sp.make_opts(schedule=100))) == 0
+    with pytest.raises(sp.SptrsvError) as e:
+        solver.solve(np.ones(m.n))
+    assert e.value.status == -15
+    x = solver.solve(np.ones(m.n * 2), rhs=2)  # another class of right-hand sides
+    assert np.isfinite(x).all()
