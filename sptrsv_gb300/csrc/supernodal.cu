@@ -111,13 +111,19 @@ __global__ void k_sn_rectcols(int S, const int* __restrict__ sstart, const int* 
 }
 
 // T_s^{-1} into the first w columns of G_s (row-major, leading dimension ld), in blocks of 32 rows:
-// k_sn_dinv inverts the diagonal blocks D_I, then k_sn_tinv builds eight columns a block upwards,
+// k_sn_dinv inverts the diagonal blocks D_I, then k_sn_tinv builds four columns a block upwards,
 //     X_I = -D_I sum_{K > I} T_IK X_K,
 // a thread per (row, column) of X_I.  w^3 / 6 FP64 FMAs a chunk bound it (2 a clock and SM); a warp per
 // column substituting row by row, as before, spent five shuffle-and-add steps and a division on each of
-// its w^2 / 2 rows instead.  Measured on GB300, 20^3 dissection factor: 743 -> 42 + 106 us.
+// its w^2 / 2 rows instead.  Measured on GB300, 20^3 dissection factor: 743 -> 43 + 130 us (four columns a CTA;
+// eight 159, two 128).
+//
+// Substitution adds a row's products in 32 chains.  To be as accurate, the sums here are short chains too
+// and each block is refined once by its own residual.  Emulated error in norm against 80 bits, as a multiple
+// of substitution's, 256 rows and a condition of 1e2 / 1e4 / 1e8: 0.98 / 1.01 / 1.03; 128, 64 and 32 rows at
+// 1e4 1.01, 1.00 and 0.98 (four long chains and no refinement: 1.38 / 1.45 / 1.55, 1.34, 1.25 and 1.12).
 constexpr int kInvB = 32;    // rows of a block
-constexpr int kInvCols = 8;  // columns of a CTA
+constexpr int kInvCols = 4;  // columns of a CTA
 
 // T[r][c] of the chunk from row a, c >= r; a skyline row may end inside the triangle.
 __device__ __forceinline__ double sn_t(const int* __restrict__ rp, const double* __restrict__ val, int a, int r, int c) {
@@ -126,9 +132,9 @@ __device__ __forceinline__ double sn_t(const int* __restrict__ rp, const double*
 }
 
 // A warp per diagonal block, a lane per column j of its inverse, upwards from row j: x_r = -acc_r / T_rr
-// (1 / T_jj at r = j), then acc_i += T_ir x_r for every row i above, the sums in registers.  An FP64
+// (1 / T_jj at r = j), then acc_i += T_ir x_r for every row i above, two sums a row in registers.  An FP64
 // operation holds its SM quarter's pipe for 64 cycles, so operations are counted: one reciprocal per
-// lane for all 32 rows instead of 32 divisions of ~14 operations.
+// lane for all 32 rows, and the quotient refined once by its remainder (3 operations a row).
 __global__ void __launch_bounds__(128) k_sn_dinv(const int* __restrict__ sstart, const int* __restrict__ rp,
                                                  const double* __restrict__ val, const long long* __restrict__ goff,
                                                  const int* __restrict__ ld, double* __restrict__ G) {
@@ -144,16 +150,17 @@ __global__ void __launch_bounds__(128) k_sn_dinv(const int* __restrict__ sstart,
         T[r][lane] = lane >= r && lane < nb ? sn_t(rp, val, a, r0 + r, r0 + lane) : (r == lane ? 1.0 : 0.0);
     __syncwarp();
     const double inv = 1.0 / T[lane][lane];
-    double acc[kInvB];
+    double acc[2][kInvB];
 #pragma unroll
-    for (int r = 0; r < kInvB; ++r) acc[r] = 0.0;
+    for (int r = 0; r < kInvB; ++r) acc[0][r] = acc[1][r] = 0.0;
     double* g = G + goff[s] + (size_t)r0 * ld[s] + r0;
 #pragma unroll
     for (int r = kInvB - 1; r >= 0; --r) {
         const double inv_r = __shfl_sync(0xffffffffu, inv, r);
-        const double x = lane < r ? 0.0 : lane == r ? inv : -acc[r] * inv_r;
+        const double y = -(acc[0][r] + acc[1][r]), q = y * inv_r;
+        const double x = lane < r ? 0.0 : lane == r ? inv : fma(fma(-T[r][r], q, y), inv_r, q);
 #pragma unroll
-        for (int i = 0; i < r; ++i) acc[i] = fma(T[i][r], x, acc[i]);
+        for (int i = 0; i < r; ++i) acc[r & 1][i] = fma(T[i][r], x, acc[r & 1][i]);
         if (r < nb && lane < nb) g[(size_t)r * ld[s] + lane] = x;
     }
 }
@@ -166,7 +173,7 @@ __global__ void __launch_bounds__(kInvB * kInvCols) k_sn_tinv(const int2* __rest
                                                                const long long* __restrict__ goff,
                                                                const int* __restrict__ ld, double* __restrict__ G) {
     __shared__ double X[kSnMaxW][kInvCols];
-    __shared__ double M[kInvB][kInvCols];
+    __shared__ double M[kInvB][kInvCols], V[kInvB][kInvCols];
     const int s = tasks[blockIdx.x].x, a = sstart[s], w = sstart[s + 1] - a, j0 = tasks[blockIdx.x].y * kInvCols;
     const int r = threadIdx.x / kInvCols, jj = threadIdx.x % kInvCols, j = j0 + jj;
     const size_t L = ld[s];
@@ -179,26 +186,50 @@ __global__ void __launch_bounds__(kInvB * kInvCols) k_sn_tinv(const int2* __rest
         if (I == jb) {
             if (in && row <= j) v = g[(size_t)row * L + j];  // k_sn_dinv's
         } else {
-            // M = sum_{K > I} T_IK X_K, four chains
-            double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;
-            const int base = rp[a + row] - row, end = min(top, rp[a + row + 1] - base);  // T[row][c] = val[base + c]
-            int c = (I + 1) * kInvB;
-            for (; c + 3 < end; c += 4) {
-                m0 = fma(val[base + c], X[c][jj], m0);
-                m1 = fma(val[base + c + 1], X[c + 1][jj], m1);
-                m2 = fma(val[base + c + 2], X[c + 2][jj], m2);
-                m3 = fma(val[base + c + 3], X[c + 3][jj], m3);
+            const int base = rp[a + row] - row, end = rp[a + row + 1] - base;  // T[row][c] = val[base + c], c < end
+            // m = sum_{K > I} T_IK X_K, a block at a time in eight chains of four
+            double m = 0.0;
+            for (int c0 = (I + 1) * kInvB; c0 < min(top, end); c0 += kInvB) {
+                const int e = min(min(top, end) - c0, kInvB);
+                double p[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+                if (e == kInvB) {
+#pragma unroll
+                    for (int u = 0; u < kInvB; ++u) p[u & 7] = fma(val[base + c0 + u], X[c0 + u][jj], p[u & 7]);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < kInvB; ++u)
+                        if (u < e) p[u & 7] = fma(val[base + c0 + u], X[c0 + u][jj], p[u & 7]);
+                }
+                m += ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
             }
-            for (; c < end; ++c) m0 = fma(val[base + c], X[c][jj], m0);
-            M[r][jj] = (m0 + m1) + (m2 + m3);
+            M[r][jj] = m;
             __syncthreads();
-            double d0 = 0.0, d1 = 0.0;
             const double* d = g + (size_t)row * L + I * kInvB;  // row r of D_I: columns r .. 31
-            for (int q = r; q < kInvB; q += 2) {
-                d0 = fma(d[q], M[q][jj], d0);
-                if (q + 1 < kInvB) d1 = fma(d[q + 1], M[q + 1][jj], d1);
-            }
-            v = -(d0 + d1);
+            // D_I times a block of columns, four chains
+            auto product = [&](const double(*B)[kInvCols]) -> double {
+                double p[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+                for (int q = r & ~3; q < kInvB; q += 4)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (q + u >= r) p[u] = fma(d[q + u], B[q + u][jj], p[u]);
+                return (p[0] + p[1]) + (p[2] + p[3]);
+            };
+            const double v0 = -product(M);
+            V[r][jj] = v0;
+            __syncthreads();
+            // what T_II V leaves of -M, once more through D_I
+            const int last = min(kInvB, end - I * kInvB);
+            double left[2] = {fma(val[base + row], v0, m), 0.0};  // (the diagonal's term cancels most of m)
+#pragma unroll 2
+            for (int q = r & ~3; q < last; q += 4)
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (q + u > r && q + u < last)
+                        left[u & 1] = fma(val[base + I * kInvB + q + u], V[q + u][jj], left[u & 1]);
+            M[r][jj] = left[0] + left[1];
+            __syncthreads();
+            v = v0 - product(M);
             if (in) g[(size_t)row * L + j] = v;
         }
         if (row < kSnMaxW) X[row][jj] = v;
