@@ -382,20 +382,22 @@ __global__ void k_radix_scatter(const unsigned* __restrict__ keys, const int* __
 // Items of a warp's tile: a warp takes them 32 at a time in order, so a long tile is a long chain (4,096
 // items 88 us a pass on GB300 whatever the count), a short one costs 1 KB of histogram to scan.  Enough
 // tiles for 16 warps an SM, between 256 items (500k keys: 88 -> 13 us) and 4,096.
-static int radix_tile(int count) { return std::min(4096, std::max(256, (count / (152 * 16) + 255) / 256 * 256)); }
+static int radix_tile(int count, int sm_count) {
+    return std::min(4096, std::max(256, (count / (sm_count * 16) + 255) / 256 * 256));
+}
 
 // Scratch bytes of a sort of `count` keys.
-size_t sort_scratch(int count) {
-    const int per = radix_tile(count), ntiles = (count + per - 1) / per;
+size_t sort_scratch(int count, int sm_count) {
+    const int per = radix_tile(count, sm_count), ntiles = (count + per - 1) / per;
     return ((size_t)3 * count + (size_t)256 * ntiles + 1 + scan_partials_needed(256 * ntiles)) * sizeof(int) + 8 * 256;
 }
 
 // Sorts keys (count items, values < 2^key_bits) stably; writes the permutation into
-// perm (perm[p] = original index of the p-th smallest).  Takes sort_scratch(count) bytes of scratch.
-int stable_sort_perm(const unsigned* keys_in, int count, int key_bits, int* perm, Scratch& scr, cudaStream_t st,
+// perm (perm[p] = original index of the p-th smallest).  Takes sort_scratch(count, sm_count) bytes of scratch.
+int stable_sort_perm(const unsigned* keys_in, int count, int key_bits, int* perm, Scratch& scr, int sm_count, cudaStream_t st,
                      int64_t* launches) {
     if (count <= 0) return 0;
-    const int per = radix_tile(count), ntiles = (count + per - 1) / per;
+    const int per = radix_tile(count, sm_count), ntiles = (count + per - 1) / per;
     const int nblocks = (ntiles + kRadixWarps - 1) / kRadixWarps;
     unsigned* ka = scr.take<unsigned>(count);
     unsigned* kb = scr.take<unsigned>(count);

@@ -187,7 +187,7 @@ int Handle::ensure_levels() {
     // the level keys -> level_rows
     if ((rc = level_ptr.ensure(sizeof(int) * (size_t)(max_level + 2)))) return rc;
     if ((rc = level_rows.ensure(sizeof(int) * (size_t)n))) return rc;
-    const size_t need = sort_scratch(n) + ((size_t)n + max_level + 2 + scan_partials_needed(max_level + 1)) * sizeof(int) + 4096;
+    const size_t need = sort_scratch(n, sm_count) + ((size_t)n + max_level + 2 + scan_partials_needed(max_level + 1)) * sizeof(int) + 4096;
     if ((rc = scratch.ensure(need))) return rc;
     Scratch scr{(char*)scratch.p, scratch.cap, 0};
     unsigned long long* passes = scr.take<unsigned long long>(3);
@@ -220,7 +220,7 @@ int Handle::ensure_levels() {
     } else {
         int bits = 0;
         while ((1ll << bits) <= (long long)max_level) ++bits;
-        if ((rc = stable_sort_perm((const unsigned*)levels.p, n, bits, level_rows.as<int>(), scr, st, &launches)))
+        if ((rc = stable_sort_perm((const unsigned*)levels.p, n, bits, level_rows.as<int>(), scr, sm_count, st, &launches)))
             return rc;
     }
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -234,7 +234,7 @@ int Handle::build_csc() {
     if ((rc = csc_ptr.ensure(sizeof(int) * (size_t)(n + 1)))) return rc;
     if ((rc = csc_row.ensure(sizeof(int) * (size_t)nnz))) return rc;
     if ((rc = csc_val.ensure(sizeof(double) * (size_t)nnz))) return rc;
-    const size_t need = sort_scratch(nnz) + ((size_t)2 * nnz + n + 2 + scan_partials_needed(n)) * sizeof(int) + 4096;
+    const size_t need = sort_scratch(nnz, sm_count) + ((size_t)2 * nnz + n + 2 + scan_partials_needed(n)) * sizeof(int) + 4096;
     if ((rc = scratch.ensure(need))) return rc;
     Scratch scr{(char*)scratch.p, scratch.cap, 0};
     int* erow = scr.take<int>(nnz);
@@ -245,7 +245,7 @@ int Handle::build_csc() {
     ++launches;
     int bits = 0;
     while ((1ll << bits) < (long long)n) ++bits;
-    if ((rc = stable_sort_perm((const unsigned*)col, nnz, bits, perm, scr, st, &launches))) return rc;
+    if ((rc = stable_sort_perm((const unsigned*)col, nnz, bits, perm, scr, sm_count, st, &launches))) return rc;
     k_gather_csc<<<sm_count * 8, 256, 0, st>>>(nnz, perm, erow, val, csc_row.as<int>(), csc_val.as<double>());
     CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)(n + 1), st));
     k_col_hist<<<sm_count * 8, 256, 0, st>>>(nnz, col, cnt);

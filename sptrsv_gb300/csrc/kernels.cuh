@@ -46,8 +46,8 @@ __global__ void k_validate_csc(int n, int nnz, const int* cp, const int* crow, c
                                Ctl* ctl);
 int scan_exclusive(const int* in, int* out, int count, int* part_scratch, cudaStream_t st, int64_t* launches);
 int scan_partials_needed(int count);
-size_t sort_scratch(int count);
-int stable_sort_perm(const unsigned* keys_in, int count, int key_bits, int* perm, Scratch& scr, cudaStream_t st,
+size_t sort_scratch(int count, int sm_count);
+int stable_sort_perm(const unsigned* keys_in, int count, int key_bits, int* perm, Scratch& scr, int sm_count, cudaStream_t st,
                      int64_t* launches);
 
 // solve.cu -- launchers (return sptrsv_status; add their launches to *launches)
