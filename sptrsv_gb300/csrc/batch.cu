@@ -1328,10 +1328,12 @@ int Batch::build_lists() {
         }
         for (BChunk b : pchunks64[s]) {
             if (!df) b.ghl = nullptr;  // double-FP32 products only in that mode
-            b.poff = poff;
-            b.cbase = cbase;
-            cbase += ng;
-            poff += (long long)b.nblk * b.w * sys[s].rhs;
+            if (!rows64) {  // (rows of panels have no partial sums)
+                b.poff = poff;
+                b.cbase = cbase;
+                cbase += ng;
+                poff += (long long)b.nblk * b.w * sys[s].rhs;
+            }
             g_entries64 += (long long)b.w * (b.w + b.m);
             g_fma64 += (long long)b.w * (b.w + b.m) * sys[s].rhs;
             ch64.push_back(b);
