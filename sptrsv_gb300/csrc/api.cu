@@ -976,7 +976,8 @@ int Handle::sync() {
     if (ctl_copied) c = *h_ctl;
     else if (int rc = read_ctl(&c)) return rc;
     if (c.status) return c.status;
-    if (last_settle && !c.done && !c.abort) settle_failed = true;
+    if (last_settle && ctl_copied && !c.done && !c.abort) settle_failed = true;
+    last_settle = false;
     if (last_mixed) {
         last_steps = c.steps;
         last_sweeps = c.inner_total;
