@@ -96,7 +96,7 @@ void Handle::drop_matrix() {
     auto_supernodes = false;
     skyline = false;
     for (bool& v : tuned_valid) v = false;
-    settle_failed = false;
+    settle_skip = settle_backoff = 0;
     n = nnz = max_level = 0;
     rp = col = nullptr;
     val = nullptr;
@@ -277,12 +277,13 @@ double Handle::exact_us(int rhs) const { return (rhs == 1 ? 0.19 : 2.0) * (level
 // Whether FP64 AUTO tries the sweeps (settle.cu) before the exact kernel: when the sweeps of a contracting
 // matrix take less than 0.7 of the exact kernel's time.  Rows that are not strictly dominant need not
 // contract, and nine sweeps in vain come on top of the exact kernel: there the sweeps have to take less than
-// 0.15 of its time, so that a failed attempt costs 6 %.  A matrix pays for one: its sweeps are not tried
-// again (settle_failed).  Measured on GB300, 8.8 entries a row: 22 times 9 us + 4.5 us per million entries and
+// 0.15 of its time, so that a failed attempt costs 6 %.  After one the exact kernel runs alone for a number
+// of solves (settle_failed): for good would be wrong, since single right-hand sides do not settle on
+// matrices that contract (one entry at the end of a long band reaches a run of rows a sweep).  Measured on GB300, 8.8 entries a row: 22 times 9 us + 4.5 us per million entries and
 // columns (10k rows 225 us, 2M rows 1.9 ms, 200k rows x 8 1.5 ms), and the longest row's walk where its tile
 // is not staged (settle_long_us).
 bool Handle::settle_pays(int rhs) const {
-    return !settle_refused && !settle_failed && mean_len <= kSettleMaxLen &&
+    return mean_len <= kSettleMaxLen &&
            22.0 * (9.0 + 4.5e-6 * (double)nnz * rhs + settle_long_us(n, nnz, rhs, longest)) < (max_ratio < 1.0 ? 0.7 : 0.15) * exact_us(rhs);
 }
 
@@ -866,11 +867,15 @@ int Handle::run_solve(const sptrsv_opts* o_in, const double* b, double* x, int r
         return SPTRSV_ERR_UNSUPPORTED;
     sptrsv_opts o = resolve(o_in, rhs);
     if (o.precision == SPTRSV_PREC_MIXED && rhs > 1024) return SPTRSV_ERR_UNSUPPORTED;
+    if (o.schedule == kSchedSettle && settle_skip > 0) {
+        --settle_skip;
+        o.schedule = exact_schedule(rhs);
+    }
     int rc = run_resolved(o, b, x, rhs, layout);
     if (rc && o.schedule == kSchedSettle) {
         // the sweeps could not be set up (no cooperative launches, no memory): the exact kernel needs neither
         (void)cudaGetLastError();
-        settle_refused = true;
+        settle_failed();
         o.schedule = exact_schedule(rhs);
         rc = run_resolved(o, b, x, rhs, layout);
     }
@@ -976,7 +981,10 @@ int Handle::sync() {
     if (ctl_copied) c = *h_ctl;
     else if (int rc = read_ctl(&c)) return rc;
     if (c.status) return c.status;
-    if (last_settle && ctl_copied && !c.done && !c.abort) settle_failed = true;
+    if (last_settle && ctl_copied && !c.abort) {
+        if (c.done) settle_backoff = 0;
+        else settle_failed();
+    }
     last_settle = false;
     if (last_mixed) {
         last_steps = c.steps;

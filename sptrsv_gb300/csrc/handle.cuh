@@ -1,6 +1,7 @@
 // handle.cuh -- the state behind an sptrsv_handle: one device, one stream, one resident
 // matrix with its analysis, grow-only work buffers and a small cache of solve graphs.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 #include <cuda_runtime.h>
@@ -166,8 +167,10 @@ struct Handle {
     int settle_most(int rhs) const;
     bool settle_pays(int rhs) const;
     bool last_settle = false;     // the last solve ran the sweeps
-    bool settle_failed = false;   // this matrix's sweeps did not settle: FP64 AUTO takes the exact kernels
-    bool settle_refused = false;  // the sweeps could not be launched: FP64 AUTO takes the exact kernels
+    // sweeps that did not settle, or could not be set up: FP64 AUTO takes the exact kernels for so many solves,
+    // 8 after the first failure of a matrix, then twice as many
+    int settle_skip = 0, settle_backoff = 0;
+    void settle_failed() { settle_skip = settle_backoff = std::min(1024, std::max(8, 2 * settle_backoff)); }
     int exact_schedule(int rhs) const;
     sptrsv_opts resolve(const sptrsv_opts* o, int rhs) const;
     int prepare(const sptrsv_opts& o, int rhs, int layout);

@@ -103,7 +103,7 @@ SETTLE = 16
 @pytest.mark.parametrize("rhs", [1, 3])
 @pytest.mark.parametrize("w,tries", [(0.9, 1), (1.0, 1), (1.001, 1), (0.5, 9)])
 def test_sweeps_that_do_not_settle_are_tried_once(w, tries, rhs):
-    """30,000 rows deep, so that an attempt is cheap beside the exact kernel: one attempt a matrix, and the exact
+    """30,000 rows deep, so that an attempt is cheap beside the exact kernel: one attempt, and the exact
     kernel's result from the first solve on (several right-hand sides: its bits)."""
     n = 30_000
     with sp.Solver(0) as s:
@@ -154,3 +154,31 @@ def test_tuned_options_that_name_the_sweeps_are_refused(solver):
     assert e.value.status == -15
     x = solver.solve(np.ones(m.n * 2), rhs=2)  # another class of right-hand sides
     assert np.isfinite(x).all()
+
+
+def test_refused_sweeps_are_tried_again_with_the_next_matrix(monkeypatch):
+    n = 30_000
+    m = gen.random_upper(n, 8.0, 0.9, 64, 5)
+    with sp.Solver(0) as s:
+        monkeypatch.setenv("SPTRSV_NO_COOPERATIVE", "1")
+        s.analyse(m.row_ptr, m.col, m.val)
+        assert SETTLE not in _kernels(s, n, 1)[1]
+        monkeypatch.delenv("SPTRSV_NO_COOPERATIVE")
+        assert SETTLE not in _kernels(s, n, 1)[1]
+        s.analyse(m.row_ptr, m.col, m.val)
+        assert SETTLE in _kernels(s, n, 1)[1]
+
+
+def test_attempts_are_spaced_out_and_come_back():
+    """After a failure 8 solves without an attempt, after the next 16; right-hand sides that settle end that."""
+    n = 30_000
+    with sp.Solver(0) as s:
+        s.analyse(*_chain(n, 0.9))
+        assert [k for k in range(30) if SETTLE in _kernels(s, n, 1)[1]] == [0, 9, 26]
+        # a band that contracts, and one entry at its end
+        s.analyse(*_chain(n, 0.7))
+        e = np.zeros(n)
+        e[-1] = 1.0
+        assert np.max(np.abs(s.solve(e) - (-0.7) ** np.arange(n - 1, -1, -1))) <= 1e-12
+        assert SETTLE in [k for _ in range(9) for k in _kernels(s, n, 1)[1]]
+        assert SETTLE in _kernels(s, n, 1)[1]
