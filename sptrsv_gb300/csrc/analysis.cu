@@ -68,7 +68,9 @@ k_check_rows(int n, int nnz, const int* __restrict__ rp, const int* __restrict__
     __shared__ int s_col[kLong ? 1 : W][kRowsCap];
     __shared__ double s_val[kLong ? 1 : W][kRowsCap];
     __shared__ struct { double off; int near; bool contiguous; int err; } s_row[32];
+    __shared__ unsigned long long s_stats[5];  // the block's statistics: one atomic a block on each address
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x < 5) s_stats[threadIdx.x] = 0ull;
     double worst = 0.0, worst_off = 0.0, worst_d = 1.0;  // the lane's row of the largest off / |d|
     float depth = 0.f;
     unsigned long long len2 = 0, gapped = 0;
@@ -159,7 +161,7 @@ k_check_rows(int n, int nnz, const int* __restrict__ rp, const int* __restrict__
         len2 += (unsigned long long)(e - s) * (unsigned long long)(e - s);
         longest = max(longest, e - s);
     }
-    __syncwarp();
+    __syncthreads();
     if (!kLong || w == 0) {
         double mr = worst_off / worst_d, dep = (double)depth;
         for (int o = 16; o > 0; o >>= 1) {
@@ -170,13 +172,18 @@ k_check_rows(int n, int nnz, const int* __restrict__ rp, const int* __restrict__
         }
         longest = __reduce_max_sync(0xffffffffu, longest);
         if (lane == 0) {
-            atomicMax(stats, (unsigned long long)__double_as_longlong(mr));  // mr >= 0: bit order = value order
-            atomicAdd(stats + 1, len2);
-            atomicAdd(reinterpret_cast<double*>(stats + 2), dep);
-            atomicAdd(stats + 3, gapped);
-            atomicMax(stats + 4, (unsigned long long)longest);
+            atomicMax(s_stats, (unsigned long long)__double_as_longlong(mr));  // mr >= 0: bit order = value order
+            atomicAdd(s_stats + 1, len2);
+            atomicAdd(reinterpret_cast<double*>(s_stats + 2), dep);
+            atomicAdd(s_stats + 3, gapped);
+            atomicMax(s_stats + 4, (unsigned long long)longest);
         }
     }
+    __syncthreads();
+    const int q = threadIdx.x;
+    if (q == 0 || q == 4) atomicMax(stats + q, s_stats[q]);
+    else if (q == 2) atomicAdd(reinterpret_cast<double*>(stats + 2), __longlong_as_double((long long)s_stats[2]));
+    else if (q < 4) atomicAdd(stats + q, s_stats[q]);
     if (blockIdx.x == 0 && threadIdx.x == 0 && rp[n] != nnz) record_error(ctl, SPTRSV_ERR_ROW_PTR);
 }
 
