@@ -462,7 +462,8 @@ def run_ours(args, dist):
             per_kind.setdefault(kind, []).append(t)
     s.profile(False)
     kind_names = {1: "fill", 2: "pull_warp", 3: "pull_thread", 4: "push_csc", 5: "levelset", 6: "init",
-                  7: "residual", 8: "check", 9: "jacobi_sweep", 10: "inner_exact", 11: "axpy", 12: "transpose"}
+                  7: "residual", 8: "check", 9: "jacobi_sweep", 10: "inner_exact", 11: "axpy", 12: "transpose",
+                  15: "window", 16: "settle"}
     shares = {kind_names.get(k, str(k)): {"launches_per_solve": len(v) / prof_steps, "total_ms_per_solve": sum(v) / prof_steps}
               for k, v in per_kind.items()}
     dom_kind = max(per_kind, key=lambda k: sum(per_kind[k]))
@@ -562,7 +563,8 @@ def run_ours(args, dist):
         "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": nbytes, "d2h_bytes_per_step": nbytes},
         "roofline": {"bound": "hbm", "kernel": dom_name, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_src, "traffic": traffic,
-                     "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": dom_avg_ms},
+                     "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": dom_avg_ms,
+                     "launches": "profiled solves: one sweep a launch; timed solves run a whole inner solve a launch"},
         "kernel_shares": shares,
         "gpu_launches": gpu_launches,
         "clocks": ck,

@@ -1371,7 +1371,6 @@ int launch_build_offdiag(int n, const int* rp, const int* col, const double* val
     k_build_roff<<<sm_count * 4, 256, 0, st>>>(n, roff_pad, rp, roff);
     *launches += 2;
     CUDA_TRY(cudaGetLastError());
-    // opt in to the sweep kernel's dynamic shared memory here, outside any stream capture
     return 0;
 }
 

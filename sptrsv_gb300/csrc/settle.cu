@@ -16,9 +16,10 @@
 // rounding flips keep a few hundred rows of millions moving by a few ulps for as many sweeps again), and
 // the sweeps go on until what is left at that rate is below 2^-54, half the rounding of one term.
 // Emulated on the CPU against 80-bit solutions, 20,000 rows, error in norm as a multiple of
-// substitution's: chains x_i = b_i + w x_i+1 with w = 0.3 / 0.5 / 0.6 / 0.7 1.01 / 1.00 / 1.12 / 1.08
-// (stopped at a record of 2^-48: 1.0 / 1.1 / 1.5 / 6.6), two entries of 0.35 0.92 (12), eight of 0.075
-// 0.66 (3.2), the random recipe 0.72 (0.72: it gains four bits a sweep).
+// substitution's: chains x_i = b_i + w x_i+1 with w = 0.3 / 0.5 / 0.6 / 0.7 / 0.8 1.01 / 1.00 / 1.12 / 1.08 /
+// 1.14 with one right-hand side (stopped at a record of 2^-48: 1.0 / 1.1 / 1.4 / 1.7 / 5.1), 1.00 or left to
+// the exact kernel with several (1.0 / 1.9 / 3.6 / 5.2 / 9.7); two entries of 0.35 0.93 (4.8 and 11), eight
+// of 0.075 0.68 (1.2 and 2.9), the random recipe 0.71 (0.71: it gains four bits a sweep).
 //
 // Sweep order.  Each warp owns a contiguous run of rows and walks it upwards from its bottom, 32 rows
 // a tile (lane per row; 32 / NC rows for NC right-hand sides): a row sees this sweep's values of
@@ -38,8 +39,8 @@
 // Bound by the FP64 pipe (57 % active by ncu at 500k rows; an operation holds its SM quarter's pipe for 64
 // cycles, and a tile takes its longest row's count, 1.9 times the mean of 7.6 off-diagonals) and, below
 // ~200k rows, by the chain of loads and FMAs through a tile.  Measured on GB300, 8.8 entries a row: 2M rows
-// 68 -> 1.8 ms (16 sweeps), 200k rows 6.9 -> 0.44 ms (18), 50k rows 1.7 -> 0.28 ms (19); 200k rows x 8 columns
-// 70 -> 1.35 ms (22).  Tried and not kept: two FP32 corrections first (their sweeps are bound by instructions
+// 68 -> 1.87 ms (16 sweeps of 116 us), 200k rows 6.9 -> 0.45 ms (20), 50k rows 1.7 -> 0.29 ms (20), 10k rows
+// 0.37 -> 0.23 ms (34 of 6 us); 200k rows x 8 columns 70 -> 1.52 ms (27).  Tried and not kept: two FP32 corrections first (their sweeps are bound by instructions
 // and L1, 90 us against 120 at 2M rows: 3.4 ms in all against 3.1 then), rows kept in shared memory for all
 // sweeps (200k rows 0.40, but 200k x 8 1.69), 16-byte copies for the staging (no change).
 //
