@@ -279,18 +279,20 @@ double Handle::exact_us(int rhs) const { return (rhs == 1 ? 0.19 : 2.0) * (level
 // contract, and nine sweeps in vain come on top of the exact kernel: there the sweeps have to take less than
 // 0.15 of its time, so that a failed attempt costs 6 %.  After one the exact kernel runs alone for a number
 // of solves (settle_failed): for good would be wrong, since single right-hand sides do not settle on
-// matrices that contract (one entry at the end of a long band reaches a run of rows a sweep).  Measured on GB300, 8.8 entries a row: 22 times 9 us + 4.5 us per million entries and
-// columns (10k rows 225 us, 2M rows 1.9 ms, 200k rows x 8 1.5 ms), and the longest row's walk where its tile
-// is not staged (settle_long_us).
+// matrices that contract (one entry at the end of a long band reaches a run of rows a sweep).
+// Measured on GB300, 8.8 entries a row: 22 times 9 us + 4.5 us per million entries and columns (10k rows
+// 225 us, 2M rows 1.9 ms, 200k rows x 8 1.5 ms), and the longest row's walk where its tile is not staged
+// (settle_long_us).
 bool Handle::settle_pays(int rhs) const {
-    return mean_len <= kSettleMaxLen &&
-           22.0 * (9.0 + 4.5e-6 * (double)nnz * rhs + settle_long_us(n, nnz, rhs, longest)) < (max_ratio < 1.0 ? 0.7 : 0.15) * exact_us(rhs);
+    const double sweep_us = 9.0 + 4.5e-6 * (double)nnz * rhs + settle_long_us(n, nnz, rhs, longest);
+    return mean_len <= kSettleMaxLen && 22.0 * sweep_us < (max_ratio < 1.0 ? 0.7 : 0.15) * exact_us(rhs);
 }
 
 // The most sweeps: as many as take the exact kernel's time.  Small systems make more and shorter sweeps than
 // the rule above counts (10k rows: 34 of 6 us).
 int Handle::settle_most(int rhs) const {
-    return (int)std::min<double>(kSettleSweeps, exact_us(rhs) / (6.0 + 4.5e-6 * (double)nnz * rhs + settle_long_us(n, nnz, rhs, longest)));
+    const double sweep_us = 6.0 + 4.5e-6 * (double)nnz * rhs + settle_long_us(n, nnz, rhs, longest);
+    return (int)std::min<double>(kSettleSweeps, exact_us(rhs) / sweep_us);
 }
 
 // The exact sync-free kernel of FP64 AUTO: for one RHS the window or the block kernel (auto_window),
